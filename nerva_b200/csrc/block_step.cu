@@ -4,7 +4,7 @@
 //     to 32 sessions that share weights (reference: hf_decode_sequence/
 //     session_api_batch_fork_destroy.inc.cu:1-310, kernels.cu:804-930 pack/scatter,
 //     projection.cu:192-262 one skinny GEMM per projection);
-//   * the chunked prefill of session_start — up to 256 prompt positions of one session at a time
+//   * the chunked prefill of session_start — up to 2048 prompt positions of one session at a time
 //     (reference: session_decode_prefill.inc.cu:1879-2245, prefill_kernels.cu:66-170).
 // Per layer: RMSNorm of the block -> QKV block projection -> (prefill: q/k-norm + RoPE + paged KV
 // publish for all rows) -> split attention, one set of blocks per row -> O block projection with
@@ -197,11 +197,11 @@ bool carve(StaticArena &arena, void *base, uint64_t count, T **out) {
 bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, void *base) {
   const ModelDims &d = s->dims;
   const uint64_t ah = d.attention_hidden(), kvh = d.kv_hidden(), qkv_rows = ah + 2 * kvh;
-  const uint64_t rows = ws->max_rows, sample = ws->sample_rows;
+  const uint64_t rows = ws->max_rows, part = ws->part_rows, sample = ws->sample_rows;
   if (s->parallel) {
     const ParallelPlan &plan = *s->parallel;
     const uint64_t words = plan.element_bytes() / 2u;
-    const uint64_t slots = std::max<uint64_t>(rows * plan.max_heads * kWindowMaxSplits, 1u);
+    const uint64_t slots = std::max<uint64_t>(part * plan.max_heads * kWindowMaxSplits, 1u);
     bool ok = carve(arena, base, rows * plan.x_width() * words, &ws->x_bf16);
     ok = ok && carve(arena, base, rows * plan.max_qkv_pad, &ws->qkv);
     ok = ok && carve(arena, base, rows * plan.max_attn_pad * words, &ws->attn);
@@ -211,7 +211,7 @@ bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, vo
     ok = ok && carve(arena, base, slots * std::max(plan.max_v_pad, 1u), &ws->partial_acc);
     ok = ok && carve(arena, base, slots, &ws->partial_m);
     ok = ok && carve(arena, base, slots, &ws->partial_l);
-    ok = ok && carve(arena, base, rows * std::max(plan.max_heads, 1u), &ws->attn_tickets);
+    ok = ok && carve(arena, base, part * std::max(plan.max_heads, 1u), &ws->attn_tickets);
     if (plan.sandwich) ok = ok && carve(arena, base, rows * plan.width_pad, &ws->h_a);
     if (plan.loop_input) ok = ok && carve(arena, base, rows * plan.width_pad, &ws->first);
     if (plan.max_space_pad != 0) {
@@ -220,7 +220,7 @@ bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, vo
       ok = ok && carve(arena, base, rows * plan.max_conv_width * words, &convolved);
       ws->convolved = convolved;
     }
-    ok = ok && carve(arena, base, gemm_tc_workspace_bytes(ws->max_rows, s->sm_count) / sizeof(float), &ws->gemm_workspace);
+    ok = ok && carve(arena, base, gemm_tc_workspace_bytes(ws->part_rows, s->sm_count) / sizeof(float), &ws->gemm_workspace);
     ok = ok && carve(arena, base, sample * kBlockArgmaxChunks, &ws->best_value);
     ok = ok && carve(arena, base, sample * kBlockArgmaxChunks, &ws->best_index);
     ok = ok && carve(arena, base, rows, &ws->attn_rows);
@@ -239,11 +239,11 @@ bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, vo
   ok = ok && carve(arena, base, rows * d.hidden, &ws->h_b);
   ok = ok && carve(arena, base, rows * d.intermediate, &ws->ff);
   ok = ok && carve(arena, base, sample * d.vocab, &ws->logits);
-  ok = ok && carve(arena, base, rows * d.heads * 16u * d.head_dim, &ws->partial_acc);
-  ok = ok && carve(arena, base, rows * d.heads * 16u, &ws->partial_m);
-  ok = ok && carve(arena, base, rows * d.heads * 16u, &ws->partial_l);
-  ok = ok && carve(arena, base, rows * d.kv_heads, &ws->attn_tickets);
-  ok = ok && carve(arena, base, gemm_tc_workspace_bytes(ws->max_rows, s->sm_count) / sizeof(float), &ws->gemm_workspace);
+  ok = ok && carve(arena, base, part * d.heads * 16u * d.head_dim, &ws->partial_acc);
+  ok = ok && carve(arena, base, part * d.heads * 16u, &ws->partial_m);
+  ok = ok && carve(arena, base, part * d.heads * 16u, &ws->partial_l);
+  ok = ok && carve(arena, base, part * d.kv_heads, &ws->attn_tickets);
+  ok = ok && carve(arena, base, gemm_tc_workspace_bytes(ws->part_rows, s->sm_count) / sizeof(float), &ws->gemm_workspace);
   ok = ok && carve(arena, base, static_cast<uint64_t>(gemm_tc_ticket_count(max_out)), &ws->gemm_tickets);
   ok = ok && carve(arena, base, sample * kBlockArgmaxChunks, &ws->best_value);
   ok = ok && carve(arena, base, sample * kBlockArgmaxChunks, &ws->best_index);
@@ -339,21 +339,23 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
     if (err != cudaSuccess) break;
     if (paged) {
       // every row's K/V (its own newest row included) is in its cache and its queries are prepared
+      for (uint32_t at = 0; err == cudaSuccess && at < b.rows; at += ws.part_rows) {
       AttentionParams ap{};
-      ap.batch = b.rows;
+      ap.batch = std::min(ws.part_rows, b.rows - at);
       ap.heads = d.heads;
       ap.kv_heads = d.kv_heads;
       ap.head_dim = d.head_dim;
-      ap.splits = attention_rows_splits(b.longest, b.rows, d.kv_heads, s->sm_count);
+      ap.splits = attention_rows_splits(b.longest, ap.batch, d.kv_heads, s->sm_count);
       ap.partial_acc = ws.partial_acc;
       ap.partial_m = ws.partial_m;
       ap.partial_l = ws.partial_l;
-      ap.out_bf16 = ws.attn;
+      ap.out_bf16 = ws.attn + static_cast<uint64_t>(at) * ah;
       ap.error_word = s->device_error;
-      ap.rows = ws.attn_rows;
+      ap.rows = ws.attn_rows + at;
       ap.layer = l;
       err = launch_attention_rows(b.stream, ap, b.k_maps.data(), b.v_maps.data(), static_cast<uint32_t>(b.k_maps.size()));
       n += 2;
+      }
       if (err != cudaSuccess) break;
     } else {
     FusedAttentionParams fp{};
@@ -370,12 +372,14 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
     fp.rope_theta = s->rope_theta;
     fp.splits = b.splits;
     fp.pdl = b.pdl ? 1u : 0u;
-    fp.rows = ws.attn_rows;
-    fp.row_count = b.rows;
     fp.layer = l;
     fp.cached_only = b.publish ? 1u : 0u;
-    err = launch_fused_attention(b.stream, fp);
-    n += 1;
+    for (uint32_t at = 0; err == cudaSuccess && at < b.rows; at += ws.part_rows) {
+      fp.rows = ws.attn_rows + at;
+      fp.row_count = std::min(ws.part_rows, b.rows - at);
+      err = launch_fused_attention(b.stream, fp);
+      n += 1;
+    }
     if (err != cudaSuccess) break;
     }
     // h_a = h_b + O(attention)
@@ -439,10 +443,11 @@ FusedAttentionRow attention_row(Session *s, const BlockWorkspace &ws, uint32_t r
   r.kv_layer_elems = s->kv_layer_elems;
   r.page_table = s->page_table;
   r.recurrent = s->recurrent;
-  r.partial_acc = ws.partial_acc + static_cast<uint64_t>(row) * d.heads * 16u * d.head_dim;
-  r.partial_m = ws.partial_m + static_cast<uint64_t>(row) * d.heads * 16u;
-  r.partial_l = ws.partial_l + static_cast<uint64_t>(row) * d.heads * 16u;
-  r.tickets = ws.attn_tickets + static_cast<uint64_t>(row) * d.kv_heads;
+  const uint64_t slot = row % ws.part_rows;  // rows of different parts run one launch after the other
+  r.partial_acc = ws.partial_acc + slot * d.heads * 16u * d.head_dim;
+  r.partial_m = ws.partial_m + slot * d.heads * 16u;
+  r.partial_l = ws.partial_l + slot * d.heads * 16u;
+  r.tickets = ws.attn_tickets + slot * d.kv_heads;
   r.out_bf16 = ws.attn + static_cast<uint64_t>(row) * d.attention_hidden();
   r.error_word = s->device_error;
   return r;
@@ -494,7 +499,9 @@ cudaError_t launch_argmax_partials(cudaStream_t stream, const float *logits, uin
 cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
   BlockWorkspace &ws = s->weights->block_ws;
   const uint32_t context_rows = (s->max_context + 15u) & ~15u;
-  ws.max_rows = std::max(kBlockSampleRows, std::min(kBlockMaxRows, context_rows));
+  const uint32_t most = s->parallel && s->parallel->f32 ? kBlockPartRows : kBlockMaxRows;
+  ws.max_rows = std::max(kBlockSampleRows, std::min(most, context_rows));
+  ws.part_rows = std::min(ws.max_rows, kBlockPartRows);
   ws.sample_rows = kBlockSampleRows;
   StaticArena sizing(UINT64_MAX / 2);
   if (!plan_workspace(s, &ws, sizing, nullptr)) return cudaErrorMemoryAllocation;
@@ -512,7 +519,7 @@ cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
   const uint32_t max_out = std::max(std::max<uint32_t>(static_cast<uint32_t>(d.attention_hidden() + 2 * d.kv_hidden()),
                                                       2u * d.intermediate),
                                     std::max(d.hidden, d.vocab));
-  err = cudaMemsetAsync(ws.attn_tickets, 0, static_cast<uint64_t>(ws.max_rows) * d.kv_heads * sizeof(uint32_t), s->stream);
+  err = cudaMemsetAsync(ws.attn_tickets, 0, static_cast<uint64_t>(ws.part_rows) * d.kv_heads * sizeof(uint32_t), s->stream);
   if (err == cudaSuccess)
     err = cudaMemsetAsync(ws.gemm_tickets, 0, static_cast<uint64_t>(gemm_tc_ticket_count(max_out)) * sizeof(uint32_t),
                           s->stream);
@@ -593,8 +600,12 @@ cudaError_t enqueue_chunked_prefill(NervaCudaHfDecodeSequenceSession *s, uint32_
   const ModelDims &d = s->dims;
   const uint64_t width = s->parallel ? s->parallel->width_pad : d.hidden;
   cudaError_t err = cudaSuccess;
-  for (uint32_t begin = first; err == cudaSuccess && begin < prompt_count; begin += ws.max_rows) {
-    const uint32_t rows = std::min(ws.max_rows, prompt_count - begin);
+  // chunks of about one size: no small remainder that would stream the weights for a few rows
+  const uint32_t chunks = (prompt_count - first + ws.max_rows - 1u) / ws.max_rows;
+  const uint32_t even = ((prompt_count - first + chunks - 1u) / chunks + 15u) & ~15u;
+  const uint32_t chunk_rows = std::min(even, ws.max_rows);
+  for (uint32_t begin = first; err == cudaSuccess && begin < prompt_count; begin += chunk_rows) {
+    const uint32_t rows = std::min(chunk_rows, prompt_count - begin);
     std::vector<FusedAttentionRow> attn(rows);
     std::vector<BlockTokenRow> tokens(rows);
     for (uint32_t r = 0; r < rows; ++r) {

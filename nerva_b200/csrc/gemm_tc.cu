@@ -36,20 +36,14 @@
 
 #include <mutex>
 
-#include "common.cuh"
-#include "kernels.cuh"
+#include "gemm_device.cuh"
 
 namespace nb {
 namespace {
 
-constexpr uint32_t kTileRows = 128;   // MMA M
-constexpr uint32_t kSliceK = 64;      // bf16 elements per ring stage along the inner dimension (128 bytes)
-constexpr uint32_t kUmmaK = 16;       // inner elements per MMA instruction
-constexpr uint32_t kATileBytes = kTileRows * kSliceK * 2u;
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kGemmThreads = 192;
 constexpr uint32_t kEpilogueThreads = 128;
-constexpr uint32_t kGroup = 16;         // tokens per tcgen05.ld
 // Blocks of up to kSmallBlockTokens tokens run two thread blocks per SM (half the shared memory and
 // a quarter of the tensor memory each): while one block of a launch drains its last tile, writes
 // its results and leaves, the block that takes its place — of this launch or, with programmatic
@@ -62,26 +56,6 @@ struct GemmShared {
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   uint32_t abort;
-};
-
-struct GemmKernelParams {
-  uint32_t rows, cols, tokens, n_pad;  // n_pad: tokens rounded up to 16 (the MMA N)
-  uint32_t stages;
-  uint32_t tmem_columns;  // allocation: two accumulator buffers of tmem_columns / 2 fp32 columns
-  uint32_t epilogue;
-  uint32_t split_row;         // kEpilogueStoreSwiglu: first row of the gate/up pairs (a multiple of 32)
-  const float *resid_in;
-  const uint16_t *row_scale;  // kEpilogueStore, optional: y is multiplied by row_scale[row] before the residual add
-  const uint16_t *row_add;    // kEpilogueStore, optional: added to y
-  uint32_t activation;        // of the gate in gate/up pairs
-  float scale;                // kEpilogueStore: 0, or a factor on y
-  float softcap;              // kEpilogueStore: 0, or y becomes softcap * tanh(y / softcap)
-  float *out_f32;
-  uint16_t *out_bf16;
-  float *workspace;
-  uint32_t *tickets;
-  uint32_t *error_word;
-  unsigned long long *stamps;
 };
 
 // Timeline stamp by an arbitrary thread of the first or the last block (common.cuh stamp() is thread 0 only).
@@ -150,118 +124,6 @@ struct SegmentWalk {
     return true;
   }
 };
-
-// ---- PTX wrappers ----
-__device__ __forceinline__ bool abortable_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort,
-                                               uint32_t *error_word) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  for (;;) {
-#pragma unroll 1
-    for (uint32_t spin = 0; spin < 64; ++spin) {
-      if (mbar_try_wait(bar, parity)) return true;
-    }
-    if (*abort != 0u) return false;
-    if (clock64() - start > kWaitCycleLimit) {
-      *abort = 1u;
-      report_error(error_word, kErrTmaWaitTimeout);
-      return false;
-    }
-  }
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar,
-                                            uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
-      "[%0], [%1, {%2, %3}], [%4], %5;" ::"r"(smem_addr(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar)), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ uint64_t l2_evict_last_policy() {
-  uint64_t policy;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
-  return policy;
-}
-__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tcgen05_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, float *v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (uint32_t i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (one swizzle atom):
-// start address, 8-row groups 1024 bytes apart, SWIZZLE_128B, descriptor version 1.
-__device__ __forceinline__ uint64_t kmajor_sw128_desc(const void *tile) {
-  const uint64_t addr = smem_addr(tile);
-  return ((addr & 0x3ffffull) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024u >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
-}
-// Instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, N = n, M = 128.
-__device__ __forceinline__ uint32_t instr_desc_bf16(uint32_t n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kTileRows >> 4) << 24);
-}
-
-// N consecutive tokens m0 .. m0 + N - 1 of accumulator row `row`, values in v.  Called by all 32 lanes
-// of a warp whose lanes hold 32 consecutive rows (the first a multiple of 32).
-template <uint32_t N>
-__device__ __forceinline__ void row_epilogue(const GemmKernelParams &p, const float (&v)[N], uint32_t row, uint32_t m0,
-                                             uint32_t lane) {
-  const bool pairs = p.epilogue == kEpilogueSwiglu || (p.epilogue == kEpilogueStoreSwiglu && row >= p.split_row);
-  if (pairs) {
-    // rows interleaved (gate, up): the neighbouring lane holds the other half of the pair
-    const uint32_t base = p.epilogue == kEpilogueStoreSwiglu ? p.split_row : 0u;
-    const uint32_t width = (p.rows - base) / 2u;
-    auto store = [&](auto act) {  // one loop per activation: the epilogue's last tile is not hidden behind anything
-#pragma unroll
-      for (uint32_t j = 0; j < N; ++j) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
-        const uint32_t m = m0 + j;
-        if ((lane & 1u) == 0 && row + 1u < p.rows && m < p.tokens)
-          p.out_bf16[static_cast<uint64_t>(m) * width + (row - base) / 2u] = f32_to_bf16_bits(act(v[j]) * other);
-      }
-    };
-    if (p.activation == kActivationSilu)
-      store([](float x) { return silu(x); });
-    else
-      store([](float x) { return activate(kActivationGeluTanh, x); });
-  } else if (row < p.rows) {
-    const uint32_t width = p.epilogue == kEpilogueStoreSwiglu ? p.split_row : p.rows;
-    const float scale = (p.row_scale != nullptr ? bf16_bits_to_f32(p.row_scale[row]) : 1.0f) * (p.scale != 0.0f ? p.scale : 1.0f);
-    const float add = p.row_add != nullptr ? bf16_bits_to_f32(p.row_add[row]) : 0.0f;
-#pragma unroll
-    for (uint32_t j = 0; j < N; ++j) {
-      const uint32_t m = m0 + j;
-      if (m < p.tokens) {
-        const uint64_t at = static_cast<uint64_t>(m) * width + row;
-        float y = fmaf(v[j], scale, add);
-        if (p.softcap > 0.0f) y = p.softcap * tanhf(y / p.softcap);
-        p.out_f32[at] = p.resid_in != nullptr ? y + __ldcg(p.resid_in + at) : y;
-      }
-    }
-  }
-}
 
 // Finishes the row tiles that more than one block of gemm_tc_kernel contributed to.  Grid (row
 // tiles, n_pad / 16), block (128 rows, 4 groups of 4 tokens): a thread adds the partials of its four
@@ -574,13 +436,18 @@ bool encode_bf16_map_2d(void *map, const uint16_t *base, uint64_t inner, uint64_
                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool gemm_tc_eligible(const GemmParams &g) {
-  return g.tokens >= 1 && g.tokens <= kGemmMaxTokens && g.cols % kSliceK == 0 && g.cols != 0 && g.rows != 0 &&
+// Everything but the number of tokens.
+static bool gemm_shape_ok(const GemmParams &g) {
+  return g.cols % kSliceK == 0 && g.cols != 0 && g.rows != 0 &&
          reinterpret_cast<uintptr_t>(g.weight) % 16u == 0 && reinterpret_cast<uintptr_t>(g.x) % 16u == 0 &&
          (g.epilogue != kEpilogueSwiglu || g.rows % 2u == 0) &&
          (g.epilogue != kEpilogueStoreSwiglu || (g.rows % 2u == 0 && g.split_row % 32u == 0 && g.split_row <= g.rows)) &&
          (g.epilogue == kEpilogueStore || g.epilogue == kEpilogueSwiglu || g.epilogue == kEpilogueStoreSwiglu);
 }
+
+bool gemm_tc_eligible(const GemmParams &g) { return g.tokens >= 1 && g.tokens <= kGemmMaxTokens && gemm_shape_ok(g); }
+
+bool gemm_wide_eligible(const GemmParams &g) { return g.tokens > kGemmMaxTokens && gemm_shape_ok(g); }
 
 uint64_t gemm_tc_workspace_bytes(uint32_t tokens, uint32_t sm_count) {
   // two partial accumulators per thread block of the 2 x sm_count grid
@@ -590,32 +457,18 @@ uint64_t gemm_tc_workspace_bytes(uint32_t tokens, uint32_t sm_count) {
 uint32_t gemm_tc_ticket_count(uint32_t rows) { return (rows + kTileRows - 1u) / kTileRows; }
 
 cudaError_t configure_gemm_tc_kernel() {
-  return cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  const cudaError_t err = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  return err == cudaSuccess ? configure_gemm_wide_kernel() : err;
 }
 
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count) {
+  // more tokens than one MMA is wide: what the caller asks for is arithmetic, not a weight stream
+  if (gemm_wide_eligible(g)) return launch_gemm_wide(stream, g, sm_count);
   if (!gemm_tc_eligible(g) || g.workspace == nullptr) return cudaErrorInvalidValue;
-  GemmKernelParams p{};
-  p.rows = g.rows;
-  p.cols = g.cols;
-  p.tokens = g.tokens;
+  GemmKernelParams p = gemm_kernel_params(g);
   p.n_pad = padded_tokens(g.tokens);
   p.stages = stages_for(p.n_pad);
   p.tmem_columns = tmem_columns_for(p.n_pad);
-  p.epilogue = g.epilogue;
-  p.split_row = g.split_row;
-  p.resid_in = g.resid_in;
-  p.row_scale = g.row_scale;
-  p.row_add = g.row_add;
-  p.activation = g.activation;
-  p.scale = g.scale;
-  p.softcap = g.softcap;
-  p.out_f32 = g.out_f32;
-  p.out_bf16 = g.out_bf16;
-  p.workspace = g.workspace;
-  p.tickets = g.tickets;
-  p.error_word = g.error_word;
-  p.stamps = g.stamps;
   CUtensorMap map_w, map_x;
   if (!make_map(&map_w, g.weight, g.cols, g.rows, kTileRows) || !make_map(&map_x, g.x, g.cols, g.tokens, p.n_pad))
     return cudaErrorNotSupported;

@@ -102,7 +102,8 @@ struct ProjectionParams {
 
 constexpr uint32_t kTimelineSlots = 8;
 
-// ---- block projection on the tensor pipe (gemm_tc.cu): 2..256 tokens, weights streamed once ----
+// ---- block projection on the tensor pipe: up to 256 tokens bound by the weight stream (gemm_tc.cu), more by the
+// tensor pipe (gemm_wide.cu) ----
 constexpr uint32_t kGemmMaxTokens = 256;
 struct GemmParams {
   const uint16_t *weight;  // [rows][cols] bf16 row-major, cols a multiple of 64
@@ -121,7 +122,7 @@ struct GemmParams {
   const float *resid_in;   // optional [tokens][rows]; may be out_f32
   float *out_f32;          // [tokens][rows]
   uint16_t *out_bf16;      // [tokens][rows/2]
-  float *workspace;        // gemm_tc_workspace_bytes(tokens, sm_count)
+  float *workspace;        // gemm_tc_workspace_bytes(tokens, sm_count); unused above kGemmMaxTokens
   uint32_t *tickets;       // unused (kept so that callers' buffer plans stay as they are)
   uint32_t *error_word;
   uint32_t pdl;
@@ -129,6 +130,7 @@ struct GemmParams {
                                // tile ready for the MMA, last MMA committed, exit
 };
 bool gemm_tc_eligible(const GemmParams &g);
+bool gemm_wide_eligible(const GemmParams &g);  // the same shapes, more than kGemmMaxTokens tokens
 uint64_t gemm_tc_workspace_bytes(uint32_t tokens, uint32_t sm_count);
 uint32_t gemm_tc_ticket_count(uint32_t rows);
 bool tensor_map_available();  // the driver exposes the tensor-map encoder the TMA kernels need
@@ -137,7 +139,10 @@ bool tensor_map_available();  // the driver exposes the tensor-map encoder the T
 // elements outside the tensor read as zero.
 bool encode_bf16_map_2d(void *map, const uint16_t *base, uint64_t inner, uint64_t outer, uint32_t box_inner,
                         uint32_t box_outer);
-cudaError_t configure_gemm_tc_kernel();
+cudaError_t configure_gemm_tc_kernel();  // and gemm_wide.cu's
+cudaError_t configure_gemm_wide_kernel();
+// launch_gemm_tc takes any number of tokens: above kGemmMaxTokens it is launch_gemm_wide.
+cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);
 
 // Number of blocks launch_projection will use (= number of arg-max partials).

@@ -129,13 +129,14 @@ extern "C" int nerva_b200_projection(const uint16_t *weight, const uint16_t *x, 
   g.tokens = tokens;
   g.epilogue = kEpilogueStore;
   g.out_f32 = d_y;
-  const bool block = tokens > 1 && gemm_tc_eligible(g);
+  const bool block = tokens > 1 && (gemm_tc_eligible(g) || gemm_wide_eligible(g));
   uint32_t *d_error = nullptr;
   if (block) {
     float *d_ws = nullptr;
     uint32_t *d_tickets = nullptr;
     if (err == cudaSuccess) err = configure_gemm_tc_kernel();
-    if (err == cudaSuccess) err = buf.alloc(&d_ws, gemm_tc_workspace_bytes(tokens, sms) / sizeof(float));
+    const uint32_t split_tokens = tokens < kGemmMaxTokens ? tokens : kGemmMaxTokens;  // more are never split
+    if (err == cudaSuccess) err = buf.alloc(&d_ws, gemm_tc_workspace_bytes(split_tokens, sms) / sizeof(float));
     if (err == cudaSuccess) err = buf.alloc(&d_tickets, static_cast<uint64_t>(gemm_tc_ticket_count(rows)) + 1u);
     if (err == cudaSuccess)
       err = cudaMemset(d_tickets, 0, (static_cast<uint64_t>(gemm_tc_ticket_count(rows)) + 1u) * sizeof(uint32_t));

@@ -191,8 +191,9 @@ struct BlockWorkspace {
   void *convolved = nullptr;    // [max_rows][convolved row] of a state-space layer
   uint16_t *ff = nullptr;       // [max_rows][intermediate]
   float *logits = nullptr;      // [sample_rows][vocab]
-  float *partial_acc = nullptr, *partial_m = nullptr, *partial_l = nullptr;  // split attention, per row
-  uint32_t *attn_tickets = nullptr;  // [max_rows][kv_heads]
+  uint32_t part_rows = 0;       // min(max_rows, kBlockPartRows)
+  float *partial_acc = nullptr, *partial_m = nullptr, *partial_l = nullptr;  // split attention, per row of a part
+  uint32_t *attn_tickets = nullptr;  // [part_rows][kv_heads]
   float *gemm_workspace = nullptr;
   uint32_t *gemm_tickets = nullptr;
   float *best_value = nullptr;  // [sample_rows][kBlockArgmaxChunks]
@@ -204,7 +205,12 @@ struct BlockWorkspace {
   uint32_t *head_rows = nullptr;  // [sample_rows] rows of the block whose logits are wanted
 };
 constexpr uint32_t kBlockArgmaxChunks = 64;
-constexpr uint32_t kBlockMaxRows = 256;       // one MMA N
+// Rows of a prefill chunk.  256 (one MMA N) made every chunk a weight stream; from about 2000 rows on the weights'
+// share of a projection's time is a tenth, and the activations of a chunk still fit the L2.
+constexpr uint32_t kBlockMaxRows = 2048;
+// Rows that have split-attention partials and stream-K workspace: launches over more rows take neither, or go in
+// parts of this many.  fp32 blocks are no larger.
+constexpr uint32_t kBlockPartRows = 256;
 constexpr uint32_t kBlockSampleRows = 32;     // sessions per packed decode step (hf_decode_sequence/types.cuh:63)
 
 // Device weights shared between a session and its forks.

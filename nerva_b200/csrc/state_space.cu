@@ -378,7 +378,7 @@ constexpr uint32_t kChunk = 64;
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanWarps = kScanThreads / 32u;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr uint32_t kScanMaxRows = 256;  // rows of a block
+constexpr uint32_t kScanMaxRows = 2048;  // rows of a block (24 KB of steps and decays)
 
 __device__ __forceinline__ void cp_async_16(void *dst, const void *src, bool valid) {  // zeros when not valid
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16u : 0u)
@@ -737,7 +737,7 @@ cudaError_t configure_state_space() {
   cudaError_t err = cudaSuccess;
   for (const void *kernel : {reinterpret_cast<const void *>(state_space_scan_kernel<1>),
                              reinterpret_cast<const void *>(state_space_scan_kernel<2>)})
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024);  // beside the static steps
   return err;
 }
 

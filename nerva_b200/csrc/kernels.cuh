@@ -466,8 +466,12 @@ cudaError_t configure_window_attention();
 cudaError_t launch_window_publish(cudaStream_t stream, const WindowAttentionParams &p);
 // One token per row: the lone decode step (rows == nullptr: prepares q and appends K/V itself) or block rows.
 cudaError_t launch_window_attention(cudaStream_t stream, const WindowAttentionParams &p);
-// Consecutive positions of one session on the tensor pipe (bf16 cache only).
+// Consecutive positions of one session on the tensor pipe (bf16 cache only): prefill_attention.cu where it takes the
+// shape and the rows fill it, mma.sync tiles otherwise.
 cudaError_t launch_window_prefill(cudaStream_t stream, const WindowAttentionParams &p);
+bool prefill_attention_supported(const WindowAttentionShape &s);
+cudaError_t configure_prefill_attention();
+cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p);
 
 // ---- state-space mixer (state_space.cu) ----
 // Per channel of x, B and C a causal convolution and silu, then per head h (group h / (heads / groups)) a state

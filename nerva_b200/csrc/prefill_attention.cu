@@ -1,0 +1,443 @@
+// Attention of a block of one session's rows (prefill chunk) on the fifth-generation tensor pipe.
+//
+// A block of threads takes 128 (position, head) rows of one KV head, so the heads that share a KV head share its keys,
+// and walks 128-key tiles up to the last row's own position:
+//   S = Q K^T      tcgen05.mma, Q and K in shared memory, S (fp32) in tensor memory
+//   P = exp2(S-m)  one thread per row: the row's 128 scores in registers, no exchange between threads
+//   O += P V       tcgen05.mma, P in tensor memory in the place of S, V in shared memory as it is cached (token-major:
+//                  the MMA takes it in the MN-major form), O (fp32) in tensor memory
+// Queries and probabilities are fp32 values; each enters as a bf16 rounding and its remainder, two MMAs into the same
+// accumulator, so a product loses only the rounding of the cached row (the contract of the other attention kernels).
+//
+// What bounds it: the tensor pipe, 4 x 512 MMA cycles per tile (two parts of Q, two of P), as long as the softmax of a
+// tile (about 8 instructions and one exponential for each of a thread's 128 scores) fits beside it.  S has two
+// buffers: S(j+1) is computed while the softmax works on S(j).  The output accumulator is rescaled only when a row's
+// maximum has grown by more than 2^8 since the reference it uses (the probabilities stay below 2^8, the sums exact
+// to fp32): after the first tiles that almost never happens.
+// One 128-row tile per block, not two in turn: with both parts of Q (64 KB) and two stages of K and V (128 KB) shared
+// memory is full, and tensor time already covers the softmax.
+//
+// Measured (whole prefill, 8B shapes, 8 layers; row by row through the decode kernel before): 3001 tokens 19.5 ms
+// (33.1), 12000 tokens 101.6 ms (279.1); vuvolix 1.7b, window 1024, 2048 tokens 18.6 ms (23.0 with mma.sync tiles).
+//
+// Roles (224 threads): warps 0..3 softmax, rescaling and the output (warp w reads tensor-memory lanes 32 w ..), warps
+// 4 and 5 copy K and V (cp.async, 16-byte pieces into the 128-byte swizzle; a 16-token page is a row range of a tile),
+// warp 6 issues the MMAs.  Tiles outside every row's window are never loaded.  Every wait is bounded; one that gives
+// up sets the error word and the block's abort flag, and all roles leave.
+#include "gemm_device.cuh"
+#include "mma_bf16.cuh"
+#include "window_device.cuh"
+
+namespace nb {
+namespace {
+
+constexpr uint32_t kRows = 128;      // (position, head) rows: the MMA M and the lanes of tensor memory
+constexpr uint32_t kKeys = 128;      // keys of a tile
+constexpr uint32_t kStages = 2;      // of K and of V, each freed on its own
+constexpr uint32_t kSoftmaxThreads = 128, kCopyThreads = 64;
+constexpr uint32_t kAttentionThreads = kSoftmaxThreads + kCopyThreads + 32u;
+constexpr uint32_t kMmaWarp = (kSoftmaxThreads + kCopyThreads) / 32u;
+constexpr uint32_t kBlockBytes = kRows * 128u;  // 128 rows of 64 bf16: one swizzled column block of a tile
+constexpr uint32_t kTmemS = 0, kTmemO = 2u * kKeys, kTmemAll = 512;
+constexpr float kRescaleAbove = 8.0f;
+
+struct AttentionShared {
+  uint64_t k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
+  uint64_t s_full[2], p_full[2];
+  uint64_t pv_done;  // PV(j): completes once per tile
+  uint64_t o_done;   // the last PV
+  uint32_t tmem_base;
+  uint32_t abort;
+};
+
+// 16-byte piece `piece` of row `row` of a tile whose 64-element column blocks follow each other.
+__device__ __forceinline__ uint32_t swizzled(uint32_t row, uint32_t piece) {
+  return (piece >> 3) * kBlockBytes + row * 128u + (((piece & 7u) ^ (row & 7u)) << 4);
+}
+// Descriptor of V for one MMA: 16 keys x D values stored [key][64 values] per column block; the 8-key groups are 1024
+// bytes apart, the column blocks kBlockBytes.
+__device__ __forceinline__ uint64_t mn_major_sw128_desc(const void *tile) {
+  const uint64_t addr = smem_addr(tile);
+  return ((addr & 0x3ffffull) >> 4) | (static_cast<uint64_t>(kBlockBytes >> 4) << 16) |
+         (static_cast<uint64_t>(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint32_t attention_instr_desc(uint32_t n, bool b_mn_major) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((n >> 3) << 17) | ((kRows >> 4) << 24);
+}
+// A from tensor memory (two bf16 per 32-bit column, a row per lane), B from shared memory.
+__device__ __forceinline__ void mma_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_load32(uint32_t taddr, float *v) {  // tmem_load_wait before the values are used
+  uint32_t *r = reinterpret_cast<uint32_t *>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t *r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::
+          "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// All lanes of a warp wait; false for all of them when one gave up.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort, uint32_t *error_word) {
+  return __all_sync(0xffffffffu, abortable_wait(bar, parity, abort, error_word));
+}
+
+template <uint32_t D, bool EXTRAS>
+__global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel(WindowAttentionParams p) {
+  constexpr uint32_t kColumnBlocks = D / 64u, kTileBytes = kColumnBlocks * kBlockBytes;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t{1023});
+  uint8_t *q_hi = smem, *q_lo = smem + kTileBytes;
+  uint8_t *k_ring = q_lo + kTileBytes, *v_ring = k_ring + kStages * kTileBytes;
+  AttentionShared &sh = *reinterpret_cast<AttentionShared *>(v_ring + kStages * kTileBytes);
+  volatile uint32_t *abort = &sh.abort;
+  const WindowAttentionShape &s = p.s;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (uint32_t i = 0; i < kStages; ++i) {
+      mbar_init(&sh.k_full[i], kCopyThreads);
+      mbar_init(&sh.v_full[i], kCopyThreads);
+      mbar_init(&sh.k_empty[i], 1);
+      mbar_init(&sh.v_empty[i], 1);
+    }
+    for (uint32_t i = 0; i < 2; ++i) {
+      mbar_init(&sh.s_full[i], 1);
+      mbar_init(&sh.p_full[i], kSoftmaxThreads);
+    }
+    mbar_init(&sh.pv_done, 1);
+    mbar_init(&sh.o_done, 1);
+    sh.abort = 0;
+    mbar_init_fence();
+  }
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)),
+                 "r"(kTmemAll)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_wait();
+  const FusedAttentionRow &r0 = p.rows[0];
+  const uint32_t group = s.heads / s.kv_heads, kvh = blockIdx.x;
+  const uint32_t total_rows = p.row_count * group;
+  const uint32_t f0 = (gridDim.y - 1u - blockIdx.y) * kRows;  // the longest walks first
+  const uint32_t f_end = f0 + kRows < total_rows ? f0 + kRows : total_rows;
+  const uint32_t base = r0.position;
+  const uint32_t pos_first = base + f0 / group, pos_last = base + (f_end - 1u) / group;
+  const bool inside = pos_last < r0.max_context;
+  const uint32_t window = s.window != 0 ? s.window : 0xffffffffu;
+  const uint32_t keep_first = EXTRAS ? s.keep_first : 0u;
+  const uint32_t window_lo = pos_first + 1u > window ? pos_first + 1u - window : 0u;  // of the first row
+  const uint32_t kv_end = pos_last + 1u;
+  const TileWalk walk(keep_first, window_lo, kKeys);
+  const uint32_t tiles = inside ? walk.count(kv_end, kKeys) : 0u;
+
+  // queries, scaled so that the softmax runs on exp2, as a bf16 rounding and its remainder
+  if (inside && warp < kMmaWarp) {
+    const float qscale = s.scale * kLog2e;
+    const bool whole_pieces = s.qk_dim == D && p.qkv_stride % 4u == 0 && reinterpret_cast<uintptr_t>(p.qkv) % 16u == 0;
+    for (uint32_t i = threadIdx.x; i < kRows * (D / 8u); i += kSoftmaxThreads + kCopyThreads) {
+      const uint32_t row = i / (D / 8u), piece = i % (D / 8u), f = f0 + row;
+      float x[8];
+#pragma unroll
+      for (uint32_t j = 0; j < 8u; ++j) x[j] = 0.0f;
+      if (f < f_end) {
+        const float *src = p.qkv + static_cast<uint64_t>(f / group) * p.qkv_stride + (kvh * group + f % group) * s.qk_dim;
+        if (whole_pieces) {
+          const float4 a = __ldcg(reinterpret_cast<const float4 *>(src + piece * 8u));
+          const float4 b = __ldcg(reinterpret_cast<const float4 *>(src + piece * 8u + 4u));
+          x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+        } else {
+#pragma unroll
+          for (uint32_t j = 0; j < 8u; ++j) x[j] = piece * 8u + j < s.qk_dim ? __ldcg(src + piece * 8u + j) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; ++j) x[j] *= qscale;
+      }
+      const uint32_t at = swizzled(row, piece);
+      *reinterpret_cast<uint4 *>(q_hi + at) =
+          make_uint4(pack_bf16_hi(x[0], x[1]), pack_bf16_hi(x[2], x[3]), pack_bf16_hi(x[4], x[5]), pack_bf16_hi(x[6], x[7]));
+      *reinterpret_cast<uint4 *>(q_lo + at) =
+          make_uint4(pack_bf16_lo(x[0], x[1]), pack_bf16_lo(x[2], x[3]), pack_bf16_lo(x[4], x[5]), pack_bf16_lo(x[6], x[7]));
+    }
+    fence_proxy_async();
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem = sh.tmem_base;
+
+  if (warp == kMmaWarp) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0 && tiles != 0) {
+      const uint32_t idesc_s = attention_instr_desc(kKeys, false), idesc_o = attention_instr_desc(D, true);
+      auto scores = [&](uint32_t j) {  // S(j) = Q K(j)^T; its buffer held P(j - 2), which PV(j - 2) has read
+        const uint32_t st = j % kStages;
+        if (!abortable_wait(&sh.k_full[st], (j / kStages) & 1u, abort, r0.error_word)) return false;
+        if (j >= 2u && !abortable_wait(&sh.pv_done, j & 1u, abort, r0.error_word)) return false;
+        tcgen05_fence_after();
+        const uint8_t *k = k_ring + st * kTileBytes;
+#pragma unroll
+        for (uint32_t part = 0; part < 2u; ++part) {
+          const uint8_t *q = part == 0 ? q_hi : q_lo;
+#pragma unroll
+          for (uint32_t ks = 0; ks < D / kUmmaK; ++ks) {
+            const uint64_t at = (ks & 3u) * 2ull;
+            tcgen05_mma_f16(tmem + kTmemS + (j & 1u) * kKeys, kmajor_sw128_desc(q + (ks >> 2) * kBlockBytes) + at,
+                            kmajor_sw128_desc(k + (ks >> 2) * kBlockBytes) + at, idesc_s, (part != 0 || ks != 0) ? 1u : 0u);
+          }
+        }
+        tcgen05_commit(&sh.k_empty[st]);
+        tcgen05_commit(&sh.s_full[j & 1u]);
+        return true;
+      };
+      bool ok = scores(0);
+      for (uint32_t j = 0; ok && j < tiles; ++j) {
+        if (j + 1u < tiles && !scores(j + 1u)) break;
+        const uint32_t st = j % kStages;
+        if (!abortable_wait(&sh.v_full[st], (j / kStages) & 1u, abort, r0.error_word)) break;
+        if (!abortable_wait(&sh.p_full[j & 1u], (j >> 1) & 1u, abort, r0.error_word)) break;
+        tcgen05_fence_after();
+        const uint64_t v = mn_major_sw128_desc(v_ring + st * kTileBytes);
+#pragma unroll
+        for (uint32_t part = 0; part < 2u; ++part) {
+#pragma unroll
+          for (uint32_t ks = 0; ks < kKeys / kUmmaK; ++ks)
+            mma_tmem_a(tmem + kTmemO, tmem + kTmemS + (j & 1u) * kKeys + part * (kKeys / 2u) + ks * (kUmmaK / 2u),
+                       v + ks * ((kUmmaK * 128u) >> 4), idesc_o, (j != 0 || part != 0 || ks != 0) ? 1u : 0u);
+        }
+        tcgen05_commit(&sh.v_empty[st]);
+        tcgen05_commit(&sh.pv_done);
+        if (j + 1u == tiles) tcgen05_commit(&sh.o_done);
+      }
+    }
+  } else if (warp >= 4u) {
+    // ---------------- K and V ----------------
+    const uint32_t copy_warp = warp - 4u;
+    const uint16_t *keys = r0.key_pages + p.key_offset, *values = r0.value_pages + p.value_offset;
+    uint32_t issued = 0, signalled = 0;  // items: K(0), V(0), K(1), V(1), ...
+    auto signal_to = [&](uint32_t end) {
+      if (signalled < end) fence_proxy_async();
+      for (; signalled < end; ++signalled) {
+        const uint32_t st = (signalled >> 1) % kStages;
+        mbar_arrive((signalled & 1u) == 0 ? &sh.k_full[st] : &sh.v_full[st]);
+      }
+    };
+    bool ok = true;
+    for (uint32_t j = 0; ok && j < tiles; ++j) {
+      const uint32_t first = walk.tile(j) * kKeys, st = j % kStages;
+      uint32_t my_page = 0;
+      if (lane < kKeys / kPageTokens && first + lane * kPageTokens < kv_end) {
+        my_page = r0.page_table[first / kPageTokens + lane];
+        if (my_page >= r0.page_count) {
+          report_error(r0.error_word, kErrPageOutOfRange);
+          my_page = 0;
+        }
+      }
+#pragma unroll 1
+      for (uint32_t what = 0; what < 2u; ++what) {
+        uint64_t *empty = what == 0 ? &sh.k_empty[st] : &sh.v_empty[st];
+        const uint32_t parity = ((j / kStages) & 1u) ^ 1u;
+        if (!__all_sync(0xffffffffu, mbar_try_wait(empty, parity))) {
+          cp_async_wait<0>();  // nothing more to issue for now: hand over what is on its way
+          signal_to(issued);
+          if (!warp_wait(empty, parity, abort, r0.error_word)) {
+            ok = false;
+            break;
+          }
+        }
+        uint8_t *stage = (what == 0 ? k_ring : v_ring) + st * kTileBytes;
+        const uint16_t *from = what == 0 ? keys : values;
+        // a warp copies whole rows: D / 8 pieces each
+#pragma unroll
+        for (uint32_t i = 0; i < kKeys * (D / 8u) / kCopyThreads; ++i) {
+          constexpr uint32_t kPerWarp = 32u / (D / 8u);  // rows a warp copies at once
+          const uint32_t row = (i * (kCopyThreads / 32u) + copy_warp) * kPerWarp + lane / (D / 8u), piece = lane % (D / 8u);
+          const uint32_t page = __shfl_sync(0xffffffffu, my_page, row / kPageTokens);
+          const bool valid = first + row < kv_end;  // rows behind the last query are filled with zeros
+          const uint16_t *src = from + (valid ? cache_row(page, first + row, s.kv_heads, kvh, D) + piece * 8u : 0u);
+          cp_async_zfill<16>(stage + swizzled(row, piece), src, valid);
+        }
+        cp_async_commit();
+        issued += 1;
+        cp_async_wait<2>();
+        if (issued > 2u) signal_to(issued - 2u);
+      }
+    }
+    cp_async_wait<0>();
+    signal_to(issued);
+  } else if (tiles != 0) {
+    // ---------------- softmax ----------------
+    const uint32_t f = f0 + threadIdx.x;
+    const bool live = f < f_end;
+    const uint32_t pos = base + (live ? f : f_end - 1u) / group;
+    const uint32_t lanes = (warp * 32u) << 16;
+    const float cap2 = s.softcap * kLog2e, inv_cap2 = cap2 > 0.0f ? 1.0f / cap2 : 0.0f;
+    float m_ref = -INFINITY, l = 0.0f;
+    bool ok = true;
+    for (uint32_t j = 0; j < tiles; ++j) {
+      const uint32_t first = walk.tile(j) * kKeys;
+      if (!warp_wait(&sh.s_full[j & 1u], (j >> 1) & 1u, abort, r0.error_word)) {
+        ok = false;
+        break;
+      }
+      tcgen05_fence_after();
+      const uint32_t s_addr = tmem + lanes + kTmemS + (j & 1u) * kKeys;
+      float v[kKeys];
+#pragma unroll
+      for (uint32_t c = 0; c < kKeys; c += 32u) tmem_load32(s_addr + c, v + c);
+      tmem_load_wait();
+#pragma unroll
+      for (uint32_t c = 0; c < kKeys; ++c) asm volatile("" : "+f"(v[c]));  // nothing that uses a score moves above the wait
+      if (EXTRAS && cap2 > 0.0f) {
+#pragma unroll
+        for (uint32_t c = 0; c < kKeys; ++c) v[c] = cap_score_fast(v[c], cap2, inv_cap2);
+      }
+      // visible: 0 <= pos - key, and pos - key < window or key < keep_first; only tiles at an edge test it
+      if (first + kKeys > pos_first + 1u || (EXTRAS && first < keep_first) || pos_last - first >= window) {
+#pragma unroll
+        for (uint32_t c = 0; c < kKeys; ++c) {
+          const uint32_t key = first + c;
+          if (!(key <= pos && (pos - key < window || (EXTRAS && key < keep_first)))) v[c] = -INFINITY;
+        }
+      }
+      float top[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+      for (uint32_t c = 4; c < kKeys; ++c) top[c & 3u] = fmaxf(top[c & 3u], v[c]);
+      const float m_tile = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+      // the accumulator keeps its reference until the maximum has left it far behind
+      const bool grow = m_tile > m_ref + kRescaleAbove;  // also the first visible key: m_ref is -inf
+      if (__any_sync(0xffffffffu, grow)) {
+        const float m_new = grow ? m_tile : m_ref;
+        const float corr = m_new == m_ref ? 1.0f : exp2_ftz(m_ref - m_new);  // 0 where nothing was seen before
+        m_ref = m_new;
+        l *= corr;
+        if (j != 0) {
+          // PV(j - 2) is done (S(j) followed it) and PV(j) waits for this warp: the parity is that of PV(j - 1)
+          if (!warp_wait(&sh.pv_done, (j - 1u) & 1u, abort, r0.error_word)) {
+            ok = false;
+            break;
+          }
+          tcgen05_fence_after();
+#pragma unroll 1
+          for (uint32_t c = 0; c < D; c += 16u) {
+            float o[16];
+            tmem_load16(tmem + lanes + kTmemO + c, o);
+#pragma unroll
+            for (uint32_t i = 0; i < 16u; ++i) o[i] *= corr;
+            tmem_store16(tmem + lanes + kTmemO + c, reinterpret_cast<const uint32_t *>(o));
+          }
+        }
+      }
+      const float ref = m_ref == -INFINITY ? 0.0f : m_ref;  // no key of the row seen yet: all probabilities are 0
+      float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (uint32_t c = 0; c < kKeys; c += 32u) {
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) {
+          const float a = exp2_ftz(v[c + 2u * i] - ref), b = exp2_ftz(v[c + 2u * i + 1u] - ref);
+          sum[i & 1u] += a;
+          sum[2u + (i & 1u)] += b;
+          hi[i] = pack_bf16_hi(a, b);
+          lo[i] = pack_bf16_hi(a - bf16x2_lo(hi[i]), b - bf16x2_hi(hi[i]));
+        }
+        tmem_store16(s_addr + c / 2u, hi);
+        tmem_store16(s_addr + kKeys / 2u + c / 2u, lo);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      tmem_store_wait();
+      tcgen05_fence_before();
+      mbar_arrive(&sh.p_full[j & 1u]);
+    }
+    if (ok && warp_wait(&sh.o_done, 0, abort, r0.error_word)) {
+      tcgen05_fence_after();
+      const uint32_t h = kvh * group + f % group;
+      const float inv = live ? output_gate<EXTRAS>(p, f / group, h) / l : 0.0f;
+      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + static_cast<uint64_t>(f / group) * p.out_stride + h * s.v_dim;
+      const bool vector = s.v_dim == D && p.out_stride % 8u == 0 && reinterpret_cast<uintptr_t>(p.out) % 16u == 0;
+#pragma unroll 1
+      for (uint32_t c = 0; c < D; c += 16u) {
+        float o[16];
+        tmem_load16(tmem + lanes + kTmemO + c, o);
+        if (!live) continue;
+        if (vector) {
+#pragma unroll
+          for (uint32_t i = 0; i < 16u; i += 8u)
+            *reinterpret_cast<uint4 *>(dst + c + i) =
+                make_uint4(pack_bf16_hi(o[i] * inv, o[i + 1] * inv), pack_bf16_hi(o[i + 2] * inv, o[i + 3] * inv),
+                           pack_bf16_hi(o[i + 4] * inv, o[i + 5] * inv), pack_bf16_hi(o[i + 6] * inv, o[i + 7] * inv));
+        } else {
+#pragma unroll
+          for (uint32_t i = 0; i < 16u; ++i)
+            if (c + i < s.v_dim) dst[c + i] = f32_to_bf16_bits(o[i] * inv);
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemAll) : "memory");
+  }
+}
+
+template <uint32_t D>
+constexpr uint32_t attention_smem() {
+  return 1024u + (2u + 2u * kStages) * (D / 64u) * kBlockBytes + static_cast<uint32_t>(sizeof(AttentionShared)) + 64u;
+}
+
+}  // namespace
+
+bool prefill_attention_supported(const WindowAttentionShape &s) {
+  return s.heads % s.kv_heads == 0 && s.qk_pad == s.v_pad && (s.qk_pad == 64u || s.qk_pad == 128u);
+}
+
+cudaError_t configure_prefill_attention() {
+  cudaError_t err = cudaSuccess;
+  auto set = [&err](void (*kernel)(WindowAttentionParams), uint32_t bytes) {
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  };
+  set(prefill_attention_kernel<64, false>, attention_smem<64>());
+  set(prefill_attention_kernel<64, true>, attention_smem<64>());
+  set(prefill_attention_kernel<128, false>, attention_smem<128>());
+  set(prefill_attention_kernel<128, true>, attention_smem<128>());
+  return err;
+}
+
+cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p) {
+  if (p.rows == nullptr || p.row_count == 0 || p.f32 != 0 || !prefill_attention_supported(p.s)) return cudaErrorInvalidValue;
+  const uint32_t rows = p.row_count * (p.s.heads / p.s.kv_heads);
+  const dim3 grid(p.s.kv_heads, (rows + kRows - 1u) / kRows);
+  const bool extras = has_extras(p.s);
+  if (p.s.qk_pad == 64u)
+    return launch_with_pdl(extras ? prefill_attention_kernel<64, true> : prefill_attention_kernel<64, false>, grid,
+                           dim3(kAttentionThreads), attention_smem<64>(), stream, p.pdl != 0, p);
+  return launch_with_pdl(extras ? prefill_attention_kernel<128, true> : prefill_attention_kernel<128, false>, grid,
+                         dim3(kAttentionThreads), attention_smem<128>(), stream, p.pdl != 0, p);
+}
+
+}  // namespace nb

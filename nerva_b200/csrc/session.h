@@ -199,6 +199,7 @@ struct BlockWorkspace {
   float *best_value = nullptr;  // [sample_rows][kBlockArgmaxChunks]
   uint32_t *best_index = nullptr;
   FusedAttentionRow *attn_rows = nullptr;  // [max_rows] device copies of the row descriptors
+  bool tile_prefill = false;    // a prefill chunk's attention may run on prefill_attention.cu
   bool paged_rows = false;      // the rows' attention runs on the paged tensor-pipe kernel (attention.cu)
   BlockTokenRow *token_rows = nullptr;
   BlockSampleRow *sample_rows_dev = nullptr;  // [sample_rows] device copies of the sampler's row descriptors

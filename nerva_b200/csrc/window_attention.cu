@@ -21,33 +21,16 @@
 //                             cached row.  Only tiles that meet some row's window are loaded.
 #include <math.h>
 
-#include "common.cuh"
-#include "kernels.cuh"
 #include "mma_bf16.cuh"
+#include "window_device.cuh"
 
 namespace nb {
 namespace {
 
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr uint32_t kPageTokens = NERVA_KV_CACHE_BLOCK_TOKENS;
 constexpr uint32_t kTile = 32;             // tokens of one score tile: one per lane
 constexpr uint32_t kWarps = 8;             // of a window_attention_kernel block
 constexpr uint32_t kHeadsPerBlock = 8;
 constexpr uint32_t kMaxSmem = 227u * 1024u;
-
-template <uint32_t BYTES>
-__device__ __forceinline__ void cp_async_zfill(void *dst, const void *src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? BYTES : 0u)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 __device__ __forceinline__ void to_cache(float *dst, float v) { *dst = v; }
 __device__ __forceinline__ void to_cache(uint16_t *dst, float v) { *dst = f32_to_bf16_bits(v); }
@@ -79,44 +62,8 @@ __device__ __forceinline__ float dot_piece(const uint16_t *k, const float *q, fl
   return fmaf(bf16x2_hi(w.w), b.w, acc);
 }
 
-// The tiles of `size` tokens a query walks: those that hold kept first positions and lie in front of the
-// window, then the window's.
-struct TileWalk {
-  uint32_t kept, first;  // tiles in front; first tile of the window
-  __device__ __forceinline__ TileWalk(uint32_t keep_first, uint32_t lo, uint32_t size) {
-    first = lo / size;
-    kept = (keep_first + size - 1u) / size;
-    if (kept > first) kept = first;
-  }
-  __device__ __forceinline__ uint32_t count(uint32_t end, uint32_t size) const {  // tiles, for a window that ends at `end`
-    return kept + (end + size - 1u) / size - first;
-  }
-  __device__ __forceinline__ uint32_t tile(uint32_t i) const { return i < kept ? i : first + (i - kept); }
-};
-
-// EXTRAS of the kernels below: kept first positions, score cap and output gates.  Without them the code
-// is the plain window's.
-__host__ __device__ inline bool has_extras(const WindowAttentionShape &s) {
-  return s.keep_first != 0 || s.softcap > 0.0f || s.head_gate != 0;
-}
-
 // Soft cap of a score that carries a factor log2(e).
 __device__ __forceinline__ float cap_score(float score, float cap2) { return cap2 * tanhf(score / cap2); }
-// The same through one exponential, absolute error a few 1e-7 of the cap.
-__device__ __forceinline__ float cap_score_fast(float score, float cap2, float inv_cap2) {
-  const float e = exp2f(score * inv_cap2 * (2.0f * kLog2e));
-  return cap2 - __fdividef(2.0f * cap2, e + 1.0f);
-}
-
-// Factor of a head's output.
-template <bool EXTRAS>
-__device__ __forceinline__ float output_gate(const WindowAttentionParams &p, uint32_t row, uint32_t h) {
-  const WindowAttentionShape &s = p.s;
-  if (!EXTRAS || s.head_gate == 0) return 1.0f;
-  const uint32_t at = (s.heads + s.kv_heads) * s.qk_dim + s.kv_heads * s.v_dim + h;
-  return sigmoid(__ldcg(p.qkv + static_cast<uint64_t>(row) * p.qkv_stride + at));
-}
-
 // (sin, cos) of pair i at a position, with the magnitude of a scaled rotation.
 __device__ __forceinline__ float2 rotation(const WindowAttentionShape &s, uint32_t position, uint32_t i) {
   float2 t;
@@ -146,11 +93,6 @@ __device__ __forceinline__ void rotate_and_norm(float *v, const WindowAttentionS
   const float scale = 1.0f / sqrtf(sumsq / static_cast<float>(s.qk_dim) + s.eps);
   for (uint32_t i = lane; i < s.qk_dim; i += 32u) v[i] *= scale;
   __syncwarp();
-}
-
-// Cached row (page, slot) of a KV head, in elements of a row of `width` per head.
-__device__ __forceinline__ uint64_t cache_row(uint32_t page, uint32_t token, uint32_t kv_heads, uint32_t kvh, uint32_t width) {
-  return ((static_cast<uint64_t>(page) * kPageTokens + token % kPageTokens) * kv_heads + kvh) * width;
 }
 
 // Grid ((heads + kv_heads) / 8, rows), a warp per head: a query head is prepared in place, a KV head's K
@@ -1172,7 +1114,7 @@ uint32_t window_rows_splits(const WindowAttentionShape &s, uint32_t rows, uint32
 }
 
 cudaError_t configure_window_attention() {
-  cudaError_t err = cudaSuccess;
+  cudaError_t err = configure_prefill_attention();
   auto set = [&](const void *kernel) {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem - 2048u));
@@ -1217,6 +1159,8 @@ cudaError_t launch_window_attention(cudaStream_t stream, const WindowAttentionPa
 cudaError_t launch_window_prefill(cudaStream_t stream, const WindowAttentionParams &p) {
   if (p.rows == nullptr || p.row_count == 0 || p.f32 != 0) return cudaErrorInvalidValue;
   const uint32_t rows = p.row_count * (p.s.heads / p.s.kv_heads);
+  // the shapes it takes, it takes at every size: 8 to 33 rows are equal within 2%, from 256 rows on it is ahead
+  if (prefill_attention_supported(p.s)) return launch_prefill_attention(stream, p);
   const dim3 grid((rows + kTileRows - 1u) / kTileRows, p.s.kv_heads);
   const uint32_t groups = prefill_groups(p.s);
   const uint32_t bytes = PrefillLayout(p.s, groups).total;

@@ -75,70 +75,76 @@ __global__ void __launch_bounds__(kNormThreads) block_norm_kernel(const float *h
   norm_single_finish(x + static_cast<uint64_t>(blockIdx.x) * x_stride, values, weights, eps, cols, scratch);
 }
 
-// Prefill: K (k-norm + RoPE) and V of every row of the chunk, rounded to bf16, into the row's page.
-// One warp per (KV head, row); the same functions, in the same order, as the decode step's append
-// (attention_fused.cu), so the cached bits are those the decode step would have written.
-// Blocks beyond the KV heads (the grid has kv_heads + heads of them per row when prepare_q is set)
-// do the query side for the paged attention kernel: bias, q-norm and RoPE of one query head, written
-// back in place as fp32 (that kernel reads its queries ready-made).
+// K (k-norm + RoPE) and V of every row of the block, rounded to bf16, into the row's page: the same functions, in the
+// same order, as the decode step's append (attention_fused.cu), so the cached bits are those the decode step would have
+// written.  With query_heads != 0 also the query side, for the attention kernels that read their queries ready-made:
+// bias, q-norm and RoPE of each query head, written back in place as fp32.
+// Grid (groups of heads, rows), a warp per head in turn.  The angles of a row are computed once per warp and not once
+// per head: with a block of one warp per (head, row) the launch took 87 us for 2048 rows x 40 heads, most of it
+// sine and power functions and block starts.
+constexpr uint32_t kPublishWarps = 8;
 template <uint32_t PER>
-__global__ void block_kv_publish_kernel(const FusedAttentionRow *rows, uint32_t layer, uint32_t heads, uint32_t kv_heads,
-                                        const uint16_t *k_bias, const uint16_t *v_bias, const uint16_t *k_norm,
-                                        const uint16_t *q_bias, const uint16_t *q_norm, float eps, float rope_theta) {
+__global__ void __launch_bounds__(kPublishWarps * 32)
+block_kv_publish_kernel(const FusedAttentionRow *rows, uint32_t layer, uint32_t heads, uint32_t query_heads, uint32_t kv_heads,
+                        const uint16_t *k_bias, const uint16_t *v_bias, const uint16_t *k_norm, const uint16_t *q_bias,
+                        const uint16_t *q_norm, float eps, float rope_theta) {
   constexpr uint32_t D = PER * 32u;
   pdl_trigger();
   const FusedAttentionRow r = rows[blockIdx.y];
   const uint32_t lane = threadIdx.x & 31u;
-  const bool query = blockIdx.x >= kv_heads;
-  const uint32_t kvh = blockIdx.x;
   const uint32_t attention_hidden = heads * D, kv_hidden = kv_heads * D;
-  const uint16_t *norm = query ? q_norm : k_norm;
-  float norm_w[PER];
+  float k_norm_w[PER], q_norm_w[PER];
 #pragma unroll
-  for (uint32_t k = 0; k < PER; ++k) norm_w[k] = norm != nullptr ? bf16_bits_to_f32(norm[lane + 32u * k]) : 1.0f;
+  for (uint32_t k = 0; k < PER; ++k) {
+    k_norm_w[k] = k_norm != nullptr ? bf16_bits_to_f32(k_norm[lane + 32u * k]) : 1.0f;
+    q_norm_w[k] = q_norm != nullptr ? bf16_bits_to_f32(q_norm[lane + 32u * k]) : 1.0f;
+  }
   RopeFactors<PER> rope;
   rope_factors<PER>(rope, rope_theta, r.position);
   pdl_wait();
   if (r.position >= r.max_context) return;
-  if (query) {
-    const uint32_t h = blockIdx.x - kv_heads;
-    float *q = const_cast<float *>(r.qkv) + h * D;  // the row's projection output is scratch of the block step
-    float qn[PER];
+  const uint32_t page = r.page_table[r.position / NERVA_KV_CACHE_BLOCK_TOKENS];
+  const bool cached = page < r.page_count;
+  if (!cached) report_error(r.error_word, kErrPageOutOfRange);
+  for (uint32_t unit = blockIdx.x * kPublishWarps + (threadIdx.x >> 5); unit < kv_heads + query_heads;
+       unit += gridDim.x * kPublishWarps) {
+    if (unit >= kv_heads) {
+      const uint32_t h = unit - kv_heads;
+      float *q = const_cast<float *>(r.qkv) + h * D;  // the row's projection output is scratch of the block step
+      float qn[PER];
+#pragma unroll
+      for (uint32_t k = 0; k < PER; ++k) {
+        const uint32_t e = lane + 32u * k;
+        qn[k] = __ldcg(q + e);
+        if (q_bias != nullptr) qn[k] += bf16_bits_to_f32(q_bias[h * D + e]);
+      }
+      head_norm_rope_pre<PER>(qn, q_norm != nullptr, q_norm_w, eps, rope);
+#pragma unroll
+      for (uint32_t k = 0; k < PER; ++k) q[lane + 32u * k] = qn[k];
+      continue;
+    }
+    const uint32_t kvh = unit;
+    float kn[PER], vn[PER];
 #pragma unroll
     for (uint32_t k = 0; k < PER; ++k) {
       const uint32_t e = lane + 32u * k;
-      qn[k] = __ldcg(q + e);
-      if (q_bias != nullptr) qn[k] += bf16_bits_to_f32(q_bias[h * D + e]);
+      kn[k] = __ldcg(r.qkv + attention_hidden + kvh * D + e);
+      vn[k] = __ldcg(r.qkv + attention_hidden + kv_hidden + kvh * D + e);
+      if (k_bias != nullptr) kn[k] += bf16_bits_to_f32(k_bias[kvh * D + e]);
+      if (v_bias != nullptr) vn[k] += bf16_bits_to_f32(v_bias[kvh * D + e]);
     }
-    head_norm_rope_pre<PER>(qn, q_norm != nullptr, norm_w, eps, rope);
+    head_norm_rope_pre<PER>(kn, k_norm != nullptr, k_norm_w, eps, rope);
+    if (!cached) continue;
+    // hf_decode_sequence/types.cuh:328-337
+    const uint64_t base = layer * r.kv_layer_elems +
+                          (static_cast<uint64_t>(page) * NERVA_KV_CACHE_BLOCK_TOKENS +
+                           r.position % NERVA_KV_CACHE_BLOCK_TOKENS) * kv_hidden + kvh * D;
 #pragma unroll
-    for (uint32_t k = 0; k < PER; ++k) q[lane + 32u * k] = qn[k];
-    return;
-  }
-  float kn[PER], vn[PER];
-#pragma unroll
-  for (uint32_t k = 0; k < PER; ++k) {
-    const uint32_t e = lane + 32u * k;
-    kn[k] = __ldcg(r.qkv + attention_hidden + kvh * D + e);
-    vn[k] = __ldcg(r.qkv + attention_hidden + kv_hidden + kvh * D + e);
-    if (k_bias != nullptr) kn[k] += bf16_bits_to_f32(k_bias[kvh * D + e]);
-    if (v_bias != nullptr) vn[k] += bf16_bits_to_f32(v_bias[kvh * D + e]);
-  }
-  head_norm_rope_pre<PER>(kn, k_norm != nullptr, norm_w, eps, rope);
-  uint32_t page = r.page_table[r.position / NERVA_KV_CACHE_BLOCK_TOKENS];
-  if (page >= r.page_count) {
-    report_error(r.error_word, kErrPageOutOfRange);
-    return;
-  }
-  // hf_decode_sequence/types.cuh:328-337
-  const uint64_t base = layer * r.kv_layer_elems +
-                        (static_cast<uint64_t>(page) * NERVA_KV_CACHE_BLOCK_TOKENS +
-                         r.position % NERVA_KV_CACHE_BLOCK_TOKENS) * kv_hidden + kvh * D;
-#pragma unroll
-  for (uint32_t k = 0; k < PER; ++k) {
-    const uint32_t e = lane + 32u * k;
-    r.key_pages[base + e] = f32_to_bf16_bits(kn[k]);
-    r.value_pages[base + e] = f32_to_bf16_bits(vn[k]);
+    for (uint32_t k = 0; k < PER; ++k) {
+      const uint32_t e = lane + 32u * k;
+      r.key_pages[base + e] = f32_to_bf16_bits(kn[k]);
+      r.value_pages[base + e] = f32_to_bf16_bits(vn[k]);
+    }
   }
 }
 
@@ -330,15 +336,14 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
     const bool tiles = b.publish && ws.tile_prefill && b.rows >= kTilePrefillMinRows;
     const bool paged = !tiles && !b.k_maps.empty();
     if (err == cudaSuccess && (b.publish || paged)) {
-      const dim3 grid(d.kv_heads + (tiles || paged ? d.heads : 0u), b.rows);
-      if (d.head_dim == 128)
-        err = launch_with_pdl(block_kv_publish_kernel<4>, grid, dim3(32), 0, b.stream, b.pdl, ws.attn_rows, l, d.heads,
-                              d.kv_heads, arena_at(s, L.k_bias), arena_at(s, L.v_bias), arena_at(s, L.k_norm),
-                              arena_at(s, L.q_bias), arena_at(s, L.q_norm), s->rms_eps, s->rope_theta);
-      else
-        err = launch_with_pdl(block_kv_publish_kernel<2>, grid, dim3(32), 0, b.stream, b.pdl, ws.attn_rows, l, d.heads,
-                              d.kv_heads, arena_at(s, L.k_bias), arena_at(s, L.v_bias), arena_at(s, L.k_norm),
-                              arena_at(s, L.q_bias), arena_at(s, L.q_norm), s->rms_eps, s->rope_theta);
+      // few rows: a head per warp; many: all heads of a row in one block
+      const uint32_t query_heads = tiles || paged ? d.heads : 0u;
+      const uint32_t groups = (d.kv_heads + query_heads + kPublishWarps - 1u) / kPublishWarps;
+      const dim3 grid(b.rows >= kTilePrefillMinRows ? 1u : groups, b.rows);
+      auto publish = d.head_dim == 128 ? block_kv_publish_kernel<4> : block_kv_publish_kernel<2>;
+      err = launch_with_pdl(publish, grid, dim3(kPublishWarps * 32), 0, b.stream, b.pdl, ws.attn_rows, l, d.heads,
+                            query_heads, d.kv_heads, arena_at(s, L.k_bias), arena_at(s, L.v_bias), arena_at(s, L.k_norm),
+                            arena_at(s, L.q_bias), arena_at(s, L.q_norm), s->rms_eps, s->rope_theta);
       n += 1;
     }
     if (err != cudaSuccess) break;
@@ -353,6 +358,9 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       wp.out = ws.attn;
       wp.out_stride = ah;
       wp.key_offset = wp.value_offset = l * s->kv_layer_elems;
+      wp.keys = s->kv_keys;
+      wp.values = s->kv_values;
+      wp.page_count = s->kv_pages;
       wp.rows = ws.attn_rows;
       wp.row_count = b.rows;
       wp.pdl = b.pdl ? 1u : 0u;

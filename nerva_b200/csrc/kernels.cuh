@@ -471,6 +471,7 @@ cudaError_t launch_window_attention(cudaStream_t stream, const WindowAttentionPa
 cudaError_t launch_window_prefill(cudaStream_t stream, const WindowAttentionParams &p);
 bool prefill_attention_supported(const WindowAttentionShape &s);
 cudaError_t configure_prefill_attention();
+// p.keys, p.values and p.page_count name the session's cache, as for one token.
 cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p);
 
 // ---- state-space mixer (state_space.cu) ----

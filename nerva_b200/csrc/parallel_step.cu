@@ -399,6 +399,9 @@ cudaError_t enqueue_block_attention(Session *s, const ParallelBlock &b, const Pa
   a.tickets = ws.attn_tickets;
   a.rows = ws.attn_rows;
   a.row_count = b.rows;
+  a.keys = s->kv_keys;  // of the one session whose rows a prefill block holds
+  a.values = s->kv_values;
+  a.page_count = s->kv_pages;
   *launches += 2;
   const cudaError_t err = launch_window_publish(b.stream, a);
   if (err != cudaSuccess) return err;

@@ -14,16 +14,19 @@
 // buffers: S(j+1) is computed while the softmax works on S(j).  The output accumulator is rescaled only when a row's
 // maximum has grown by more than 2^8 since the reference it uses (the probabilities stay below 2^8, the sums exact
 // to fp32): after the first tiles that almost never happens.
-// One 128-row tile per block, not two in turn: with both parts of Q (64 KB) and two stages of K and V (128 KB) shared
-// memory is full, and tensor time already covers the softmax.
+// One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), but two
+// groups of softmax warps, each with every second tile, a running maximum, a sum and an output accumulator of its own,
+// added at the end: a tile's softmax is a chain of about 6000 cycles for one warp per scheduler, which one group could
+// not hide behind 2048 cycles of MMA (2048 tokens, 32 heads: 117 us with one group).
 //
 // Measured (whole prefill, 8B shapes, 8 layers; row by row through the decode kernel before): 3001 tokens 19.5 ms
 // (33.1), 12000 tokens 101.6 ms (279.1); vuvolix 1.7b, window 1024, 2048 tokens 18.6 ms (23.0 with mma.sync tiles).
 //
-// Roles (224 threads): warps 0..3 softmax, rescaling and the output (warp w reads tensor-memory lanes 32 w ..), warps
-// 4 and 5 copy K and V (cp.async, 16-byte pieces into the 128-byte swizzle; a 16-token page is a row range of a tile),
-// warp 6 issues the MMAs.  Tiles outside every row's window are never loaded.  Every wait is bounded; one that gives
-// up sets the error word and the block's abort flag, and all roles leave.
+// Roles (320 threads): warps 0..3 and 4..7 softmax, rescaling and the output (warp w reads tensor-memory lanes
+// 32 (w % 4) ..), warp 8 brings K and V (one 2-D TMA box per page and 64 columns, 128-byte swizzle), warp 9 issues the MMAs.  (cp.async by
+// two warps instead of TMA: their 1800 instructions per tile took 10,700 cycles, five times the MMAs.)  Tiles outside
+// every row's window are never loaded.  Every wait is bounded; one that gives up sets the error word and the block's
+// abort flag, and all roles leave.
 #include "gemm_device.cuh"
 #include "mma_bf16.cuh"
 #include "window_device.cuh"
@@ -34,9 +37,9 @@ namespace {
 constexpr uint32_t kRows = 128;      // (position, head) rows: the MMA M and the lanes of tensor memory
 constexpr uint32_t kKeys = 128;      // keys of a tile
 constexpr uint32_t kStages = 2;      // of K and of V, each freed on its own
-constexpr uint32_t kSoftmaxThreads = 128, kCopyThreads = 64;
-constexpr uint32_t kAttentionThreads = kSoftmaxThreads + kCopyThreads + 32u;
-constexpr uint32_t kMmaWarp = (kSoftmaxThreads + kCopyThreads) / 32u;
+constexpr uint32_t kTilePages = kKeys / kPageTokens;
+constexpr uint32_t kCopyWarp = 8, kMmaWarp = 9;  // in front of them two softmax groups of 128, a thread per row in each
+constexpr uint32_t kAttentionThreads = 320;
 constexpr uint32_t kBlockBytes = kRows * 128u;  // 128 rows of 64 bf16: one swizzled column block of a tile
 constexpr uint32_t kTmemS = 0, kTmemO = 2u * kKeys, kTmemAll = 512;
 constexpr float kRescaleAbove = 8.0f;
@@ -44,8 +47,9 @@ constexpr float kRescaleAbove = 8.0f;
 struct AttentionShared {
   uint64_t k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
   uint64_t s_full[2], p_full[2];
-  uint64_t pv_done;  // PV(j): completes once per tile
-  uint64_t o_done;   // the last PV
+  uint64_t pv_done[2];  // PV of a group's tile
+  uint64_t o_done;      // the last PV
+  float m[2][kRows], l[2][kRows];  // the groups' softmax states
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -104,7 +108,9 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volati
 }
 
 template <uint32_t D, bool EXTRAS>
-__global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel(WindowAttentionParams p) {
+__global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel(const __grid_constant__ CUtensorMap map_k,
+                                                                               const __grid_constant__ CUtensorMap map_v,
+                                                                               WindowAttentionParams p) {
   constexpr uint32_t kColumnBlocks = D / 64u, kTileBytes = kColumnBlocks * kBlockBytes;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t{1023});
@@ -114,20 +120,21 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   volatile uint32_t *abort = &sh.abort;
   const WindowAttentionShape &s = p.s;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint64_t policy = l2_evict_last_policy();
 
   pdl_trigger();
   if (threadIdx.x == 0) {
     for (uint32_t i = 0; i < kStages; ++i) {
-      mbar_init(&sh.k_full[i], kCopyThreads);
-      mbar_init(&sh.v_full[i], kCopyThreads);
+      mbar_init(&sh.k_full[i], 1);
+      mbar_init(&sh.v_full[i], 1);
       mbar_init(&sh.k_empty[i], 1);
       mbar_init(&sh.v_empty[i], 1);
     }
     for (uint32_t i = 0; i < 2; ++i) {
       mbar_init(&sh.s_full[i], 1);
-      mbar_init(&sh.p_full[i], kSoftmaxThreads);
+      mbar_init(&sh.p_full[i], kRows);
+      mbar_init(&sh.pv_done[i], 1);
     }
-    mbar_init(&sh.pv_done, 1);
     mbar_init(&sh.o_done, 1);
     sh.abort = 0;
     mbar_init_fence();
@@ -144,7 +151,9 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   const uint32_t total_rows = p.row_count * group;
   const uint32_t f0 = (gridDim.y - 1u - blockIdx.y) * kRows;  // the longest walks first
   const uint32_t f_end = f0 + kRows < total_rows ? f0 + kRows : total_rows;
-  const uint32_t base = r0.position;
+  const uint32_t base = r0.position, page_count = r0.page_count;
+  const uint32_t *page_table = r0.page_table;
+  uint32_t *error_word = r0.error_word;
   const uint32_t pos_first = base + f0 / group, pos_last = base + (f_end - 1u) / group;
   const bool inside = pos_last < r0.max_context;
   const uint32_t window = s.window != 0 ? s.window : 0xffffffffu;
@@ -155,10 +164,10 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   const uint32_t tiles = inside ? walk.count(kv_end, kKeys) : 0u;
 
   // queries, scaled so that the softmax runs on exp2, as a bf16 rounding and its remainder
-  if (inside && warp < kMmaWarp) {
+  if (inside) {
     const float qscale = s.scale * kLog2e;
     const bool whole_pieces = s.qk_dim == D && p.qkv_stride % 4u == 0 && reinterpret_cast<uintptr_t>(p.qkv) % 16u == 0;
-    for (uint32_t i = threadIdx.x; i < kRows * (D / 8u); i += kSoftmaxThreads + kCopyThreads) {
+    for (uint32_t i = threadIdx.x; i < kRows * (D / 8u); i += kAttentionThreads) {
       const uint32_t row = i / (D / 8u), piece = i % (D / 8u), f = f0 + row;
       float x[8];
 #pragma unroll
@@ -190,14 +199,15 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   const uint32_t tmem = sh.tmem_base;
 
   if (warp == kMmaWarp) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0 && tiles != 0) {
+    // ---------------- MMA issuer: the warp waits together, its first lane issues ----------------
+    if (tiles != 0) {
       const uint32_t idesc_s = attention_instr_desc(kKeys, false), idesc_o = attention_instr_desc(D, true);
       auto scores = [&](uint32_t j) {  // S(j) = Q K(j)^T; its buffer held P(j - 2), which PV(j - 2) has read
         const uint32_t st = j % kStages;
-        if (!abortable_wait(&sh.k_full[st], (j / kStages) & 1u, abort, r0.error_word)) return false;
-        if (j >= 2u && !abortable_wait(&sh.pv_done, j & 1u, abort, r0.error_word)) return false;
+        if (!warp_wait(&sh.k_full[st], (j / kStages) & 1u, abort, error_word)) return false;
+        if (j >= 2u && !warp_wait(&sh.pv_done[j & 1u], ((j >> 1) & 1u) ^ 1u, abort, error_word)) return false;
         tcgen05_fence_after();
+        if (lane != 0) return true;
         const uint8_t *k = k_ring + st * kTileBytes;
 #pragma unroll
         for (uint32_t part = 0; part < 2u; ++part) {
@@ -213,98 +223,84 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
         tcgen05_commit(&sh.s_full[j & 1u]);
         return true;
       };
-      bool ok = scores(0);
+      bool ok = scores(0) && (tiles < 2u || scores(1));
       for (uint32_t j = 0; ok && j < tiles; ++j) {
-        if (j + 1u < tiles && !scores(j + 1u)) break;
         const uint32_t st = j % kStages;
-        if (!abortable_wait(&sh.v_full[st], (j / kStages) & 1u, abort, r0.error_word)) break;
-        if (!abortable_wait(&sh.p_full[j & 1u], (j >> 1) & 1u, abort, r0.error_word)) break;
-        tcgen05_fence_after();
-        const uint64_t v = mn_major_sw128_desc(v_ring + st * kTileBytes);
-#pragma unroll
-        for (uint32_t part = 0; part < 2u; ++part) {
-#pragma unroll
-          for (uint32_t ks = 0; ks < kKeys / kUmmaK; ++ks)
-            mma_tmem_a(tmem + kTmemO, tmem + kTmemS + (j & 1u) * kKeys + part * (kKeys / 2u) + ks * (kUmmaK / 2u),
-                       v + ks * ((kUmmaK * 128u) >> 4), idesc_o, (j != 0 || part != 0 || ks != 0) ? 1u : 0u);
+        if (!warp_wait(&sh.v_full[st], (j / kStages) & 1u, abort, error_word)) break;
+        if (j + 1u == tiles && kv_end % kPageTokens != 0) {
+          // the last page's rows behind the last query hold whatever the pool had: a zero probability times a NaN
+          // would still be one
+          const uint32_t from = kv_end - walk.tile(j) * kKeys;
+          const uint32_t rows = kPageTokens - kv_end % kPageTokens;
+          for (uint32_t i = lane; i < rows * (D / 8u); i += 32u)
+            *reinterpret_cast<uint4 *>(v_ring + st * kTileBytes + swizzled(from + i / (D / 8u), i % (D / 8u))) = make_uint4(0, 0, 0, 0);
+          fence_proxy_async();
+          __syncwarp();
         }
-        tcgen05_commit(&sh.v_empty[st]);
-        tcgen05_commit(&sh.pv_done);
-        if (j + 1u == tiles) tcgen05_commit(&sh.o_done);
+        if (!warp_wait(&sh.p_full[j & 1u], (j >> 1) & 1u, abort, error_word)) break;
+        tcgen05_fence_after();
+        if (lane == 0) {
+          const uint64_t v = mn_major_sw128_desc(v_ring + st * kTileBytes);
+#pragma unroll
+          for (uint32_t part = 0; part < 2u; ++part) {
+#pragma unroll
+            for (uint32_t ks = 0; ks < kKeys / kUmmaK; ++ks)
+              mma_tmem_a(tmem + kTmemO + (j & 1u) * D, tmem + kTmemS + (j & 1u) * kKeys + part * (kKeys / 2u) + ks * (kUmmaK / 2u),
+                         v + ks * ((kUmmaK * 128u) >> 4), idesc_o, (j >= 2u || part != 0 || ks != 0) ? 1u : 0u);
+          }
+          tcgen05_commit(&sh.v_empty[st]);
+          tcgen05_commit(&sh.pv_done[j & 1u]);
+          if (j + 1u == tiles) tcgen05_commit(&sh.o_done);
+        }
+        __syncwarp();
+        if (j + 2u < tiles) ok = scores(j + 2u);
       }
     }
-  } else if (warp >= 4u) {
-    // ---------------- K and V ----------------
-    const uint32_t copy_warp = warp - 4u;
-    const uint16_t *keys = r0.key_pages + p.key_offset, *values = r0.value_pages + p.value_offset;
-    uint32_t issued = 0, signalled = 0;  // items: K(0), V(0), K(1), V(1), ...
-    auto signal_to = [&](uint32_t end) {
-      if (signalled < end) fence_proxy_async();
-      for (; signalled < end; ++signalled) {
-        const uint32_t st = (signalled >> 1) % kStages;
-        mbar_arrive((signalled & 1u) == 0 ? &sh.k_full[st] : &sh.v_full[st]);
-      }
-    };
+  } else if (warp == kCopyWarp) {
+    // ---------------- K and V: lane i < 8 brings page i of the tile ----------------
     bool ok = true;
     for (uint32_t j = 0; ok && j < tiles; ++j) {
       const uint32_t first = walk.tile(j) * kKeys, st = j % kStages;
-      uint32_t my_page = 0;
-      if (lane < kKeys / kPageTokens && first + lane * kPageTokens < kv_end) {
-        my_page = r0.page_table[first / kPageTokens + lane];
-        if (my_page >= r0.page_count) {
-          report_error(r0.error_word, kErrPageOutOfRange);
-          my_page = 0;
-        }
+      uint32_t y = 0xffffffffu;  // a page behind the last query: rows outside the map, which read as zeros
+      if (lane < kTilePages && first + lane * kPageTokens < kv_end) {
+        const uint32_t page = page_table[first / kPageTokens + lane];
+        if (page < page_count)
+          y = page * kPageTokens;
+        else
+          report_error(error_word, kErrPageOutOfRange);
       }
-#pragma unroll 1
-      for (uint32_t what = 0; what < 2u; ++what) {
-        uint64_t *empty = what == 0 ? &sh.k_empty[st] : &sh.v_empty[st];
-        const uint32_t parity = ((j / kStages) & 1u) ^ 1u;
-        if (!__all_sync(0xffffffffu, mbar_try_wait(empty, parity))) {
-          cp_async_wait<0>();  // nothing more to issue for now: hand over what is on its way
-          signal_to(issued);
-          if (!warp_wait(empty, parity, abort, r0.error_word)) {
-            ok = false;
-            break;
-          }
-        }
-        uint8_t *stage = (what == 0 ? k_ring : v_ring) + st * kTileBytes;
-        const uint16_t *from = what == 0 ? keys : values;
-        // a warp copies whole rows: D / 8 pieces each
+      if (y == 0xffffffffu) y = page_count * kPageTokens;
 #pragma unroll
-        for (uint32_t i = 0; i < kKeys * (D / 8u) / kCopyThreads; ++i) {
-          constexpr uint32_t kPerWarp = 32u / (D / 8u);  // rows a warp copies at once
-          const uint32_t row = (i * (kCopyThreads / 32u) + copy_warp) * kPerWarp + lane / (D / 8u), piece = lane % (D / 8u);
-          const uint32_t page = __shfl_sync(0xffffffffu, my_page, row / kPageTokens);
-          const bool valid = first + row < kv_end;  // rows behind the last query are filled with zeros
-          const uint16_t *src = from + (valid ? cache_row(page, first + row, s.kv_heads, kvh, D) + piece * 8u : 0u);
-          cp_async_zfill<16>(stage + swizzled(row, piece), src, valid);
+      for (uint32_t what = 0; what < 2u; ++what) {
+        uint64_t *full = what == 0 ? &sh.k_full[st] : &sh.v_full[st];
+        if (ok && !warp_wait(what == 0 ? &sh.k_empty[st] : &sh.v_empty[st], ((j / kStages) & 1u) ^ 1u, abort, error_word)) ok = false;
+        if (!ok) break;
+        if (lane == 0) mbar_arrive_expect_tx(full, kTileBytes);
+        __syncwarp();
+        uint8_t *stage = (what == 0 ? k_ring : v_ring) + st * kTileBytes + lane * kPageTokens * 128u;
+        if (lane < kTilePages) {
+#pragma unroll
+          for (uint32_t c = 0; c < kColumnBlocks; ++c)
+            tma_load_2d(stage + c * kBlockBytes, what == 0 ? &map_k : &map_v, kvh * D + c * 64u, y, full, policy);
         }
-        cp_async_commit();
-        issued += 1;
-        cp_async_wait<2>();
-        if (issued > 2u) signal_to(issued - 2u);
       }
     }
-    cp_async_wait<0>();
-    signal_to(issued);
   } else if (tiles != 0) {
     // ---------------- softmax ----------------
-    const uint32_t f = f0 + threadIdx.x;
-    const bool live = f < f_end;
-    const uint32_t pos = base + (live ? f : f_end - 1u) / group;
-    const uint32_t lanes = (warp * 32u) << 16;
+    const uint32_t half = warp >> 2, row = threadIdx.x & (kRows - 1u), f = f0 + row;
+    const uint32_t pos = base + (f < f_end ? f : f_end - 1u) / group;
+    const uint32_t lanes = ((warp & 3u) * 32u) << 16;
+    const uint32_t s_addr = tmem + lanes + kTmemS + half * kKeys, o_addr = tmem + lanes + kTmemO + half * D;
     const float cap2 = s.softcap * kLog2e, inv_cap2 = cap2 > 0.0f ? 1.0f / cap2 : 0.0f;
     float m_ref = -INFINITY, l = 0.0f;
     bool ok = true;
-    for (uint32_t j = 0; j < tiles; ++j) {
+    for (uint32_t j = half; j < tiles; j += 2u) {
       const uint32_t first = walk.tile(j) * kKeys;
-      if (!warp_wait(&sh.s_full[j & 1u], (j >> 1) & 1u, abort, r0.error_word)) {
+      if (!warp_wait(&sh.s_full[half], (j >> 1) & 1u, abort, error_word)) {
         ok = false;
         break;
       }
       tcgen05_fence_after();
-      const uint32_t s_addr = tmem + lanes + kTmemS + (j & 1u) * kKeys;
       float v[kKeys];
 #pragma unroll
       for (uint32_t c = 0; c < kKeys; c += 32u) tmem_load32(s_addr + c, v + c);
@@ -334,20 +330,14 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
         const float corr = m_new == m_ref ? 1.0f : exp2_ftz(m_ref - m_new);  // 0 where nothing was seen before
         m_ref = m_new;
         l *= corr;
-        if (j != 0) {
-          // PV(j - 2) is done (S(j) followed it) and PV(j) waits for this warp: the parity is that of PV(j - 1)
-          if (!warp_wait(&sh.pv_done, (j - 1u) & 1u, abort, r0.error_word)) {
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
+        if (j >= 2u) {  // the group's last PV is done: S(j) followed it
 #pragma unroll 1
           for (uint32_t c = 0; c < D; c += 16u) {
             float o[16];
-            tmem_load16(tmem + lanes + kTmemO + c, o);
+            tmem_load16(o_addr + c, o);
 #pragma unroll
             for (uint32_t i = 0; i < 16u; ++i) o[i] *= corr;
-            tmem_store16(tmem + lanes + kTmemO + c, reinterpret_cast<const uint32_t *>(o));
+            tmem_store16(o_addr + c, reinterpret_cast<const uint32_t *>(o));
           }
         }
       }
@@ -370,30 +360,43 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       tmem_store_wait();
       tcgen05_fence_before();
-      mbar_arrive(&sh.p_full[j & 1u]);
+      mbar_arrive(&sh.p_full[half]);
     }
-    if (ok && warp_wait(&sh.o_done, 0, abort, r0.error_word)) {
-      tcgen05_fence_after();
-      const uint32_t h = kvh * group + f % group;
-      const float inv = live ? output_gate<EXTRAS>(p, f / group, h) / l : 0.0f;
-      uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + static_cast<uint64_t>(f / group) * p.out_stride + h * s.v_dim;
-      const bool vector = s.v_dim == D && p.out_stride % 8u == 0 && reinterpret_cast<uintptr_t>(p.out) % 16u == 0;
+    sh.m[half][row] = m_ref;
+    sh.l[half][row] = l;
+    if (ok) ok = warp_wait(&sh.o_done, 0, abort, error_word);
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  if (warp < kCopyWarp && tiles != 0 && sh.abort == 0u) {
+    // ---------------- output: half of a row's columns per thread, the two groups' parts added ----------------
+    const uint32_t half = warp >> 2, row = threadIdx.x & (kRows - 1u), f = f0 + row;
+    const uint32_t o_addr = tmem + (((warp & 3u) * 32u) << 16) + kTmemO;
+    const bool live = f < f_end;
+    const uint32_t h = kvh * group + f % group;
+    const float m = fmaxf(sh.m[0][row], sh.m[1][row]);  // one of the groups has seen the row's own key: finite
+    const float w0 = exp2_ftz(sh.m[0][row] - m), w1 = exp2_ftz(sh.m[1][row] - m);  // 0: nothing seen, maybe never written
+    const float inv = live ? output_gate<EXTRAS>(p, f / group, h) / (sh.l[0][row] * w0 + sh.l[1][row] * w1) : 0.0f;
+    uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + static_cast<uint64_t>(f / group) * p.out_stride + h * s.v_dim;
+    const bool vector = s.v_dim == D && p.out_stride % 8u == 0 && reinterpret_cast<uintptr_t>(p.out) % 16u == 0;
 #pragma unroll 1
-      for (uint32_t c = 0; c < D; c += 16u) {
-        float o[16];
-        tmem_load16(tmem + lanes + kTmemO + c, o);
-        if (!live) continue;
-        if (vector) {
+    for (uint32_t c = half * (D / 2u); c < (half + 1u) * (D / 2u); c += 16u) {
+      float o[16], o1[16];
+      tmem_load16(o_addr + c, o);
+      tmem_load16(o_addr + D + c, o1);
+      if (!live) continue;
 #pragma unroll
-          for (uint32_t i = 0; i < 16u; i += 8u)
-            *reinterpret_cast<uint4 *>(dst + c + i) =
-                make_uint4(pack_bf16_hi(o[i] * inv, o[i + 1] * inv), pack_bf16_hi(o[i + 2] * inv, o[i + 3] * inv),
-                           pack_bf16_hi(o[i + 4] * inv, o[i + 5] * inv), pack_bf16_hi(o[i + 6] * inv, o[i + 7] * inv));
-        } else {
+      for (uint32_t i = 0; i < 16u; ++i) o[i] = ((w0 > 0.0f ? o[i] * w0 : 0.0f) + (w1 > 0.0f ? o1[i] * w1 : 0.0f)) * inv;
+      if (vector) {
 #pragma unroll
-          for (uint32_t i = 0; i < 16u; ++i)
-            if (c + i < s.v_dim) dst[c + i] = f32_to_bf16_bits(o[i] * inv);
-        }
+        for (uint32_t i = 0; i < 16u; i += 8u)
+          *reinterpret_cast<uint4 *>(dst + c + i) = make_uint4(pack_bf16_hi(o[i], o[i + 1]), pack_bf16_hi(o[i + 2], o[i + 3]),
+                                                               pack_bf16_hi(o[i + 4], o[i + 5]), pack_bf16_hi(o[i + 6], o[i + 7]));
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i)
+          if (c + i < s.v_dim) dst[c + i] = f32_to_bf16_bits(o[i]);
       }
     }
   }
@@ -418,7 +421,7 @@ bool prefill_attention_supported(const WindowAttentionShape &s) {
 
 cudaError_t configure_prefill_attention() {
   cudaError_t err = cudaSuccess;
-  auto set = [&err](void (*kernel)(WindowAttentionParams), uint32_t bytes) {
+  auto set = [&err](void (*kernel)(CUtensorMap, CUtensorMap, WindowAttentionParams), uint32_t bytes) {
     if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   };
   set(prefill_attention_kernel<64, false>, attention_smem<64>());
@@ -429,15 +432,22 @@ cudaError_t configure_prefill_attention() {
 }
 
 cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p) {
-  if (p.rows == nullptr || p.row_count == 0 || p.f32 != 0 || !prefill_attention_supported(p.s)) return cudaErrorInvalidValue;
-  const uint32_t rows = p.row_count * (p.s.heads / p.s.kv_heads);
+  if (p.rows == nullptr || p.row_count == 0 || p.f32 != 0 || p.keys == nullptr || p.values == nullptr ||
+      !prefill_attention_supported(p.s))
+    return cudaErrorInvalidValue;
+  const uint32_t rows = p.row_count * (p.s.heads / p.s.kv_heads), D = p.s.qk_pad;
+  const uint64_t width = static_cast<uint64_t>(p.s.kv_heads) * D, tokens = static_cast<uint64_t>(p.page_count) * kPageTokens;
+  CUtensorMap map_k, map_v;
+  if (!encode_bf16_map_2d(&map_k, static_cast<const uint16_t *>(p.keys) + p.key_offset, width, tokens, 64, kPageTokens) ||
+      !encode_bf16_map_2d(&map_v, static_cast<const uint16_t *>(p.values) + p.value_offset, width, tokens, 64, kPageTokens))
+    return cudaErrorNotSupported;
   const dim3 grid(p.s.kv_heads, (rows + kRows - 1u) / kRows);
   const bool extras = has_extras(p.s);
-  if (p.s.qk_pad == 64u)
+  if (D == 64u)
     return launch_with_pdl(extras ? prefill_attention_kernel<64, true> : prefill_attention_kernel<64, false>, grid,
-                           dim3(kAttentionThreads), attention_smem<64>(), stream, p.pdl != 0, p);
+                           dim3(kAttentionThreads), attention_smem<64>(), stream, p.pdl != 0, map_k, map_v, p);
   return launch_with_pdl(extras ? prefill_attention_kernel<128, true> : prefill_attention_kernel<128, false>, grid,
-                         dim3(kAttentionThreads), attention_smem<128>(), stream, p.pdl != 0, p);
+                         dim3(kAttentionThreads), attention_smem<128>(), stream, p.pdl != 0, map_k, map_v, p);
 }
 
 }  // namespace nb

@@ -204,9 +204,25 @@ bool carve(StaticArena &arena, void *base, uint64_t count, T **out) {
   return true;
 }
 
+// The largest of the sparse layers.
+struct MoeWidths {
+  uint64_t moe = 0, shared = 0, top_k = 0, num_experts = 0;
+};
+MoeWidths moe_widths(const Session *s) {
+  MoeWidths w;
+  for (const LayerLayout &L : s->layout.layers) {
+    if (L.mlp_kind != NERVA_MLP_KIND_SPARSE_MOE) continue;
+    w.moe = std::max<uint64_t>(w.moe, L.moe_intermediate);
+    w.shared = std::max<uint64_t>(w.shared, L.shared_intermediate);
+    w.top_k = std::max<uint64_t>(w.top_k, L.top_k);
+    w.num_experts = std::max<uint64_t>(w.num_experts, L.num_experts);
+  }
+  return w;
+}
+
 bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, void *base) {
   const ModelDims &d = s->dims;
-  const uint64_t ah = d.attention_hidden(), kvh = d.kv_hidden(), qkv_rows = ah + 2 * kvh;
+  const uint64_t ah = d.attention_hidden(), qkv_rows = d.qkv_rows();
   const uint64_t rows = ws->max_rows, part = ws->part_rows, sample = ws->sample_rows;
   if (s->parallel) {
     const ParallelPlan &plan = *s->parallel;
@@ -261,11 +277,55 @@ bool plan_workspace(const Session *s, BlockWorkspace *ws, StaticArena &arena, vo
   ok = ok && carve(arena, base, rows, &ws->token_rows);
   ok = ok && carve(arena, base, sample, &ws->sample_rows_dev);
   ok = ok && carve(arena, base, sample, &ws->head_rows);
+  if (d.mla()) {
+    ok = ok && carve(arena, base, rows * d.heads * d.mla_rank, &ws->mla_ql);
+    ok = ok && carve(arena, base, rows * d.heads * d.mla_rank, &ws->mla_latent);
+  }
+  if (s->has_moe) {
+    const MoeWidths most = moe_widths(s);
+    const uint64_t slots = rows * most.top_k;
+    MoeBlockParams &m = ws->moe;
+    ok = ok && carve(arena, base, slots, &m.ids) && carve(arena, base, slots, &m.slot_of) && carve(arena, base, slots, &m.row_of);
+    ok = ok && carve(arena, base, most.num_experts + 1u, &m.offsets);
+    ok = ok && carve(arena, base, slots, &m.weights) && carve(arena, base, slots, &m.slot_weight) && carve(arena, base, rows, &m.shared_gate);
+    ok = ok && carve(arena, base, rows * d.hidden, &m.x_hi) && carve(arena, base, rows * d.hidden, &m.x_lo);
+    ok = ok && carve(arena, base, slots * d.hidden, &m.slot_hi) && carve(arena, base, slots * d.hidden, &m.slot_lo);
+    ok = ok && carve(arena, base, slots * most.moe, &m.act_hi) && carve(arena, base, slots * most.moe, &m.act_lo);
+    ok = ok && carve(arena, base, slots * d.hidden, &m.y);
+    if (most.shared != 0) {
+      ok = ok && carve(arena, base, rows * most.shared, &m.shared_act_hi) && carve(arena, base, rows * most.shared, &m.shared_act_lo);
+      ok = ok && carve(arena, base, rows * d.hidden, &m.y_shared);
+    }
+  }
   return ok;
 }
 
 const uint16_t *arena_at(const Session *s, uint64_t offset) {
   return offset == kMissingOffset ? nullptr : s->weights->arena + offset;
+}
+
+// A sparse layer's weights and shape, with the workspace's scratch.
+MoeBlockParams moe_layer(const Session *s, const LayerLayout &L) {
+  MoeBlockParams p = s->weights->block_ws.moe;
+  p.hidden = s->dims.hidden;
+  p.moe_intermediate = L.moe_intermediate;
+  p.shared_intermediate = L.shared_intermediate;
+  p.num_experts = L.num_experts;
+  p.top_k = L.top_k;
+  p.norm_topk_prob = L.norm_topk_prob;
+  p.eps = s->rms_eps;
+  p.norm_weight = arena_at(s, L.rms_mlp);
+  p.w_router = arena_at(s, L.w_router);
+  p.w_expert_gate_up = arena_at(s, L.w_expert_gate_up);
+  p.w_expert_down = arena_at(s, L.w_expert_down);
+  p.w_shared_gate = arena_at(s, L.w_shared_gate);
+  p.w_shared_up = arena_at(s, L.w_shared_up);
+  p.w_shared_down = arena_at(s, L.w_shared_down);
+  p.w_shared_router = arena_at(s, L.w_shared_router);
+  p.expert_stride = L.expert_stride;
+  p.expert_up_offset = L.expert_up_offset;
+  p.error_word = s->device_error;
+  return p;
 }
 
 struct BlockPlan {
@@ -310,8 +370,8 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
   Session *s = b.model;
   const ModelDims &d = s->dims;
   const BlockWorkspace &ws = s->weights->block_ws;
-  const uint32_t ah = static_cast<uint32_t>(d.attention_hidden()), kvh = static_cast<uint32_t>(d.kv_hidden());
-  const uint32_t qkv_rows = ah + 2u * kvh;
+  const uint32_t ah = static_cast<uint32_t>(d.attention_hidden());
+  const uint32_t qkv_rows = static_cast<uint32_t>(d.qkv_rows());
   uint64_t n = 0;
   cudaError_t err = launch_with_pdl(block_embed_kernel, dim3(b.rows), dim3(256), 0, b.stream, false, ws.token_rows,
                                     arena_at(s, s->layout.embeddings), d.hidden, ws.h_b,
@@ -334,8 +394,34 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
                        ws.x_bf16, d.hidden, kEpilogueStore, nullptr, ws.qkv, nullptr);
     n += 2;
     const bool tiles = b.publish && ws.tile_prefill && b.rows >= kTilePrefillMinRows;
-    const bool paged = !tiles && !b.k_maps.empty();
-    if (err == cudaSuccess && (b.publish || paged)) {
+    // Sparse models keep short blocks on the fused kernel's row form: it adds in the decode step's order, so hardly a
+    // rounding differs from the token-by-token prefill, and with it hardly a router's choice between near equals.
+    const bool paged = !tiles && !b.k_maps.empty() && !s->has_moe;
+    if (err == cudaSuccess && d.mla()) {
+      MlaBlockParams mp{};
+      mp.first_position = b.longest - b.rows;
+      mp.rows = b.rows;
+      mp.max_context = s->max_context;
+      mp.qkv = ws.qkv;
+      mp.qkv_stride = qkv_rows;
+      mp.w_kv_b = arena_at(s, L.w_v);
+      mp.kv_a_norm = arena_at(s, L.k_norm);
+      mp.cache = s->kv_keys + l * s->kv_layer_elems;
+      mp.page_table = s->page_table;
+      mp.page_count = s->kv_pages;
+      mp.heads = d.heads;
+      mp.rank = d.mla_rank;
+      mp.nope = d.mla_nope;
+      mp.rope = d.mla_rope;
+      mp.v_dim = d.head_dim;
+      mp.eps = s->rms_eps;
+      mp.rope_theta = s->rope_theta;
+      mp.ql = ws.mla_ql;
+      mp.latent = ws.mla_latent;
+      mp.out = ws.attn;
+      mp.error_word = s->device_error;
+      err = launch_mla_block(b.stream, mp, b.pdl, &n);
+    } else if (err == cudaSuccess && (b.publish || paged)) {
       // few rows: a head per warp; many: all heads of a row in one block
       const uint32_t query_heads = tiles || paged ? d.heads : 0u;
       const uint32_t groups = (d.kv_heads + query_heads + kPublishWarps - 1u) / kPublishWarps;
@@ -347,7 +433,9 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       n += 1;
     }
     if (err != cudaSuccess) break;
-    if (tiles) {
+    if (d.mla()) {
+      // done above
+    } else if (tiles) {
       WindowAttentionParams wp{};
       wp.s.heads = d.heads;
       wp.s.kv_heads = d.kv_heads;
@@ -415,6 +503,15 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
     // h_a = h_b + O(attention)
     err = block_gemm(b, arena_at(s, L.w_o), d.hidden, ah, ws.attn, ah, kEpilogueStore, ws.h_b, ws.h_a, nullptr);
     // MLP half
+    if (L.mlp_kind == NERVA_MLP_KIND_SPARSE_MOE) {
+      MoeBlockParams mp = moe_layer(s, L);
+      mp.h = ws.h_a;
+      mp.out = ws.h_b;
+      mp.rows = b.rows;
+      if (err == cudaSuccess) err = launch_moe_block(b.stream, mp, s->sm_count, b.pdl, &n);
+      n += 1;
+      continue;
+    }
     if (err == cudaSuccess)
       err = launch_with_pdl(block_norm_kernel, dim3(b.rows), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_a,
                             arena_at(s, L.rms_mlp), s->rms_eps, d.hidden, ws.x_bf16, d.hidden, nullptr);
@@ -462,7 +559,7 @@ uint32_t block_attention_splits(const Session *s, uint32_t rows, uint32_t longes
 
 FusedAttentionRow attention_row(Session *s, const BlockWorkspace &ws, uint32_t row, uint32_t position) {
   const ModelDims &d = s->dims;
-  const uint64_t qkv_rows = d.attention_hidden() + 2 * d.kv_hidden();
+  const uint64_t qkv_rows = d.qkv_rows();
   FusedAttentionRow r{};
   r.position = position;
   r.max_context = s->max_context;
@@ -507,17 +604,34 @@ cudaError_t upload_rows(const BlockWorkspace &ws, const std::vector<FusedAttenti
 
 }  // namespace
 
-bool block_step_supported(const NervaCudaHfDecodeSequenceSession *s) {
+bool block_step_supported(const Session *s) {
   const ModelDims &d = s->dims;
   if (s->parallel) return s->parallel->f32 || tensor_map_available();
-  if (s->tp_world > 1 || s->has_moe || d.mla() || !s->fused_attention || d.dtype != NERVA_DTYPE_BF16) return false;
+  if (s->tp_world > 1 || (!d.mla() && !s->fused_attention) || d.dtype != NERVA_DTYPE_BF16) return false;
   const uint64_t ah = d.attention_hidden();
-  if (d.hidden % 64u != 0 || ah % 64u != 0 || d.intermediate % 64u != 0) return false;
-  if (d.hidden % 4u != 0 || d.hidden / 4u > kNormRegIters * kNormThreads) return false;  // block_norm_kernel's reach
+  if (d.hidden % 64u != 0 || ah % 64u != 0) return false;
+  if (d.hidden / 4u > kNormRegIters * kNormThreads) return false;  // block_norm_kernel's reach
+  auto aligned = [s](uint64_t offset) { return reinterpret_cast<uintptr_t>(arena_at(s, offset)) % 16u == 0; };
   for (const LayerLayout &L : s->layout.layers) {
-    if (L.mlp_kind != NERVA_MLP_KIND_DENSE || L.o_bias != kMissingOffset) return false;
+    if (L.o_bias != kMissingOffset) return false;
+    if (L.mlp_kind == NERVA_MLP_KIND_SPARSE_MOE) {
+      // these models also run token by token: what the block kernels cannot take stays there
+      if (!moe_block_supported(moe_layer(s, L))) return false;
+    } else if (L.mlp_kind != NERVA_MLP_KIND_DENSE || d.intermediate % 64u != 0) {
+      return false;
+    }
+    if ((s->has_moe || d.mla()) && (!aligned(L.w_o) || !aligned(L.rms_attn) || !aligned(L.rms_mlp) || !aligned(s->layout.lm_head) ||
+                                    (L.mlp_kind == NERVA_MLP_KIND_DENSE && !aligned(L.w_down))))
+      return false;
   }
   return tensor_map_available();
+}
+
+// Blocks of a few rows of a latent attention walk the cache without a split over its length (about 3.5 us per 32
+// cached rows and layer), where a decode step takes about 80 us a layer: short blocks behind a long context stay steps.
+bool prefill_in_blocks(const Session *s, uint32_t rows, uint32_t context) {
+  if (s->weights->block_ws.block == nullptr || s->engine != 0 || rows < 2u) return false;
+  return !s->dims.mla() || (rows >= 4u && rows >= context / 700u);
 }
 
 cudaError_t launch_argmax_partials(cudaStream_t stream, const float *logits, uint32_t vocab, uint32_t rows, uint32_t chunks,
@@ -529,14 +643,25 @@ cudaError_t launch_argmax_partials(cudaStream_t stream, const float *logits, uin
 cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
   BlockWorkspace &ws = s->weights->block_ws;
   const uint32_t context_rows = (s->max_context + 15u) & ~15u;
-  const uint32_t most = s->parallel && s->parallel->f32 ? kBlockPartRows : kBlockMaxRows;
+  uint32_t most = s->parallel && s->parallel->f32 ? kBlockPartRows : kBlockMaxRows;
+  if (s->has_moe) {  // half a gigabyte for the slots' activations and outputs
+    const uint64_t fit = (64ull << 20) / (moe_widths(s).top_k * s->dims.hidden) / 64u * 64u;
+    most = static_cast<uint32_t>(std::min<uint64_t>(most, std::max<uint64_t>(fit, 64u)));
+  }
   ws.max_rows = std::max(kBlockSampleRows, std::min(most, context_rows));
   ws.part_rows = std::min(ws.max_rows, kBlockPartRows);
   ws.sample_rows = kBlockSampleRows;
   StaticArena sizing(UINT64_MAX / 2);
   if (!plan_workspace(s, &ws, sizing, nullptr)) return cudaErrorMemoryAllocation;
   ws.bytes = sizing.used();
+  ws.packed_steps = !s->has_moe && !s->dims.mla();
   cudaError_t err = cudaMalloc(&ws.block, ws.bytes);
+  if (err != cudaSuccess && !ws.packed_steps) {
+    // sparse models and latent attention do without blocks, token by token
+    cudaGetLastError();
+    ws = BlockWorkspace{};
+    return cudaSuccess;
+  }
   if (err != cudaSuccess) return err;
   StaticArena arena(ws.bytes);
   if (!plan_workspace(s, &ws, arena, ws.block)) return cudaErrorMemoryAllocation;
@@ -546,7 +671,7 @@ cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
     err = cudaMemsetAsync(ws.block, 0, ws.bytes, s->stream);
     return err == cudaSuccess ? configure_gemm_tc_kernel() : err;
   }
-  const uint32_t max_out = std::max(std::max<uint32_t>(static_cast<uint32_t>(d.attention_hidden() + 2 * d.kv_hidden()),
+  const uint32_t max_out = std::max(std::max<uint32_t>(static_cast<uint32_t>(d.qkv_rows()),
                                                       2u * d.intermediate),
                                     std::max(d.hidden, d.vocab));
   err = cudaMemsetAsync(ws.attn_tickets, 0, static_cast<uint64_t>(ws.part_rows) * d.kv_heads * sizeof(uint32_t), s->stream);
@@ -554,12 +679,14 @@ cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
     err = cudaMemsetAsync(ws.gemm_tickets, 0, static_cast<uint64_t>(gemm_tc_ticket_count(max_out)) * sizeof(uint32_t),
                           s->stream);
   if (err == cudaSuccess) err = configure_gemm_tc_kernel();
+  if (err == cudaSuccess && s->has_moe) err = configure_moe_block();
+  if (err == cudaSuccess && d.mla()) err = configure_mla_block();
   // NERVA_B200_ROW_ATTENTION=fused keeps the fused kernel's row form (comparison and fallback)
   const char *row_attention = getenv("NERVA_B200_ROW_ATTENTION");
   const bool tile_or_paged = !(row_attention != nullptr && strcmp(row_attention, "fused") == 0);
-  ws.tile_prefill = tile_or_paged && (d.head_dim == 64u || d.head_dim == 128u);
+  ws.tile_prefill = tile_or_paged && !d.mla() && (d.head_dim == 64u || d.head_dim == 128u);
   if (err == cudaSuccess && ws.tile_prefill) err = configure_prefill_attention();
-  ws.paged_rows = attention_rows_supported(d.heads, d.kv_heads, d.head_dim) && tile_or_paged;
+  ws.paged_rows = !d.mla() && attention_rows_supported(d.heads, d.kv_heads, d.head_dim) && tile_or_paged;
   return err;
 }
 
@@ -568,7 +695,7 @@ cudaError_t enqueue_block_decode(NervaCudaHfDecodeSequenceSession *const *sessio
   if (count == 0 || count > kBlockSampleRows) return cudaErrorInvalidValue;
   Session *model = sessions[0];
   const BlockWorkspace &ws = model->weights->block_ws;
-  if (ws.block == nullptr || count > ws.max_rows) return cudaErrorNotSupported;
+  if (ws.block == nullptr || !ws.packed_steps || count > ws.max_rows) return cudaErrorNotSupported;
   const ModelDims &d = model->dims;
   std::vector<FusedAttentionRow> attn(count);
   std::vector<BlockTokenRow> tokens(count);
@@ -658,6 +785,8 @@ cudaError_t enqueue_chunked_prefill(NervaCudaHfDecodeSequenceSession *s, uint32_
       // the last position's residual stream becomes the session's own, where the head expects it
       err = cudaMemcpyAsync(s->h_b, ws.h_b + static_cast<uint64_t>(rows - 1u) * width, width * sizeof(float),
                             cudaMemcpyDeviceToDevice, s->stream);
+      // (a model with sparse layers adds the last sublayer's output in the head: it is in the stream already)
+      if (err == cudaSuccess && s->has_moe) err = cudaMemsetAsync(s->down, 0, width * sizeof(float), s->stream);
     }
     // the wanted positions of this chunk, up to sample_rows of them per head launch
     std::vector<uint32_t> place, row;

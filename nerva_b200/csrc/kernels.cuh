@@ -291,6 +291,24 @@ uint32_t mla_attention_splits(uint32_t target_context);
 cudaError_t launch_mla_attention(cudaStream_t stream, const MlaParams &p, uint32_t splits, bool pdl);
 cudaError_t configure_mla_kernels();  // once per device before the first launch
 
+// The same attention for consecutive positions of one session (mla_block.cu).
+struct MlaBlockParams {
+  uint32_t first_position, rows, max_context;
+  float *qkv;              // [rows][qkv_stride]: as MlaParams::qkv
+  uint32_t qkv_stride;
+  const uint16_t *w_kv_b, *kv_a_norm;
+  uint16_t *cache;
+  const uint32_t *page_table;
+  uint32_t page_count;
+  uint32_t heads, rank, nope, rope, v_dim;
+  float eps, rope_theta;
+  float *ql, *latent;      // scratch [rows][heads][rank]: absorbed queries, attended latent rows
+  uint16_t *out;           // [rows][heads * v_dim]
+  uint32_t *error_word;
+};
+cudaError_t configure_mla_block();
+cudaError_t launch_mla_block(cudaStream_t stream, const MlaBlockParams &p, bool pdl, uint64_t *launches);
+
 // ---- softmax top-k sparse MoE MLP (moe.cu) ----
 struct MoeExpertParams {
   // residual add + RMSNorm prologue (as ProjectionParams), fp32 result
@@ -334,6 +352,29 @@ bool moe_supported(uint32_t hidden, uint32_t moe_intermediate, uint32_t shared_i
 cudaError_t configure_moe_kernels();
 // Two launches: routing + gate/up of the chosen experts, then SwiGLU + down and the weighted sum.
 cudaError_t launch_moe_experts(cudaStream_t stream, const MoeExpertParams &p, uint32_t sm_count, bool pdl);
+
+// The sparse MLP of a block of rows (moe_block.cu).
+struct MoeBlockParams {
+  const float *h;                    // [rows][hidden] residual stream
+  float *out;                        // [rows][hidden] h + the MLP's output
+  uint32_t rows, hidden, moe_intermediate, shared_intermediate, num_experts, top_k, norm_topk_prob;
+  float eps;
+  const uint16_t *norm_weight, *w_router;
+  const uint16_t *w_expert_gate_up, *w_expert_down, *w_shared_gate, *w_shared_up, *w_shared_down, *w_shared_router;
+  uint64_t expert_stride, expert_up_offset;  // as MoeExpertParams
+  uint32_t *error_word;
+  // scratch
+  uint32_t *ids, *slot_of, *row_of, *offsets;  // [rows][top_k] x 2, [rows * top_k], [num_experts + 1]
+  float *weights, *slot_weight, *shared_gate;  // [rows][top_k], [rows * top_k], [rows]
+  uint16_t *x_hi, *x_lo;                       // [rows][hidden]
+  uint16_t *slot_hi, *slot_lo;                 // [rows * top_k][hidden]
+  uint16_t *act_hi, *act_lo;                   // [rows * top_k][moe_intermediate]
+  uint16_t *shared_act_hi, *shared_act_lo;     // [rows][shared_intermediate]
+  float *y, *y_shared;                         // [rows * top_k][hidden], [rows][hidden]
+};
+bool moe_block_supported(const MoeBlockParams &p);
+cudaError_t configure_moe_block();
+cudaError_t launch_moe_block(cudaStream_t stream, const MoeBlockParams &p, uint32_t sm_count, bool pdl, uint64_t *launches);
 
 // ---- projections of decoders described layer by layer (parallel_projection.cu) ----
 // All vectors are padded to multiples of 64 with zeros, matrices have zero columns (and rows) there.

@@ -1996,6 +1996,26 @@ extern "C" int nerva_b200_session_set_engine(Session *s, uint32_t engine) {
   return 0;
 }
 
+namespace {
+// The block workspace of a weight set, for one session's launches at a time: forks may be driven by several threads.
+// Given back when nothing of this session's stream uses it any more.
+struct BlockWorkspaceHold {
+  std::unique_lock<std::mutex> lock;
+  cudaStream_t stream = nullptr;
+  void take(Session *s) {
+    lock = std::unique_lock<std::mutex>(s->weights->block_mutex);
+    stream = s->stream;
+  }
+  cudaError_t give_back() {
+    if (!lock.owns_lock()) return cudaSuccess;
+    const cudaError_t err = cudaStreamSynchronize(stream);
+    lock.unlock();
+    return err;
+  }
+  ~BlockWorkspaceHold() { give_back(); }
+};
+}  // namespace
+
 extern "C" int nerva_cuda_hf_decode_sequence_session_start(
     const NervaCudaHfDecodeSequenceSessionStartRequest *request,
     NervaCudaHfDecodeSequenceResult *out) {
@@ -2022,9 +2042,11 @@ extern "C" int nerva_cuda_hf_decode_sequence_session_start(
   // NERVA_B200_PREFILL=decode keeps the token-by-token prefill on models that have the block path
   // (comparison runs); read per call.
   const char *prefill_env = getenv("NERVA_B200_PREFILL");
-  const bool chunked = s->weights->block_ws.block != nullptr && s->engine == 0 && s->prompt_count > 1 &&
+  const bool chunked = prefill_in_blocks(s, s->prompt_count, s->prompt_count) &&
                        !(prefill_env != nullptr && prefill_env[0] == 'd');
+  BlockWorkspaceHold hold;
   if (chunked) {
+    hold.take(s);
     // Chunked prefill: up to block_ws.max_rows prompt positions through every layer at a time
     // (block projections on the tensor pipe, paged K/V published per chunk), then the head for the
     // last position (session_decode_prefill.inc.cu:1879-2245 is the reference's counterpart).
@@ -2205,12 +2227,14 @@ extern "C" int nerva_cuda_hf_decode_sequence_session_run(
   cudaError_t err = reset_request_state(s, request->prompt_tokens, request->prompt_token_count, out);
   GraphEntry *graph = nullptr;
   const char *prefill_env = getenv("NERVA_B200_PREFILL");
-  const bool chunked = s->weights->block_ws.block != nullptr && s->engine == 0 && s->prompt_count > 1 &&
+  const bool chunked = prefill_in_blocks(s, s->prompt_count, s->prompt_count) &&
                        !(prefill_env != nullptr && prefill_env[0] == 'd');
   if (err == cudaSuccess) err = ensure_graph(s, splits_for(s, context_steps), s->sample_kind, &graph, out);
   if (err == cudaSuccess) err = cudaEventRecord(s->ev_start, s->stream);
   uint32_t first_step = 0;
   if (chunked) {
+    BlockWorkspaceHold hold;
+    hold.take(s);
     // The prompt goes through the chunked prefill, exactly as session_start runs it, so that
     // run == start + advance bit for bit; the decode steps follow.
     uint64_t launches = 0, head_launches = 0;
@@ -2222,6 +2246,8 @@ extern "C" int nerva_cuda_hf_decode_sequence_session_run(
       err = enqueue_step(s, splits_for(s, s->prompt_count), s->sample_kind, &head_launches, nullptr, true);
     out->kernel_launches += launches + head_launches;
     first_step = s->prompt_count;
+    const cudaError_t prefilled = hold.give_back();  // other sessions may prefill beside this one's steps
+    if (err == cudaSuccess) err = prefilled;
   }
   // One sampling graph replayed for every (remaining) position; samples at prompt positions are
   // never read (session_api_lifecycle.inc.cu:849-920).
@@ -2371,12 +2397,14 @@ extern "C" int nerva_cuda_hf_decode_sequence_batch_advance_one(
   bool packed = selected.size() >= 2 && selected.size() <= kBlockSampleRows;
   for (uint32_t index : selected) {
     const Session *s = request->sessions[index];
-    packed = packed && s->weights->block_ws.block != nullptr && s->sample_kind == 1 && s->engine == 0;
+    packed = packed && s->weights->block_ws.packed_steps && s->sample_kind == 1 && s->engine == 0;
   }
   if (packed) {
     std::vector<Session *> block;
     for (uint32_t index : selected) block.push_back(request->sessions[index]);
     cudaStream_t stream = block[0]->stream;
+    BlockWorkspaceHold hold;
+    hold.take(block[0]);
     for (Session *s : block) {  // idle sessions: this only orders their earlier work before the block's
       if (err == cudaSuccess) err = cudaStreamSynchronize(s->stream);
       out->sync_calls += 1;
@@ -2574,6 +2602,9 @@ extern "C" int nerva_b200_session_append(Session *s, const uint32_t *tokens, uin
     if (want[i] >= count) return -1;
   }
   const uint32_t end = begin + count;
+  const bool chunked = prefill_in_blocks(s, count, end);
+  BlockWorkspaceHold hold;
+  if (chunked) hold.take(s);
   NervaCudaHfDecodeSequenceResult counters{};
   cudaError_t err;
   if (fresh) {
@@ -2587,7 +2618,7 @@ extern "C" int nerva_b200_session_append(Session *s, const uint32_t *tokens, uin
   }
   s->started = false;
   s->prompt_count = end;
-  if (s->weights->block_ws.block != nullptr && s->engine == 0 && count > 1) {
+  if (chunked) {
     const WantedLogits wanted{want, want_count, logits};
     if (err == cudaSuccess) err = enqueue_chunked_prefill(s, begin, end, wanted, nullptr);
     const uint32_t last = end - 1u;

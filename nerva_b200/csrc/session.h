@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <deque>
 #include <vector>
@@ -204,6 +205,10 @@ struct BlockWorkspace {
   BlockTokenRow *token_rows = nullptr;
   BlockSampleRow *sample_rows_dev = nullptr;  // [sample_rows] device copies of the sampler's row descriptors
   uint32_t *head_rows = nullptr;  // [sample_rows] rows of the block whose logits are wanted
+  // sparse layers: the scratch pointers (moe_block.cu), sized for the largest layer; latent attention: [max_rows][heads][rank]
+  MoeBlockParams moe{};
+  float *mla_ql = nullptr, *mla_latent = nullptr;
+  bool packed_steps = false;    // rows of several sessions may share a block (enqueue_block_decode)
 };
 constexpr uint32_t kBlockArgmaxChunks = 64;
 // Rows of a prefill chunk.  256 (one MMA N) made every chunk a weight stream; from about 2000 rows on the weights'
@@ -222,6 +227,7 @@ struct SharedWeights {
   uint16_t *qkv_packed = nullptr;     // [layers][(A + 2 KV) x H]
   uint16_t *gate_up_packed = nullptr; // [layers][2 I x H], rows interleaved gate/up
   BlockWorkspace block_ws;            // empty when the model has no block-step path
+  std::mutex block_mutex;             // held from the first launch of a block step to the end of its last: forks share the workspace
   ~SharedWeights() {
     if (block != nullptr) cudaFree(block);
     if (block_ws.block != nullptr) cudaFree(block_ws.block);
@@ -257,9 +263,12 @@ cudaError_t configure_step_kernel();
 cudaError_t launch_step_kernel(cudaStream_t stream, const StepKernelParams &p, uint32_t blocks);
 
 // ---- block steps (block_step.cu) ----
-// True when every layer is dense SwiGLU without biases, the fused attention kernel serves the head
-// shape and every projection width is a multiple of 64: the shapes the block kernels run.
+// True when the layers are dense SwiGLU without biases or sparse MLPs that moe_block.cu takes, the fused attention
+// kernel serves the head shape or the attention is latent, and every projection width is a multiple of 64: the shapes
+// the block kernels run.
 bool block_step_supported(const NervaCudaHfDecodeSequenceSession *s);
+// Whether `rows` positions that end at `context` go through the layers as blocks.
+bool prefill_in_blocks(const NervaCudaHfDecodeSequenceSession *s, uint32_t rows, uint32_t context);
 // Allocates s->weights->block_ws (at create).
 cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s);
 // One token for each of `count` sessions that share weights, on `stream`: the weights are streamed

@@ -323,21 +323,21 @@ struct MoeExpertParams {
   const uint16_t *w_expert_down;     // [E][hidden][moe_intermediate]
   const uint16_t *w_shared_gate, *w_shared_up, *w_shared_down;  // shared expert, optional
   const uint16_t *w_shared_router;   // its gate sigmoid(router . x); null: always on (scale 1)
-  // Routing happens inside the gate/up launch: router logits W_router . x for all experts, softmax,
-  // top-k, optional renormalisation; block 0 stores the new residual stream (resid_out, optional)
-  // and the result, which the down launch reads.
+  // Router logits W_router . x for all experts, softmax, top-k, optional renormalisation; the new residual stream goes
+  // to resid_out (optional).
   const uint16_t *w_router;          // [num_experts][hidden]
   uint32_t num_experts, norm_topk_prob;
   float *resid_out;
+  float *router_logits;              // [num_experts] scratch
+  float *x_norm;                     // [hidden] scratch: the normalised row
   uint32_t *expert_ids;              // [top_k] scratch: the routing result
   float *route_weights;              // [top_k]
-  float *gate_up_out;                // scratch: per expert gate then up rows (+ the shared expert's), fp32
+  float *gate_up_out;                // scratch: silu(gate) * up of the chosen experts held here, then of the shared
+                                     // expert, fp32
   float *shared_gate;                // scratch: 1 float
   float *out_f32;                    // [hidden] the MLP output
-  float *partial;                    // scratch: [17][hidden] per-expert contributions before they are added
-  uint32_t *ticket;                  // scratch: one counter, zero between launches
   uint32_t *error_word;
-  uint32_t max_intermediate, max_rows_per_block;  // filled by the launcher
+  uint32_t gate_up_slots, down_slots, down_x_floats;  // filled by the launcher
   // Expert parallel: this rank holds experts [expert_base, expert_base + expert_local) of the layer
   // (the matrices above are indexed by id - expert_base) and, of the shared expert, a slice of the
   // intermediate dimension; chosen experts held elsewhere are skipped.  With push.world > 1 the
@@ -350,7 +350,7 @@ struct MoeExpertParams {
 bool moe_supported(uint32_t hidden, uint32_t moe_intermediate, uint32_t shared_intermediate,
                    uint32_t num_experts, uint32_t top_k, uint32_t sm_count);
 cudaError_t configure_moe_kernels();
-// Two launches: routing + gate/up of the chosen experts, then SwiGLU + down and the weighted sum.
+// Three launches: norm + router logits, top-k + gate/up + SwiGLU of the chosen experts, down and the weighted sum.
 cudaError_t launch_moe_experts(cudaStream_t stream, const MoeExpertParams &p, uint32_t sm_count, bool pdl);
 
 // The sparse MLP of a block of rows (moe_block.cu).

@@ -26,6 +26,7 @@
 
 #include "gemm_device.cuh"
 #include "mma_bf16.cuh"
+#include "moe_route.cuh"
 
 namespace nb {
 namespace {
@@ -34,11 +35,6 @@ namespace {
 constexpr uint32_t kRouteWarps = 8;
 constexpr uint32_t kRouteRows = 8;       // rows of a block, a warp per row in the norm and the routing
 constexpr uint32_t kRouteExperts = 4;    // experts a warp takes at a time: a row's activations are read once for all
-constexpr uint32_t kRouteMaxExperts = 256, kRouteMaxTopK = 16;
-
-__device__ __forceinline__ bool route_before(float w, uint32_t e, float best_w, uint32_t best_e) {
-  return w > best_w || (w == best_w && e < best_e);
-}
 
 // Shared memory: rows_per_block x hidden fp32 (per row two planes: the first four of every eight elements, the last
 // four), then rows x experts logits.
@@ -131,54 +127,9 @@ __global__ void __launch_bounds__(kRouteWarps * 32) moe_block_route_kernel(MoeBl
   }
   __syncthreads();
 
-  constexpr uint32_t kNone = 0xffffffffu, kPerLane = kRouteMaxExperts / 32u;
   for (uint32_t r = warp; r < rows; r += kRouteWarps) {
-    const float *row_logits = logits + r * p.num_experts;
-    float w[kPerLane], m = -INFINITY, sum = 0.0f;
-#pragma unroll
-    for (uint32_t k = 0; k < kPerLane; ++k) {
-      const uint32_t e = lane + 32u * k;
-      w[k] = e < p.num_experts ? row_logits[e] : -INFINITY;
-      m = fmaxf(m, w[k]);
-    }
-    m = warp_max(m);
-#pragma unroll
-    for (uint32_t k = 0; k < kPerLane; ++k) {
-      w[k] = lane + 32u * k < p.num_experts ? expf(w[k] - m) : 0.0f;
-      sum += w[k];
-    }
-    sum = warp_sum(sum);
-    const bool divide = sum > 0.0f && isfinite(sum);
-    uint32_t taken = 0;
-    float chosen_sum = 0.0f, mine = 0.0f;
-    uint32_t my_id = 0;
-    for (uint32_t rank = 0; rank < p.top_k; ++rank) {
-      float bw = -INFINITY;
-      uint32_t be = kNone;
-#pragma unroll
-      for (uint32_t k = 0; k < kPerLane; ++k) {
-        const uint32_t e = lane + 32u * k;
-        if (e >= p.num_experts || ((taken >> k) & 1u) != 0) continue;
-        const float v = divide ? w[k] / sum : w[k];
-        if (be == kNone || route_before(v, e, bw, be)) bw = v, be = e;
-      }
-      for (int offset = 16; offset > 0; offset >>= 1) {
-        const float ow = __shfl_xor_sync(0xffffffffu, bw, offset);
-        const uint32_t oe = __shfl_xor_sync(0xffffffffu, be, offset);
-        if (oe != kNone && (be == kNone || route_before(ow, oe, bw, be))) bw = ow, be = oe;
-      }
-      // a weight that is not a number compares with nothing, so the lanes may differ: the first one's choice counts
-      bw = __shfl_sync(0xffffffffu, bw, 0);
-      be = __shfl_sync(0xffffffffu, be, 0);
-      if ((be & 31u) == lane) taken |= 1u << (be >> 5);
-      chosen_sum += bw;
-      if (lane == rank) mine = bw, my_id = be;
-    }
-    if (p.norm_topk_prob != 0 && chosen_sum > 0.0f) mine /= chosen_sum;
-    if (lane < p.top_k) {
-      p.ids[static_cast<uint64_t>(row0 + r) * p.top_k + lane] = my_id;
-      p.weights[static_cast<uint64_t>(row0 + r) * p.top_k + lane] = mine;
-    }
+    const uint64_t at = static_cast<uint64_t>(row0 + r) * p.top_k;
+    moe_route_warp(logits + r * p.num_experts, p.num_experts, p.top_k, p.norm_topk_prob, p.ids + at, p.weights + at);
   }
 }
 
@@ -187,11 +138,11 @@ constexpr uint32_t kGroupThreads = 1024;
 
 // Slots of an expert's tokens follow each other; the order inside an expert does not enter any result.
 __global__ void __launch_bounds__(kGroupThreads) moe_block_group_kernel(MoeBlockParams p) {
-  __shared__ uint32_t count[kRouteMaxExperts], next[kRouteMaxExperts];
+  __shared__ uint32_t count[kMoeMaxExperts], next[kMoeMaxExperts];
   pdl_trigger();
   pdl_wait();
   const uint32_t pairs = p.rows * p.top_k;
-  for (uint32_t e = threadIdx.x; e < kRouteMaxExperts; e += blockDim.x) count[e] = 0;
+  for (uint32_t e = threadIdx.x; e < kMoeMaxExperts; e += blockDim.x) count[e] = 0;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(&count[__ldcg(p.ids + i)], 1u);
   __syncthreads();
@@ -240,7 +191,7 @@ __global__ void __launch_bounds__(256) moe_block_combine_kernel(MoeBlockParams p
   pdl_trigger();
   pdl_wait();
   const uint32_t row = blockIdx.x;
-  __shared__ uint32_t slots[kRouteMaxTopK];
+  __shared__ uint32_t slots[kMoeMaxTopK];
   if (threadIdx.x < p.top_k) slots[threadIdx.x] = __ldcg(p.slot_of + static_cast<uint64_t>(row) * p.top_k + threadIdx.x);
   __syncthreads();
   const uint64_t at = static_cast<uint64_t>(row) * p.hidden;
@@ -286,7 +237,7 @@ struct ExpertShared {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base, abort;
-  uint32_t first_tile[kRouteMaxExperts + 1];
+  uint32_t first_tile[kMoeMaxExperts + 1];
 };
 
 struct ExpertTile {
@@ -535,7 +486,7 @@ uint32_t route_rows(uint32_t hidden, uint32_t experts) {
 
 bool moe_block_supported(const MoeBlockParams &p) {
   auto aligned = [](const void *ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16u == 0; };
-  return p.num_experts != 0 && p.num_experts <= kRouteMaxExperts && p.top_k != 0 && p.top_k <= kRouteMaxTopK &&
+  return p.num_experts != 0 && p.num_experts <= kMoeMaxExperts && p.top_k != 0 && p.top_k <= kMoeMaxTopK &&
          p.top_k <= p.num_experts && p.hidden % 64u == 0 && p.moe_intermediate % 8u == 0 && p.shared_intermediate % 8u == 0 &&
          route_rows(p.hidden, p.num_experts) != 0 && p.expert_stride % p.hidden == 0 && p.expert_up_offset % p.hidden == 0 &&
          aligned(p.norm_weight) && aligned(p.w_router) && aligned(p.w_expert_gate_up) && aligned(p.w_expert_down) &&

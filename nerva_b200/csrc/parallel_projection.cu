@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
   }
   __syncthreads();
 
-  stream_consume<false, SLOTS>(rs, sh.first, 0, x0, total0, p.error_word);
-  if (second) stream_consume<false, SLOTS>(rs, sh.second, 1, x1, total1, p.error_word);
+  stream_consume<SLOTS>(rs, sh.first, 0, x0, total0, p.error_word);
+  if (second) stream_consume<SLOTS>(rs, sh.second, 1, x1, total1, p.error_word);
   __syncthreads();
 
   if (KIND == kParallelIn || KIND == kSandwichIn || KIND == kSandwichOut) {

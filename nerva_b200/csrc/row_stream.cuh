@@ -261,33 +261,12 @@ __device__ __forceinline__ float dot8_f32(const uint4 &w, const float4 &xa, cons
   acc = fmaf(bf16x2_hi(w.w), xb.w, acc);
   return acc;
 }
-// fp32 activations (XF32) sit in shared memory in two planes, so that the lanes of a warp read
-// consecutive 16-byte pieces (a plain [cols] array would put a lane's two float4 32 bytes from the
-// next lane's: a two-way bank conflict on every load): element i of a `cols`-wide vector is at
-// xf32_index(i, cols) — the first four of every eight elements in plane A, the last four in plane B.
-__host__ __device__ inline uint32_t xf32_index(uint32_t i, uint32_t cols) {
-  return ((i & 4u) != 0 ? cols / 2u : 0u) + ((i >> 3) << 2) + (i & 3u);
-}
-// One 16-byte piece of weights at `wp + off` times the matching activations: bf16 at byte offset
-// `off` of xp, or (XF32) the piece's two float4 at index off / 16 of the planes xa and xb.
-template <bool XF32>
-__device__ __forceinline__ float dot_piece(const uint8_t *wp, const uint8_t *xp, const float4 *xa, const float4 *xb,
-                                           uint32_t off, float acc) {
-  if (XF32) return dot8_f32(lds128(wp + off), xa[off / 16u], xb[off / 16u], acc);
-  return dot8(lds128(wp + off), lds128(xp + off), acc);
-}
-__device__ __forceinline__ float2 dot_piece_x2(const uint8_t *wp, const float4 *xa, const float4 *xb, uint32_t off,
-                                               float2 acc) {
-  return dot8_f32x2(lds128(wp + off), xa[off / 16u], xb[off / 16u], acc);
-}
-
 // Consumes job `index` (jobs are consumed in order, each exactly once, by every
 // warp of the block).  `x` is the bf16 activation vector in shared memory;
 // row_total[r] (shared, one float per block-local row, zeroed by the caller
 // before the block's previous synchronisation) receives the total of every row
 // that lies wholly inside this warp's range; partial rows go to sh.edge.
-// XF32: `x` points at fp32 activations instead of bf16 ones.
-template <bool XF32 = false, uint32_t SLOTS = kStreamSlots>
+template <uint32_t SLOTS = kStreamSlots>
 __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, uint32_t index,
                                                const void *x, float *row_total,
                                                uint32_t *error_word) {
@@ -316,43 +295,7 @@ __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, 
     const uint8_t *wp = rs.ring + slot * kChunkBytes + lane * 16u;
     const uint32_t row_offset = pos - (row_end - job.row_bytes);  // bytes into the row
     const uint8_t *xp = reinterpret_cast<const uint8_t *>(x) + row_offset + lane * 16u;
-    if (XF32) {
-      // planes A and B of the fp32 vector (xf32_index), at this lane's first piece of the chunk
-      const float4 *xa = reinterpret_cast<const float4 *>(x) + row_offset / 16u + lane;
-      const float4 *xb = xa + job.row_bytes / 16u;
-      // packed multiply-adds: every accumulator splits into an even and an odd half for the chunk
-      float2 a2[4] = {make_float2(acc[0], 0.0f), make_float2(acc[1], 0.0f), make_float2(acc[2], 0.0f),
-                      make_float2(acc[3], 0.0f)};
-      uint32_t off = 0;
-      if (len == kChunkBytes) {
-#pragma unroll
-        for (uint32_t i = 0; i < kChunkBytes / kSweepBytes; i += 4) {
-          a2[0] = dot_piece_x2(wp, xa, xb, (i + 0) * kSweepBytes, a2[0]);
-          a2[1] = dot_piece_x2(wp, xa, xb, (i + 1) * kSweepBytes, a2[1]);
-          a2[2] = dot_piece_x2(wp, xa, xb, (i + 2) * kSweepBytes, a2[2]);
-          a2[3] = dot_piece_x2(wp, xa, xb, (i + 3) * kSweepBytes, a2[3]);
-        }
-        off = kChunkBytes;
-      } else if (len == kChunkBytes / 2u) {
-#pragma unroll
-        for (uint32_t i = 0; i < kChunkBytes / kSweepBytes / 2u; i += 4) {
-          a2[0] = dot_piece_x2(wp, xa, xb, (i + 0) * kSweepBytes, a2[0]);
-          a2[1] = dot_piece_x2(wp, xa, xb, (i + 1) * kSweepBytes, a2[1]);
-          a2[2] = dot_piece_x2(wp, xa, xb, (i + 2) * kSweepBytes, a2[2]);
-          a2[3] = dot_piece_x2(wp, xa, xb, (i + 3) * kSweepBytes, a2[3]);
-        }
-        off = kChunkBytes / 2u;
-      }
-      for (; off + 4u * kSweepBytes <= len; off += 4u * kSweepBytes) {
-        a2[0] = dot_piece_x2(wp, xa, xb, off, a2[0]);
-        a2[1] = dot_piece_x2(wp, xa, xb, off + kSweepBytes, a2[1]);
-        a2[2] = dot_piece_x2(wp, xa, xb, off + 2u * kSweepBytes, a2[2]);
-        a2[3] = dot_piece_x2(wp, xa, xb, off + 3u * kSweepBytes, a2[3]);
-      }
-      for (; off + lane * 16u < len; off += kSweepBytes) a2[0] = dot_piece_x2(wp, xa, xb, off, a2[0]);
-#pragma unroll
-      for (uint32_t i = 0; i < 4; ++i) acc[i] = a2[i].x + a2[i].y;
-    } else if (len == kChunkBytes) {
+    if (len == kChunkBytes) {
 #pragma unroll
       for (uint32_t i = 0; i < kChunkBytes / kSweepBytes; i += 4) {
         const uint4 w0 = lds128(wp + (i + 0) * kSweepBytes), x0 = lds128(xp + (i + 0) * kSweepBytes);

@@ -409,15 +409,14 @@ bool plan_state(Session *s, StaticArena &arena, void *base) {
   uint64_t moe_scratch = 0;
   for (const LayerLayout &L : s->layout.layers) {
     if (L.mlp_kind == NERVA_MLP_KIND_SPARSE_MOE)
-      moe_scratch = std::max<uint64_t>(moe_scratch, 2ull * L.top_k * L.moe_intermediate + 2ull * L.shared_intermediate);
+      moe_scratch = std::max<uint64_t>(moe_scratch, static_cast<uint64_t>(L.top_k) * L.moe_intermediate + L.shared_intermediate);
   }
   ok = ok && carve(arena, base, uint64_t{256}, &s->router_logits);
   ok = ok && carve(arena, base, uint64_t{16}, &s->route_ids);
   ok = ok && carve(arena, base, uint64_t{16}, &s->route_weights);
   ok = ok && carve(arena, base, uint64_t{4}, &s->shared_gate);
   ok = ok && carve(arena, base, moe_scratch + 4u, &s->moe_gate_up);
-  ok = ok && carve(arena, base, moe_scratch != 0 ? uint64_t{17} * d.hidden : uint64_t{4}, &s->moe_partial);
-  ok = ok && carve(arena, base, uint64_t{4}, &s->moe_ticket);
+  ok = ok && carve(arena, base, moe_scratch != 0 ? uint64_t{d.hidden} : uint64_t{4}, &s->moe_x);
   s->timeline_nodes = 5u * d.layers + 1u;
   ok = ok && carve(arena, base, static_cast<uint64_t>(s->timeline_nodes) * kTimelineSlots, &s->timeline);
   return ok;
@@ -893,15 +892,14 @@ cudaError_t enqueue_step(Session *s, uint32_t splits, uint32_t sample, uint64_t 
       ep.gate_up_out = s->moe_gate_up;
       ep.shared_gate = s->shared_gate;
       ep.out_f32 = s->down;
-      ep.partial = s->moe_partial;
-      ep.ticket = s->moe_ticket;
+      ep.router_logits = s->router_logits;
+      ep.x_norm = s->moe_x;
       ep.error_word = s->device_error;
       ep.expert_base = L.expert_base;
       ep.expert_local = L.expert_local;
       if (ep_on) ep.push = push_to(ep_buffer(l), l + 1u);
-      // routing + gate/up, then down: two launches
       err = launch_moe_experts(s->stream, ep, s->sm_count, s->use_pdl);
-      n += 2;
+      n += 3;
       profile_mark(s, prof, kBucketDown);
       continue;
     }
@@ -1197,7 +1195,6 @@ cudaError_t reset_request_state(Session *s, const uint32_t *prompt, uint32_t cou
   if (err == cudaSuccess) err = cudaMemsetAsync(s->device_cursor, 0, sizeof(uint32_t), s->stream);
   if (err == cudaSuccess) err = cudaMemsetAsync(s->device_error, 0, sizeof(uint32_t), s->stream);
   // completion counters are zero between launches; a request that failed half-way may have left one mid-count
-  if (err == cudaSuccess) err = cudaMemsetAsync(s->moe_ticket, 0, 4 * sizeof(uint32_t), s->stream);
   if (err == cudaSuccess) err = cudaMemsetAsync(s->attn_tickets, 0, s->dims.heads * sizeof(uint32_t), s->stream);
   const uint64_t bytes = static_cast<uint64_t>(count) * sizeof(uint32_t);
   if (err == cudaSuccess)
@@ -1534,7 +1531,6 @@ cudaError_t allocate_state(Session *s, int32_t *stage) {
   if (err == cudaSuccess) err = cudaMemsetAsync(s->device_cursor, 0, sizeof(uint32_t), s->stream);
   if (err == cudaSuccess)
     err = cudaMemsetAsync(s->attn_tickets, 0, s->dims.heads * sizeof(uint32_t), s->stream);
-  if (err == cudaSuccess) err = cudaMemsetAsync(s->moe_ticket, 0, 4 * sizeof(uint32_t), s->stream);
   if (s->parallel && err == cudaSuccess) {
     // the padding behind a layer's activations multiplies zero weights, so it only has to be finite
     const uint64_t bytes = s->parallel->element_bytes();

@@ -385,8 +385,7 @@ struct NervaCudaHfDecodeSequenceSession {
   float *mla_ql = nullptr;             // [heads][rank] absorbed queries
   float *router_logits = nullptr, *route_weights = nullptr, *shared_gate = nullptr, *moe_gate_up = nullptr;
   uint32_t *route_ids = nullptr;
-  float *moe_partial = nullptr;        // [17][hidden] per-expert contributions of a sparse MLP (moe.cu)
-  uint32_t *moe_ticket = nullptr;      // completion counter of the expert down launch, zero between launches
+  float *moe_x = nullptr;              // [hidden] normalised row of a sparse MLP (moe.cu)
   // tensor parallel (nerva_b200_session_create_sharded)
   uint32_t tp_world = 1, tp_rank = 0;
   bool tp_two_stage = false;   // two ranks only: use the two-stage gather of the larger worlds

@@ -21,6 +21,9 @@ MOE = synth.DecoderConfig("moe", layers=2, hidden=320, heads=8, kv_heads=2, head
                           rope_theta=1e6, qk_norm=True, num_experts=12, top_k=3, moe_intermediate=136,
                           shared_intermediate=0, norm_topk_prob=True)
 MOE_SHARED = dataclasses.replace(MOE, hidden=512, num_experts=40, top_k=5, moe_intermediate=256, shared_intermediate=72)
+# a step's activations of all experts exceed shared memory: the down projection goes in passes
+MOE_WIDE = dataclasses.replace(MOE, layers=1, hidden=1600, intermediate=5120, num_experts=16, top_k=12, moe_intermediate=5120,
+                               shared_intermediate=2056)
 LATENT = dataclasses.replace(synth.DEEPSEEK_V2_LITE, layers=3, vocab=4096, hidden=512, heads=4, kv_heads=4, head_dim=64,
                              intermediate=1024, num_experts=8, top_k=2, moe_intermediate=128, shared_intermediate=256,
                              kv_lora_rank=128, qk_nope_head_dim=64, qk_rope_head_dim=32)
@@ -55,7 +58,7 @@ def _steps_apart(a, b):
     return 0.0 if top == 0.0 else float(np.abs(fa - fb).max() / 2.0 ** (np.floor(np.log2(top)) - 7))
 
 
-@pytest.mark.parametrize("cfg,count", [(MOE, 2), (MOE, 7), (MOE, 129), (MOE_SHARED, 9), (MOE_SHARED, 300), (LATENT, 4),
+@pytest.mark.parametrize("cfg,count", [(MOE, 2), (MOE, 7), (MOE, 129), (MOE_SHARED, 9), (MOE_SHARED, 300), (MOE_WIDE, 5), (LATENT, 4),
                                        (LATENT, 35), (LATENT, 257), (LATENT_256, 66), (FULL, 33), (FULL, 210)])
 def test_block_prefill_matches_prefill_by_decode(built_lib, cfg, count):
     checkpoint = _checkpoint(cfg)

@@ -740,6 +740,8 @@ cudaError_t enqueue_block_decode(NervaCudaHfDecodeSequenceSession *const *sessio
     st.vocab = d.embed_vocab;
     st.error_word = s->device_error;
     sample[r].logits = s->logits;
+    sample[r].host_slots = s->host_slots;
+    sample[r].host_error = s->host_error;
   }
   if (err == cudaSuccess)  // pageable source: staged before the call returns
     err = cudaMemcpyAsync(ws.sample_rows_dev, sample.data(), sample.size() * sizeof(BlockSampleRow),

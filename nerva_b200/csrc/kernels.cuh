@@ -587,6 +587,9 @@ cudaError_t launch_argmax_partials(cudaStream_t stream, const float *logits, uin
 struct BlockSampleRow {
   StepState state;
   float *logits;
+  // pinned host memory: the session's token ring and error word, where the row's slot and errors so far go too
+  NervaCudaSyntheticTokenSlot *host_slots;
+  uint32_t *host_error;
 };
 // Arg-max of every row (from `partials` candidates per row) into the row's own session, and the
 // rows' logits into the sessions' own buffers, in one launch.

@@ -2405,18 +2405,15 @@ extern "C" int nerva_cuda_hf_decode_sequence_batch_advance_one(
       if (err == cudaSuccess) err = cudaStreamSynchronize(s->stream);
       out->sync_calls += 1;
     }
-    uint64_t launches = 0;
-    if (err == cudaSuccess) err = enqueue_block_decode(block.data(), static_cast<uint32_t>(block.size()), stream, &launches);
     for (Session *s : block) {
-      const uint32_t slot = s->prompt_count - 1u + s->observed;
-      if (err == cudaSuccess)
-        err = cudaMemcpyAsync(s->host_slots + slot, s->device_slots + slot, sizeof(NervaCudaSyntheticTokenSlot),
-                              cudaMemcpyDeviceToHost, stream);
-      if (err == cudaSuccess)
-        err = cudaMemcpyAsync(s->host_error, s->device_error, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+      // the step's last launch writes the token's slot and the error word here
+      s->host_slots[s->prompt_count - 1u + s->observed].completion = 0;
+      *s->host_error = 0;
       out->d2h_bytes += sizeof(NervaCudaSyntheticTokenSlot);
       out->sampling_kernel_launches += 1;
     }
+    uint64_t launches = 0;
+    if (err == cudaSuccess) err = enqueue_block_decode(block.data(), static_cast<uint32_t>(block.size()), stream, &launches);
     out->projection_kernel_launches += 4ull * block[0]->dims.layers + 1u;
     const cudaError_t sync = cudaStreamSynchronize(stream);
     out->sync_calls += 1;

@@ -273,7 +273,8 @@ bool prefill_in_blocks(const NervaCudaHfDecodeSequenceSession *s, uint32_t rows,
 cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s);
 // One token for each of `count` sessions that share weights, on `stream`: the weights are streamed
 // once for the block.  Every session must be idle, positioned at its next token, and its stream
-// synchronised.  Enqueues only; the caller copies the token slots back and synchronises.
+// synchronised.  Enqueues only; the tokens' slots and the sessions' error words are in host memory once the stream has
+// been synchronised.
 cudaError_t enqueue_block_decode(NervaCudaHfDecodeSequenceSession *const *sessions, uint32_t count,
                                  cudaStream_t stream, uint64_t *launches);
 // Logits wanted from a prefill: places[i] counts from the first position of the call, values go to

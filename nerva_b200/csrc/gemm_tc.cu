@@ -408,8 +408,8 @@ uint32_t gemm_smem_bytes(uint32_t n_pad, uint32_t stages) {
 
 // Two runs per SM whatever the block size, so that the split points — and with them the order in
 // which a row's partial sums are added — depend on the matrix shape alone: a token gets the same
-// bits in a block of 2 and in a block of 256.  Blocks too large for two per SM run the grid in two waves.
-uint32_t gemm_blocks(uint32_t rows, uint32_t cols, uint32_t sm_count) {
+// bits in a block of 2 and in a block of 64.  Blocks too large for two per SM run the grid in two waves.
+uint32_t gemm_blocks(uint32_t rows, uint32_t cols, uint32_t sm_count) {  // (blocks of up to 64 tokens: wide_from_65_tokens)
   const Partition p = make_partition(rows, cols, 1);
   const uint32_t want = 2u * sm_count;
   // Between (about) one and two row tiles per SM (gate/up of the 8B shapes: 192 tiles): one block per
@@ -461,9 +461,18 @@ cudaError_t configure_gemm_tc_kernel() {
   return err == cudaSuccess ? configure_gemm_wide_kernel() : err;
 }
 
+// With more than kSmallBlockTokens tokens a block here is alone on its SM and its runs come in two waves of their own
+// start and end.  Matrices whose 256-row tiles occupy most pairs of SMs go to gemm_wide.cu then: 24576 x 4096, 70 / 125 /
+// 200 tokens 66 / 73 / 87 us where two waves took 80 / 93 / 113.  Fewer rows leave pairs idle there: 6144 x 4096, 125
+// tokens 35 us on either path; 4096 x 4096 and 4096 x 12288 61 us on average, here 41 with the fix-up.
+static bool wide_from_65_tokens(const GemmParams &g, uint32_t sm_count) {
+  return g.tokens > kSmallBlockTokens && g.tokens <= kGemmMaxTokens && gemm_shape_ok(g) &&
+         (g.rows + 2u * kTileRows - 1u) / (2u * kTileRows) >= sm_count / 2u * 3u / 4u;
+}
+
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count) {
   // more tokens than one MMA is wide: what the caller asks for is arithmetic, not a weight stream
-  if (gemm_wide_eligible(g)) return launch_gemm_wide(stream, g, sm_count);
+  if (gemm_wide_eligible(g) || wide_from_65_tokens(g, sm_count)) return launch_gemm_wide(stream, g, sm_count);
   if (!gemm_tc_eligible(g) || g.workspace == nullptr) return cudaErrorInvalidValue;
   GemmKernelParams p = gemm_kernel_params(g);
   p.n_pad = padded_tokens(g.tokens);

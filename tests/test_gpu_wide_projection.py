@@ -18,6 +18,8 @@ PROJ_ATOL = 2e-3
     (768, 512, 511), (512, 1536, 513),   # one token on either side of two full tiles
     (6144, 4096, 640), (4096, 12288, 1500), (24576, 4096, 300),  # more tiles than pairs, several waves
     (1000, 1408, 2048), (130, 64, 2049),
+    # 65 to 256 tokens of matrices with many rows, and one row tile fewer than that takes
+    (24576, 4096, 65), (13825, 128, 100), (16384, 64, 256), (13824, 128, 100),
 ])
 def test_wide_projection_matches_a_64_bit_product(built_lib, rows, cols, tokens):
     import torch

@@ -14,6 +14,9 @@
 //   mla_output_kernel     blocks (head h, 8 output rows): merge of the spans, then out[h] = W_UV[h] . lat[h] -> bf16
 // Cache rows are (rank + rope) bf16 values in the session's K pages, addressed through the page
 // table like every other cache row (hf_decode_sequence/types.cuh:328-337).
+// What bounds the three launches is round trips to the L2, not bytes (W_kv_b of 16 heads is 4 MB): so the weights of the
+// first and the last are requested before their dependency waits, and queries and spans are read with all loads of a
+// thread in flight together.  Context 1024, 6 layers: the step 498 -> 460 us (the launches themselves about 24 us a layer before).
 #include <math.h>
 
 #include "common.cuh"
@@ -42,6 +45,7 @@ __device__ __forceinline__ void rope_pair(float &left, float &right, uint32_t pa
 }
 
 constexpr uint32_t kMlaPrepareSlice = 64;  // absorbed-query elements per block
+constexpr uint32_t kMlaPrepareKeep = 32;   // of a thread's weights in registers: a quarter of 128
 
 // Grid: heads * (rank / 64) blocks for the absorbed queries, one more for the cache row.
 __global__ void __launch_bounds__(256) mla_prepare_kernel(MlaParams p) {
@@ -49,13 +53,26 @@ __global__ void __launch_bounds__(256) mla_prepare_kernel(MlaParams p) {
   __shared__ float part[4][kMlaPrepareSlice];
   __shared__ float scratch[40];
   pdl_trigger();
+  const uint32_t qdim = p.nope + p.rope, width = p.rank + p.rope;
+  const uint32_t slices = p.rank / kMlaPrepareSlice;
+  const uint32_t h = blockIdx.x / slices, slice = blockIdx.x % slices;
+  const bool query = blockIdx.x < p.heads * slices;
+  const uint32_t r_local = threadIdx.x & (kMlaPrepareSlice - 1u), quarter = threadIdx.x / kMlaPrepareSlice;
+  const uint32_t r = slice * kMlaPrepareSlice + r_local;
+  const uint32_t per = (p.nope + 3u) / 4u;
+  const uint32_t n_begin = quarter * per, n_end = n_begin + per < p.nope ? n_begin + per : p.nope;
+  const uint16_t *w_uk = p.w_kv_b + static_cast<uint64_t>(h) * (p.nope + p.v_dim) * p.rank;
+  // the weights depend on nothing: they are on their way while the projection ends
+  uint16_t w[kMlaPrepareKeep];
+  if (query) {
+#pragma unroll
+    for (uint32_t k = 0; k < kMlaPrepareKeep; ++k)
+      w[k] = n_begin + k < n_end ? __ldg(w_uk + static_cast<uint64_t>(n_begin + k) * p.rank + r) : static_cast<uint16_t>(0);
+  }
   pdl_wait();  // the fused projection of this step
   const uint32_t position = *p.cursor;
   if (position >= p.max_context) return;
-  const uint32_t qdim = p.nope + p.rope, width = p.rank + p.rope;
-  const uint32_t slices = p.rank / kMlaPrepareSlice;
-  if (blockIdx.x < p.heads * slices) {
-    const uint32_t h = blockIdx.x / slices, slice = blockIdx.x % slices;
+  if (query) {
     float *q = p.qkv + static_cast<uint64_t>(h) * qdim;
     for (uint32_t i = threadIdx.x; i < p.nope; i += blockDim.x) q_nope[i] = q[i];
     if (slice == 0 && p.rope_theta > 0.0f && threadIdx.x < p.rope / 2u) {
@@ -69,14 +86,12 @@ __global__ void __launch_bounds__(256) mla_prepare_kernel(MlaParams p) {
     // ql[r] = sum_n q_nope[n] W_UK[h][n][r] for 64 consecutive r: thread (r, quarter) adds a quarter
     // of the n range (64 consecutive threads read one 128-byte piece of a W_UK row, all of a
     // thread's loads are independent), the quarters are added in order
-    const uint16_t *w_uk = p.w_kv_b + static_cast<uint64_t>(h) * (p.nope + p.v_dim) * p.rank;
-    const uint32_t r_local = threadIdx.x & (kMlaPrepareSlice - 1u), quarter = threadIdx.x / kMlaPrepareSlice;
-    const uint32_t r = slice * kMlaPrepareSlice + r_local;
-    const uint32_t per = (p.nope + 3u) / 4u;
-    const uint32_t n_begin = quarter * per, n_end = n_begin + per < p.nope ? n_begin + per : p.nope;
     float acc = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < kMlaPrepareKeep; ++k)
+      if (n_begin + k < n_end) acc = fmaf(q_nope[n_begin + k], bf16_bits_to_f32(w[k]), acc);
 #pragma unroll 8
-    for (uint32_t n = n_begin; n < n_end; ++n)
+    for (uint32_t n = n_begin + kMlaPrepareKeep; n < n_end; ++n)
       acc = fmaf(q_nope[n], bf16_bits_to_f32(w_uk[static_cast<uint64_t>(n) * p.rank + r]), acc);
     part[quarter][r_local] = acc;
     __syncthreads();
@@ -161,28 +176,30 @@ __global__ void __launch_bounds__(512) mla_attention_kernel(MlaParams p) {
   // padding zero
   if (tile_begin < tile_end) {
     const float qscale = kLog2e * rsqrtf(static_cast<float>(p.nope + p.rope));
-    const uint32_t padded = row_bytes / 2u, total = kMlaHeadsTile * padded;
-    constexpr uint32_t kBatch = 8;  // loads in flight per thread
+    const uint32_t quads = row_bytes / 8u, total = kMlaHeadsTile * quads;  // the padding is two quads
+    constexpr uint32_t kBatch = 5;  // loads in flight per thread: all of them at rank 512
     for (uint32_t base = threadIdx.x; base < total; base += blockDim.x * kBatch) {
-      float v[kBatch];
+      float4 v[kBatch];
 #pragma unroll
       for (uint32_t u = 0; u < kBatch; ++u) {
         const uint32_t i = base + u * blockDim.x;
-        const uint32_t h = i / padded, k = i % padded;
-        v[u] = 0.0f;
-        if (i < total && h < p.heads && k < RANK) v[u] = __ldcg(p.ql + static_cast<uint64_t>(h) * RANK + k);
-        else if (i < total && h < p.heads && k < width)
-          v[u] = __ldcg(p.qkv + static_cast<uint64_t>(h) * (p.nope + p.rope) + p.nope + (k - RANK));
+        const uint32_t h = i / quads, k = 4u * (i % quads);
+        v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < total && h < p.heads && k < RANK) {
+          v[u] = __ldcg(reinterpret_cast<const float4 *>(p.ql + static_cast<uint64_t>(h) * RANK + k));
+        } else if (i < total && h < p.heads && k < width) {  // rotary parts need not be aligned to more than a float
+          const float *src = p.qkv + static_cast<uint64_t>(h) * (p.nope + p.rope) + p.nope + (k - RANK);
+          v[u] = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
+        }
       }
 #pragma unroll
       for (uint32_t u = 0; u < kBatch; ++u) {
         const uint32_t i = base + u * blockDim.x;
         if (i >= total) break;
-        const uint32_t h = i / padded, k = i % padded;
-        const float scaled = v[u] * qscale;
-        const uint16_t hi = f32_to_bf16_bits(scaled);
-        reinterpret_cast<uint16_t *>(q_hi + h * row_bytes)[k] = hi;
-        reinterpret_cast<uint16_t *>(q_lo + h * row_bytes)[k] = f32_to_bf16_bits(scaled - bf16_bits_to_f32(hi));
+        const uint32_t h = i / quads, at = h * row_bytes + 8u * (i % quads);
+        const float x = v[u].x * qscale, y = v[u].y * qscale, z = v[u].z * qscale, w = v[u].w * qscale;
+        *reinterpret_cast<uint2 *>(q_hi + at) = make_uint2(pack_bf16_hi(x, y), pack_bf16_hi(z, w));
+        *reinterpret_cast<uint2 *>(q_lo + at) = make_uint2(pack_bf16_lo(x, y), pack_bf16_lo(z, w));
       }
     }
   }
@@ -348,10 +365,21 @@ __global__ void __launch_bounds__(256) mla_output_kernel(MlaParams p, uint32_t s
   __shared__ float lat[kMlaMaxRank];
   __shared__ float weight[kMlaMaxSplits];
   pdl_trigger();
+  const uint32_t h = blockIdx.x;
+  const uint16_t *w_uv = p.w_kv_b + (static_cast<uint64_t>(h) * (p.nope + p.v_dim) + p.nope) * p.rank;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  // the weights of the warp's row depend on nothing: they are on their way while the attention ends
+  constexpr uint32_t kKeep = kMlaMaxRank / 256u;
+  uint4 kept[kKeep];
+  const uint32_t v0 = blockIdx.y * warps + warp;
+#pragma unroll
+  for (uint32_t k = 0; k < kKeep; ++k)
+    kept[k] = v0 < p.v_dim && lane + 32u * k < p.rank / 8u
+                  ? __ldg(reinterpret_cast<const uint4 *>(w_uv + static_cast<uint64_t>(v0) * p.rank) + lane + 32u * k)
+                  : make_uint4(0u, 0u, 0u, 0u);
   pdl_wait();
   const uint32_t position = *p.cursor;
   if (position >= p.max_context) return;
-  const uint32_t h = blockIdx.x;
   uint32_t splits;  // spans that hold something; `slots` of them were launched and are the stride
   {
     // spans beyond the context's last tile hold nothing (the attention kernel's split arithmetic)
@@ -362,7 +390,6 @@ __global__ void __launch_bounds__(256) mla_output_kernel(MlaParams p, uint32_t s
   }
   if (threadIdx.x < 32u) {
     // one lane per span (two when there are more than 32): the (m, l) pairs become normalised weights
-    const uint32_t lane = threadIdx.x;
     float m = -INFINITY;
     for (uint32_t s = lane; s < splits; s += 32u)
       if (__ldcg(p.partial_l + h * slots + s) > 0.0f) m = fmaxf(m, __ldcg(p.partial_m + h * slots + s));
@@ -380,31 +407,36 @@ __global__ void __launch_bounds__(256) mla_output_kernel(MlaParams p, uint32_t s
     for (uint32_t s = lane; s < splits; s += 32u) weight[s] *= inv;
   }
   __syncthreads();
-  for (uint32_t r = threadIdx.x; r < p.rank; r += blockDim.x) {
-    float a = 0.0f;
-    uint32_t s = 0;
-    for (; s + 8u <= splits; s += 8u) {
-      float v[8];
+  for (uint32_t r = 2u * threadIdx.x; r < p.rank; r += 2u * blockDim.x) {
+    float2 a = make_float2(0.0f, 0.0f);
+    const float *part = p.partial_acc + static_cast<uint64_t>(h) * slots * p.rank + r;
+    constexpr uint32_t kBatch = 16;  // loads in flight: a span is a round trip to L2 otherwise
+    for (uint32_t s = 0; s < splits; s += kBatch) {
+      float2 v[kBatch];
 #pragma unroll
-      for (uint32_t u = 0; u < 8u; ++u) v[u] = __ldcg(p.partial_acc + (static_cast<uint64_t>(h) * slots + s + u) * p.rank + r);
+      for (uint32_t u = 0; u < kBatch; ++u)
+        v[u] = s + u < splits ? __ldcg(reinterpret_cast<const float2 *>(part + static_cast<uint64_t>(s + u) * p.rank)) : make_float2(0.0f, 0.0f);
 #pragma unroll
-      for (uint32_t u = 0; u < 8u; ++u) a = fmaf(v[u], weight[s + u], a);
+      for (uint32_t u = 0; u < kBatch; ++u) {
+        if (s + u >= splits) break;
+        a.x = fmaf(v[u].x, weight[s + u], a.x);
+        a.y = fmaf(v[u].y, weight[s + u], a.y);
+      }
     }
-    for (; s < splits; ++s)
-      a = fmaf(__ldcg(p.partial_acc + (static_cast<uint64_t>(h) * slots + s) * p.rank + r), weight[s], a);
-    lat[r] = a;
+    *reinterpret_cast<float2 *>(lat + r) = a;
   }
   __syncthreads();
   // out[v] = sum_r lat[r] W_UV[h][v][r]: one warp per output row, 16-byte loads along r; block
   // (h, y) takes rows y * warps .. of the head (the merge above is repeated by the head's blocks:
   // it reads a few KB that stay in L2, the value projection reads the weights)
-  const uint16_t *w_uv = p.w_kv_b + (static_cast<uint64_t>(h) * (p.nope + p.v_dim) + p.nope) * p.rank;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  for (uint32_t v = blockIdx.y * warps + warp; v < p.v_dim; v += gridDim.y * warps) {
+  for (uint32_t v = v0; v < p.v_dim; v += gridDim.y * warps) {
     const uint4 *row = reinterpret_cast<const uint4 *>(w_uv + static_cast<uint64_t>(v) * p.rank);
     float acc = 0.0f;
-    for (uint32_t i = lane; i < p.rank / 8u; i += 32u) {
-      const uint4 w = row[i];
+#pragma unroll
+    for (uint32_t k = 0; k < kKeep; ++k) {
+      const uint32_t i = lane + 32u * k;
+      if (i >= p.rank / 8u) break;
+      const uint4 w = v == v0 ? kept[k] : row[i];
       const float *x = lat + 8u * i;
       acc = fmaf(bf16x2_lo(w.x), x[0], acc);
       acc = fmaf(bf16x2_hi(w.x), x[1], acc);

@@ -118,6 +118,20 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, float *v) {
   for (uint32_t i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// A block that gives up a wait still owns what it has issued: its shared memory and its tensor memory go to the next block
+// of the SM only when the copies into its rings have landed and its MMAs are done, or a bounded wait for them has run out.
+__device__ __forceinline__ void drain_copies(uint64_t *full, uint32_t stages) {
+  for (uint32_t s = 0; s < stages; ++s) {
+    mbar_wait_bounded(&full[s], 0);
+    mbar_wait_bounded(&full[s], 1);
+  }
+}
+// By the thread that issued the MMAs; `bar` has one arrival and no other use.
+__device__ __forceinline__ void drain_mmas(uint64_t *bar) {
+  tcgen05_commit(bar);
+  mbar_wait_bounded(bar, 0);
+}
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (one swizzle atom):
 // start address, 8-row groups 1024 bytes apart, SWIZZLE_128B, descriptor version 1.
 __device__ __forceinline__ uint64_t kmajor_sw128_desc(const void *tile) {

@@ -54,6 +54,7 @@ constexpr uint32_t kSmallBlockTokens = 64;
 struct GemmShared {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t drained;
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -215,6 +216,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       mbar_init(&sh.acc_full[a], 1);
       mbar_init(&sh.acc_empty[a], kEpilogueThreads);
     }
+    mbar_init(&sh.drained, 1);
     sh.abort = 0;
     mbar_init_fence();
     const uint64_t w_policy = l2_evict_first_policy();  // weights are read once
@@ -345,12 +347,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   // ---- teardown: nothing of this block may still be in flight when its memory is released ----
   tcgen05_fence_before();
   __syncthreads();
-  if (sh.abort != 0u && threadIdx.x == 0) {
-    // a wait gave up: give the copies that were issued one more bounded chance to land
-    for (uint32_t s = 0; s < p.stages; ++s) {
-      mbar_wait_bounded(&sh.full[s], 0);
-      mbar_wait_bounded(&sh.full[s], 1);
-    }
+  if (sh.abort != 0u) {
+    if (threadIdx.x == 0) drain_copies(sh.full, p.stages);
+    if (warp == 1 && lane == 0) drain_mmas(&sh.drained);
   }
   __syncthreads();
   if (warp == 1) {

@@ -38,6 +38,7 @@ constexpr uint32_t kLeaderMask = 0xfeffffffu;   // clears the bit of a shared::c
 struct WideShared {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t drained;
   uint32_t tmem_base;
   uint32_t abort;
 };
@@ -70,11 +71,11 @@ __device__ __forceinline__ void pair_mma(uint32_t tmem_d, uint64_t desc_a, uint6
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrives at the same barrier of both blocks once the MMAs issued so far are done.
-__device__ __forceinline__ void pair_commit(uint64_t *bar) {
+// Arrives at the same barrier of the blocks in `mask` (bit 0: the pair's first) once the MMAs issued so far are done.
+__device__ __forceinline__ void pair_commit(uint64_t *bar, uint16_t mask = 3) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_addr(bar)),
-      "h"(static_cast<uint16_t>(3))
+      "h"(mask)
       : "memory");
 }
 // Arrives at a barrier of the pair's first block.
@@ -112,6 +113,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       mbar_init(&sh.acc_full[a], 1);
       mbar_init(&sh.acc_empty[a], 2u * kEpilogueWarps);  // the epilogue warps of both blocks
     }
+    mbar_init(&sh.drained, 1);
     sh.abort = 0;
     mbar_init_fence();
   }
@@ -207,11 +209,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   // ---- teardown: the pair leaves together, with nothing in flight ----
   tcgen05_fence_before();
   __syncthreads();
-  if (sh.abort != 0u && threadIdx.x == 0 && rank == 0) {
-    // a wait gave up: give the copies that were issued, the other block's too, one more bounded chance to land
-    for (uint32_t s = 0; s < p.stages; ++s) {
-      mbar_wait_bounded(&sh.full[s], 0);
-      mbar_wait_bounded(&sh.full[s], 1);
+  if (sh.abort != 0u && rank == 0) {  // the first block counts the copies of both and issues the MMAs
+    if (threadIdx.x == 0) drain_copies(sh.full, p.stages);
+    if (warp == 1 && lane == 0) {
+      pair_commit(&sh.drained, 1);
+      mbar_wait_bounded(&sh.drained, 0);
     }
   }
   __syncthreads();

@@ -236,6 +236,7 @@ struct ExpertGemm {
 struct ExpertShared {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t drained;
   uint32_t tmem_base, abort;
   uint32_t first_tile[kMoeMaxExperts + 1];
 };
@@ -288,6 +289,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       mbar_init(&sh.acc_full[a], 1);
       mbar_init(&sh.acc_empty[a], kEpilogueThreads);
     }
+    mbar_init(&sh.drained, 1);
     sh.abort = 0;
     mbar_init_fence();
   }
@@ -429,11 +431,9 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   // ---- teardown: nothing stays in flight ----
   tcgen05_fence_before();
   __syncthreads();
-  if (sh.abort != 0u && threadIdx.x == 0) {
-    for (uint32_t s = 0; s < g.stages; ++s) {
-      mbar_wait_bounded(&sh.full[s], 0);
-      mbar_wait_bounded(&sh.full[s], 1);
-    }
+  if (sh.abort != 0u) {
+    if (threadIdx.x == 0) drain_copies(sh.full, g.stages);
+    if (warp == 1 && lane == 0) drain_mmas(&sh.drained);
   }
   __syncthreads();
   if (warp == 1) {

@@ -49,6 +49,7 @@ struct AttentionShared {
   uint64_t s_full[2], p_full[2];
   uint64_t pv_done[2];  // PV of a group's tile
   uint64_t o_done;      // the last PV
+  uint64_t drained;
   float m[2][kRows], l[2][kRows];  // the groups' softmax states
   uint32_t tmem_base;
   uint32_t abort;
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
       mbar_init(&sh.pv_done[i], 1);
     }
     mbar_init(&sh.o_done, 1);
+    mbar_init(&sh.drained, 1);
     sh.abort = 0;
     mbar_init_fence();
   }
@@ -400,7 +402,14 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
       }
     }
   }
+  // ---- teardown: nothing stays in flight ----
   tcgen05_fence_before();
+  __syncthreads();
+  if (sh.abort != 0u) {
+    if (threadIdx.x == 0) drain_copies(sh.k_full, kStages);
+    if (threadIdx.x == 32) drain_copies(sh.v_full, kStages);
+    if (warp == kMmaWarp && lane == 0) drain_mmas(&sh.drained);
+  }
   __syncthreads();
   if (warp == kMmaWarp) {
     tcgen05_fence_after();

@@ -1,0 +1,44 @@
+"""Rules that the tensor-pipe kernels keep on paths no test may take on a GPU (a wait that gives up, a circular wait),
+checked on their sources."""
+import glob
+import os
+import re
+
+import pytest
+
+from tests.conftest import ROOT
+
+CSRC = os.path.join(ROOT, "nerva_b200", "csrc")
+
+
+def _kernels():
+    """name -> body of every kernel that allocates tensor memory."""
+    out = {}
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        text = open(path).read()
+        for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\([^{]*\)\s*\{", text):
+            end = text.index("\n}\n", m.end())
+            body = text[m.end():end]
+            if "tcgen05.alloc" in body:
+                out[m.group(1)] = body
+    return out
+
+
+KERNELS = _kernels()
+
+
+def test_all_tensor_memory_kernels_are_looked_at():
+    assert set(KERNELS) == {"gemm_tc_kernel", "gemm_wide_kernel", "moe_block_gemm_kernel", "prefill_attention_kernel"}
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_a_block_that_gave_up_drains_before_it_frees_tensor_memory(name):
+    body = KERNELS[name]
+    teardown = body[body.rindex("sh.abort != 0u"):body.index("tcgen05.dealloc")]
+    rings = set(re.findall(r"mbar_arrive_expect_tx\(&sh\.(\w*full)", body))  # named directly ...
+    rings |= {r for r in ("k_full", "v_full") if f"&sh.{r}[st]" in body}     # ... or through a choice of two
+    assert rings
+    for ring in rings:
+        assert f"drain_copies(sh.{ring}," in teardown, ring
+    assert "drain_mmas(&sh.drained)" in teardown or "mbar_wait_bounded(&sh.drained, 0)" in teardown
+    assert teardown.count("__syncthreads();") == 1  # the drains end before the memory is freed

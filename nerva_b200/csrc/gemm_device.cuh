@@ -76,6 +76,11 @@ __device__ __forceinline__ bool abortable_wait(uint64_t *bar, uint32_t parity, v
     }
   }
 }
+// All lanes of a warp wait; false for all of them when one gave up: what a wait in front of warp-wide tensor-memory accesses
+// has to be, since each lane runs out of time, or sees the abort flag, by itself.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort, uint32_t *error_word) {
+  return __all_sync(0xffffffffu, abortable_wait(bar, parity, abort, error_word));
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }

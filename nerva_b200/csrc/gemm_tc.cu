@@ -317,7 +317,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const uint64_t slot_floats = static_cast<uint64_t>(p.n_pad) * kTileRows;
     while (walk.next(&seg)) {
       const uint32_t acc = segment_index & 1u;
-      if (!abortable_wait(&sh.acc_full[acc], (segment_index >> 1) & 1u, abort, p.error_word)) break;
+      if (!warp_wait(&sh.acc_full[acc], (segment_index >> 1) & 1u, abort, p.error_word)) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * acc_stride + ((quarter * 32u) << 16);
       const bool whole = seg.slice_begin == 0 && seg.slice_end == part.slices;

@@ -190,7 +190,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     uint32_t index = 0;
     for (uint32_t tile = pair; tile < tiles; tile += pairs, ++index) {
       const uint32_t acc = index & 1u;
-      if (!abortable_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, p.error_word)) break;
+      if (!warp_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, p.error_word)) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * kAccStride + ((quarter * 32u) << 16);
       const uint32_t row = (tile / t.token_tiles) * kPairRows + rank * kTileRows + quarter * 32u + lane;

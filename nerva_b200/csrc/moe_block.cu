@@ -390,8 +390,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++index) {
       const uint32_t acc = index & 1u;
       const ExpertTile t = expert_tile(g, sh, tile);
-      // all lanes leave together: the accumulator loads are warp-wide
-      if (!__all_sync(0xffffffffu, abortable_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, g.error_word))) break;
+      if (!warp_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, g.error_word)) break;
       tcgen05_fence_after();
       const uint32_t d0 = tmem_base + acc * 2u * g.tile_tokens + ((quarter * 32u) << 16), d1 = d0 + g.tile_tokens;
       const uint32_t row = t.row + quarter * 32u + lane;

@@ -103,11 +103,6 @@ __device__ __forceinline__ float exp2_ftz(float x) {
   return y;
 }
 
-// All lanes of a warp wait; false for all of them when one gave up.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort, uint32_t *error_word) {
-  return __all_sync(0xffffffffu, abortable_wait(bar, parity, abort, error_word));
-}
-
 template <uint32_t D, bool EXTRAS>
 __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                const __grid_constant__ CUtensorMap map_v,

@@ -42,3 +42,14 @@ def test_a_block_that_gave_up_drains_before_it_frees_tensor_memory(name):
         assert f"drain_copies(sh.{ring}," in teardown, ring
     assert "drain_mmas(&sh.drained)" in teardown or "mbar_wait_bounded(&sh.drained, 0)" in teardown
     assert teardown.count("__syncthreads();") == 1  # the drains end before the memory is freed
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_waits_in_front_of_warp_wide_accesses_are_taken_by_the_whole_warp(name):
+    """Between a wait that a single lane may leave early and the role's end there is no tensor-memory access of the warp."""
+    body = KERNELS[name]
+    for wait in re.finditer(r"\babortable_wait\(", body):
+        role = body[wait.end():]
+        ends = [role.find(end) for end in ("} else if (warp", "} else {\n    // ------", "} else {\n    const uint32_t quarter",
+                                           "// ---- teardown") if end in role]
+        assert not re.search(r"tmem_(load|store)\w*\(|tcgen05\.(ld|st)", role[:min(ends)]), role[:80]

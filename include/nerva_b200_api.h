@@ -1013,6 +1013,10 @@ int nerva_b200_projection_sustained(const uint16_t *weight, const uint16_t *x, f
                                     uint32_t cols, uint32_t tokens, uint32_t copies, uint32_t warmup,
                                     uint32_t iterations, uint64_t *avg_ns);
 
+/* Dynamic shared memory (bytes) and tensor memory (columns) of every shape the kernels with tensor memory are launched
+ * with; returns their number, of which up to `capacity` are written.  Needs no device. */
+int nerva_b200_tensor_memory_launches(uint32_t *smem_bytes, uint32_t *columns, uint32_t capacity);
+
 /* Isolated GQA paged decode attention for `batch` sequences of `context`
  * tokens each: q f32 [batch][heads*head_dim]; K/V pages bf16
  * [batch][pages][16][kv_heads*head_dim]; page_table uint32 [batch][pages];

@@ -15,6 +15,21 @@ constexpr uint32_t kUmmaK = 16;       // inner elements per MMA instruction
 constexpr uint32_t kATileBytes = kTileRows * kSliceK * 2u;
 constexpr uint32_t kGroup = 16;       // tokens per tcgen05.ld
 
+// The 512 columns of an SM's tensor memory are shared by the blocks that are resident together, and an allocation that does
+// not fit waits until another block leaves.  With programmatic dependent launch the other block may be of a later launch
+// that waits for this one's end, so blocks that can be resident together must never ask for more than there is.  Launches
+// of up to kSharedColumns may share an SM (four of them fit); a launch that takes more asks for so much shared memory that
+// no other block with tensor memory fits beside it, whatever registers and launch order would allow.
+constexpr uint32_t kSharedColumns = 128;
+constexpr uint32_t kSmemPerSm = 228u * 1024u, kSmemReserved = 1024u;  // per SM; by the system, per block
+constexpr uint32_t kLeastTmemSmem = 88u * 1024u;                      // of every launch with tensor memory
+constexpr uint32_t kAloneTmemSmem = kSmemPerSm - 2u * kSmemReserved - kLeastTmemSmem + 128u;
+// Dynamic shared memory of a launch that takes `columns` of tensor memory and needs `bytes`.
+__host__ __device__ constexpr uint32_t tensor_memory_smem(uint32_t columns, uint32_t bytes) {
+  const uint32_t least = columns > kSharedColumns ? kAloneTmemSmem : kLeastTmemSmem;
+  return bytes > least ? bytes : least;
+}
+
 struct GemmKernelParams {
   uint32_t rows, cols, tokens, n_pad;  // n_pad: tokens rounded up to 16 (the MMA N)
   uint32_t stages;

@@ -402,7 +402,8 @@ uint32_t stages_for(uint32_t n_pad) {
 uint32_t tmem_columns_for(uint32_t n_pad) { return two_blocks_per_sm(n_pad) ? 128u : 512u; }
 
 uint32_t gemm_smem_bytes(uint32_t n_pad, uint32_t stages) {
-  return 1024u + stages * (kATileBytes + n_pad * kSliceK * 2u) + static_cast<uint32_t>(sizeof(GemmShared)) + 64u;
+  const uint32_t bytes = 1024u + stages * (kATileBytes + n_pad * kSliceK * 2u) + static_cast<uint32_t>(sizeof(GemmShared)) + 64u;
+  return tensor_memory_smem(tmem_columns_for(n_pad), bytes);
 }
 
 // Two runs per SM whatever the block size, so that the split points — and with them the order in
@@ -451,6 +452,11 @@ bool gemm_wide_eligible(const GemmParams &g) { return g.tokens > kGemmMaxTokens 
 uint64_t gemm_tc_workspace_bytes(uint32_t tokens, uint32_t sm_count) {
   // two partial accumulators per thread block of the 2 x sm_count grid
   return 2ull * (2ull * sm_count) * padded_tokens(tokens) * kTileRows * sizeof(float);
+}
+
+void gemm_tc_launches(std::vector<TensorMemoryLaunch> *out) {
+  for (uint32_t n_pad = 16; n_pad <= kGemmMaxTokens; n_pad += 16)
+    out->push_back({gemm_smem_bytes(n_pad, stages_for(n_pad)), tmem_columns_for(n_pad)});
 }
 
 uint32_t gemm_tc_ticket_count(uint32_t rows) { return (rows + kTileRows - 1u) / kTileRows; }

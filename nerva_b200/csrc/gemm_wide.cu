@@ -27,7 +27,7 @@ namespace nb {
 namespace {
 
 constexpr uint32_t kPairRows = 2u * kTileRows;  // MMA M over the pair
-constexpr uint32_t kMaxTileTokens = 256;        // MMA N
+constexpr uint32_t kMinTileTokens = 64, kMaxTileTokens = 256;  // MMA N
 constexpr uint32_t kTokenStep = 32;             // tile sizes: whole 8-row swizzle atoms in each half, N a multiple of 16
 constexpr uint32_t kMaxStages = 8;
 constexpr uint32_t kThreads = 192;
@@ -231,6 +231,11 @@ uint32_t wide_stages(uint32_t tile_tokens) {
   return stages < kMaxStages ? stages : kMaxStages;
 }
 
+uint32_t wide_smem_bytes(uint32_t tile_tokens) {
+  return tensor_memory_smem(kTmemColumns, 1024u + wide_stages(tile_tokens) * wide_stage_bytes(tile_tokens) +
+                                              static_cast<uint32_t>(sizeof(WideShared)) + 64u);
+}
+
 // Tokens per tile: the size with the shortest run of the slowest pair.  A slice costs a pair the larger of its MMA
 // time (2 cycles per token) and the time its shared memory takes to fill (about 45 bytes per cycle and SM with all
 // SMs loading), so narrow tiles pay for the weight rows they re-read; wide ones may leave a last wave nearly empty.
@@ -238,7 +243,7 @@ uint32_t choose_tile_tokens(uint32_t rows, uint32_t tokens, uint32_t pairs) {
   const uint32_t row_tiles = (rows + kPairRows - 1u) / kPairRows;
   uint32_t best = kMaxTileTokens;
   uint64_t best_cost = ~0ull;
-  for (uint32_t n = kMaxTileTokens; n >= 64u; n -= kTokenStep) {
+  for (uint32_t n = kMaxTileTokens; n >= kMinTileTokens; n -= kTokenStep) {
     const uint32_t tiles = row_tiles * ((tokens + n - 1u) / n);
     const uint64_t waves = (tiles + pairs - 1u) / pairs;
     const uint64_t fill = wide_stage_bytes(n) / 45u, mma = 2u * n;
@@ -257,6 +262,10 @@ cudaError_t configure_gemm_wide_kernel() {
   return cudaFuncSetAttribute(gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 
+void gemm_wide_launches(std::vector<TensorMemoryLaunch> *out) {
+  for (uint32_t n = kMinTileTokens; n <= kMaxTileTokens; n += kTokenStep) out->push_back({wide_smem_bytes(n), kTmemColumns});
+}
+
 cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t sm_count) {
   const uint32_t pairs = sm_count / 2u;
   WideTiles t{};
@@ -270,9 +279,8 @@ cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t 
       !encode_bf16_map_2d(&map_x, g.x, g.cols, g.tokens, kSliceK, t.tile_tokens / 2u))
     return cudaErrorNotSupported;
   const uint32_t tiles = t.row_tiles * t.token_tiles;
-  const uint32_t smem = 1024u + p.stages * wide_stage_bytes(t.tile_tokens) + static_cast<uint32_t>(sizeof(WideShared)) + 64u;
-  return launch_with_pdl(gemm_wide_kernel, dim3(2u * (tiles < pairs ? tiles : pairs)), dim3(kThreads), smem, stream,
-                         g.pdl != 0, map_w, map_x, p, t);
+  return launch_with_pdl(gemm_wide_kernel, dim3(2u * (tiles < pairs ? tiles : pairs)), dim3(kThreads),
+                         wide_smem_bytes(t.tile_tokens), stream, g.pdl != 0, map_w, map_x, p, t);
 }
 
 }  // namespace nb

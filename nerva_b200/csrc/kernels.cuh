@@ -102,6 +102,16 @@ struct ProjectionParams {
 
 constexpr uint32_t kTimelineSlots = 8;
 
+// Shared and tensor memory of a launch: what decides which blocks can be resident together (gemm_device.cuh).
+struct TensorMemoryLaunch {
+  uint32_t smem, columns;
+};
+// Appends every shape that the file's kernel is launched with.
+void gemm_tc_launches(std::vector<TensorMemoryLaunch> *out);
+void gemm_wide_launches(std::vector<TensorMemoryLaunch> *out);
+void moe_block_launches(std::vector<TensorMemoryLaunch> *out);
+void prefill_attention_launches(std::vector<TensorMemoryLaunch> *out);
+
 // ---- block projection on the tensor pipe: up to 256 tokens bound by the weight stream (gemm_tc.cu), more by the
 // tensor pipe (gemm_wide.cu) ----
 constexpr uint32_t kGemmMaxTokens = 256;

@@ -267,6 +267,8 @@ __device__ __forceinline__ ExpertTile expert_tile(const ExpertGemm &g, const Exp
   return t;
 }
 
+__host__ __device__ constexpr uint32_t expert_columns(uint32_t tile_tokens) { return 4u * tile_tokens; }  // two buffers of two accumulators
+
 __global__ void __launch_bounds__(kThreads, 1)
 moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo, ExpertGemm g) {
@@ -277,7 +279,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   ExpertShared &sh = *reinterpret_cast<ExpertShared *>(ring + g.stages * stage_bytes);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   volatile uint32_t *abort = &sh.abort;
-  const uint32_t tmem_columns = 4u * g.tile_tokens;  // two buffers of two accumulators
+  const uint32_t tmem_columns = expert_columns(g.tile_tokens);
 
   pdl_trigger();
   if (threadIdx.x == 0) {
@@ -449,6 +451,13 @@ uint32_t expert_tile_tokens(uint32_t tokens, uint32_t groups) {
   return room <= 32u ? 32u : room <= 64u ? 64u : kMaxTokens;
 }
 
+uint32_t expert_stage_bytes(uint32_t tile_tokens) { return 2u * kATileBytes + 2u * tile_tokens * kSliceK * 2u; }
+uint32_t expert_stages(uint32_t tile_tokens) { return std::min(kMaxStages, 216u * 1024u / expert_stage_bytes(tile_tokens)); }
+uint32_t expert_smem_bytes(uint32_t tile_tokens) {
+  return tensor_memory_smem(expert_columns(tile_tokens), 1024u + expert_stages(tile_tokens) * expert_stage_bytes(tile_tokens) +
+                                                             static_cast<uint32_t>(sizeof(ExpertShared)) + 64u);
+}
+
 struct ExpertOperands {
   const uint16_t *a, *b;      // weights: first and second tile of a pair
   uint64_t map_rows_a, map_rows_b;
@@ -460,8 +469,7 @@ struct ExpertOperands {
 cudaError_t launch_expert_gemm(cudaStream_t stream, ExpertGemm g, const ExpertOperands &o, uint32_t sm_count, bool pdl) {
   g.tile_tokens = expert_tile_tokens(o.x_rows, g.groups);
   g.slices = (o.cols + kSliceK - 1u) / kSliceK;
-  const uint32_t stage_bytes = 2u * kATileBytes + 2u * g.tile_tokens * kSliceK * 2u;
-  g.stages = std::min(kMaxStages, 216u * 1024u / stage_bytes);
+  g.stages = expert_stages(g.tile_tokens);
   CUtensorMap map_a, map_b, map_hi, map_lo;
   if (!encode_bf16_map_2d(&map_a, o.a, o.cols, o.map_rows_a, kSliceK, kTileRows) ||
       !encode_bf16_map_2d(&map_b, o.b, o.cols, o.map_rows_b, kSliceK, kTileRows) ||
@@ -472,8 +480,8 @@ cudaError_t launch_expert_gemm(cudaStream_t stream, ExpertGemm g, const ExpertOp
   const uint64_t row_tiles = (g.rows + g.step - 1u) / g.step;
   const uint64_t most = row_tiles * (o.x_rows / g.tile_tokens + std::min(g.groups, o.x_rows));
   const uint32_t blocks = static_cast<uint32_t>(std::min<uint64_t>(most, sm_count));
-  const uint32_t smem = 1024u + g.stages * stage_bytes + static_cast<uint32_t>(sizeof(ExpertShared)) + 64u;
-  return launch_with_pdl(moe_block_gemm_kernel, dim3(blocks), dim3(kThreads), smem, stream, pdl, map_a, map_b, map_hi, map_lo, g);
+  return launch_with_pdl(moe_block_gemm_kernel, dim3(blocks), dim3(kThreads), expert_smem_bytes(g.tile_tokens), stream, pdl, map_a,
+                         map_b, map_hi, map_lo, g);
 }
 
 uint32_t route_rows(uint32_t hidden, uint32_t experts) {
@@ -497,6 +505,10 @@ cudaError_t configure_moe_block() {
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(moe_block_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
   return err;
+}
+
+void moe_block_launches(std::vector<TensorMemoryLaunch> *out) {
+  for (uint32_t tokens : {32u, 64u, kMaxTokens}) out->push_back({expert_smem_bytes(tokens), expert_columns(tokens)});
 }
 
 cudaError_t launch_moe_block(cudaStream_t stream, const MoeBlockParams &p, uint32_t sm_count, bool pdl, uint64_t *launches) {

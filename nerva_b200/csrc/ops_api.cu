@@ -300,6 +300,19 @@ extern "C" int nerva_b200_projection_sustained(const uint16_t *weight, const uin
   return 0;
 }
 
+extern "C" int nerva_b200_tensor_memory_launches(uint32_t *smem_bytes, uint32_t *columns, uint32_t capacity) {
+  std::vector<TensorMemoryLaunch> all;
+  gemm_tc_launches(&all);
+  gemm_wide_launches(&all);
+  moe_block_launches(&all);
+  prefill_attention_launches(&all);
+  for (uint32_t i = 0; i < all.size() && i < capacity && smem_bytes != nullptr && columns != nullptr; ++i) {
+    smem_bytes[i] = all[i].smem;
+    columns[i] = all[i].columns;
+  }
+  return static_cast<int>(all.size());
+}
+
 // Reference: native/cuda/nerva_cuda_projection_bench.cu.  Same deterministic
 // inputs (((17 i + 13) mod 127) - 63) / 128 for the matrix and the vector
 // (:38-41,84-101).  `custom_*` time this library's projection kernel as single

@@ -414,7 +414,8 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
 
 template <uint32_t D>
 constexpr uint32_t attention_smem() {
-  return 1024u + (2u + 2u * kStages) * (D / 64u) * kBlockBytes + static_cast<uint32_t>(sizeof(AttentionShared)) + 64u;
+  return tensor_memory_smem(kTmemAll, 1024u + (2u + 2u * kStages) * (D / 64u) * kBlockBytes +
+                                          static_cast<uint32_t>(sizeof(AttentionShared)) + 64u);
 }
 
 }  // namespace
@@ -433,6 +434,11 @@ cudaError_t configure_prefill_attention() {
   set(prefill_attention_kernel<128, false>, attention_smem<128>());
   set(prefill_attention_kernel<128, true>, attention_smem<128>());
   return err;
+}
+
+void prefill_attention_launches(std::vector<TensorMemoryLaunch> *out) {
+  out->push_back({attention_smem<64>(), kTmemAll});
+  out->push_back({attention_smem<128>(), kTmemAll});
 }
 
 cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p) {

@@ -4,6 +4,7 @@ import glob
 import os
 import re
 
+import numpy as np
 import pytest
 
 from tests.conftest import ROOT
@@ -53,3 +54,18 @@ def test_waits_in_front_of_warp_wide_accesses_are_taken_by_the_whole_warp(name):
         ends = [role.find(end) for end in ("} else if (warp", "} else {\n    // ------", "} else {\n    const uint32_t quarter",
                                            "// ---- teardown") if end in role]
         assert not re.search(r"tmem_(load|store)\w*\(|tcgen05\.(ld|st)", role[:min(ends)]), role[:80]
+
+
+def test_blocks_that_fit_on_an_sm_together_never_ask_for_more_tensor_memory_than_there_is(built_lib):
+    """An allocation that does not fit waits for another block to leave, and that block may be of a dependent launch that
+    waits for this one: so no set of blocks whose shared memory fits an SM may exceed its 512 columns."""
+    smem, columns = np.zeros(256, np.uint32), np.zeros(256, np.uint32)
+    n = built_lib.nerva_b200_tensor_memory_launches(smem.ctypes.data, columns.ctypes.data, 256)
+    shapes = sorted({(int(s), int(c)) for s, c in zip(smem[:n], columns[:n])})
+    assert 4 <= n <= 256 and all(c in (128, 256, 512) and 0 < s <= 227 * 1024 for s, c in shapes)
+    per_sm, reserved = 228 * 1024, 1024  # shared memory of an SM; what the system takes of it per block
+
+    def most_columns(room):
+        return max((c + most_columns(room - s - reserved) for s, c in shapes if s + reserved <= room), default=0)
+
+    assert most_columns(per_sm) <= 512

@@ -1017,6 +1017,9 @@ int nerva_b200_projection_sustained(const uint16_t *weight, const uint16_t *x, f
  * with; returns their number, of which up to `capacity` are written.  Needs no device. */
 int nerva_b200_tensor_memory_launches(uint32_t *smem_bytes, uint32_t *columns, uint32_t capacity);
 
+/* Thread blocks of the state-space scan that one SM holds, for a state of `state` values per channel; -1 on an error. */
+int nerva_b200_state_space_scan_blocks_per_sm(uint32_t state);
+
 /* Isolated GQA paged decode attention for `batch` sequences of `context`
  * tokens each: q f32 [batch][heads*head_dim]; K/V pages bf16
  * [batch][pages][16][kv_heads*head_dim]; page_table uint32 [batch][pages];

@@ -562,9 +562,11 @@ struct StateSpaceParams {
   // block step: the rows' positions and sessions
   const struct FusedAttentionRow *rows;
   uint32_t row_count;
+  uint32_t sm_count;
 };
 bool state_space_supported(const StateSpaceShape &s);
 cudaError_t configure_state_space();
+cudaError_t state_space_scan_blocks_per_sm(const StateSpaceShape &s, int *blocks);
 // One token per row: the lone step (rows == nullptr) or rows of different sessions.
 cudaError_t launch_state_space_step(cudaStream_t stream, const StateSpaceParams &p);
 // Consecutive positions of one session: convolution, then the recurrence (two launches).

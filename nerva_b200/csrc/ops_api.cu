@@ -313,6 +313,17 @@ extern "C" int nerva_b200_tensor_memory_launches(uint32_t *smem_bytes, uint32_t 
   return static_cast<int>(all.size());
 }
 
+extern "C" int nerva_b200_state_space_scan_blocks_per_sm(uint32_t state) {
+  StateSpaceShape s{};
+  s.heads = s.groups = s.taps = s.norm_groups = 1;
+  s.v_dim = 64;
+  s.state = state;
+  int blocks = 0;
+  const cudaError_t err = state_space_supported(s) ? state_space_scan_blocks_per_sm(s, &blocks) : cudaErrorInvalidValue;
+  if (err != cudaSuccess) set_last_error(cudaGetErrorString(err));
+  return err == cudaSuccess ? blocks : -1;
+}
+
 // Reference: native/cuda/nerva_cuda_projection_bench.cu.  Same deterministic
 // inputs (((17 i + 13) mod 127) - 63) / 128 for the matrix and the vector
 // (:38-41,84-101).  `custom_*` time this library's projection kernel as single

@@ -36,6 +36,7 @@ StateSpaceParams layer_state_space(const Session *s, const ParallelLayerPlan &l,
   p.history_offset = run.history_offset;
   p.f32 = s->parallel->f32 ? 1u : 0u;
   p.pdl = s->use_pdl ? 1u : 0u;
+  p.sm_count = s->sm_count;
   return p;
 }
 

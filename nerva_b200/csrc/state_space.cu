@@ -378,7 +378,11 @@ constexpr uint32_t kChunk = 64;
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanWarps = kScanThreads / 32u;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr uint32_t kScanMaxRows = 2048;  // rows of a block (24 KB of steps and decays)
+// Step sizes and decays are kept for kStepChunks chunks at a time, a chunk per warp, and made again when they are used up.
+// Arrays for all of a block's rows (24 KB at 2048) left room for one thread block per SM where two fit at a state of 128,
+// which at hidden 4096 (256 thread blocks) is a second wave: 2048 tokens through 8 layer runs, 4 of them scans, 11.1 ms; 10.3
+// so.
+constexpr uint32_t kStepChunks = 4, kStepRows = kStepChunks * kChunk;
 
 __device__ __forceinline__ void cp_async_16(void *dst, const void *src, bool valid) {  // zeros when not valid
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16u : 0u)
@@ -409,7 +413,7 @@ template <uint32_t MT>
 __global__ void __launch_bounds__(kScanThreads) state_space_scan_kernel(StateSpaceParams p) {
   constexpr uint32_t NT = kColumns / 8u, YT = NT / 2u;
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ float log_decay_all[kScanMaxRows], steps_all[kScanMaxRows], to_end_all[kScanMaxRows];
+  __shared__ float log_decay_all[kStepRows], steps_all[kStepRows], to_end_all[kStepRows];
   const StateSpaceShape &s = p.s;
   const ScanLayout L(s);
   uint8_t *fed_hi = smem + 2u * L.stage, *fed_lo = fed_hi + L.fed;
@@ -485,16 +489,23 @@ __global__ void __launch_bounds__(kScanThreads) state_space_scan_kernel(StateSpa
 
   const uint32_t chunks = (p.row_count + kChunk - 1u) / kChunk;
   issue(0);
-  for (uint32_t chunk = warp; chunk < chunks; chunk += kScanWarps) {
-    // step sizes and their running sums, a chunk per warp: tokens 2 lane, 2 lane + 1; rows behind the block change nothing
-    float d[2], sum[2];
+  // the step inputs of this warp's next chunk, on their way a chunk ahead of their use
+  float raw[2];
+  auto load_steps = [&](uint32_t first_chunk) {
+    if (warp >= kStepChunks) return;
 #pragma unroll
     for (uint32_t i = 0; i < 2u; ++i) {
-      const uint32_t r = chunk * kChunk + 2u * lane + i;
-      d[i] = r < p.row_count
-                 ? softplus(__ldcg(p.in + static_cast<uint64_t>(r) * p.in_stride + s.inner() + s.channels() + head) + bias)
-                 : 0.0f;
+      const uint32_t r = (first_chunk + warp) * kChunk + 2u * lane + i;
+      raw[i] = r < p.row_count ? __ldcg(p.in + static_cast<uint64_t>(r) * p.in_stride + s.inner() + s.channels() + head) : 0.0f;
     }
+  };
+  // step sizes and their running sums, a chunk per warp: tokens 2 lane, 2 lane + 1; rows behind the block change nothing
+  auto make_steps = [&](uint32_t first_chunk) {
+    if (warp >= kStepChunks) return;
+    float d[2], sum[2];
+#pragma unroll
+    for (uint32_t i = 0; i < 2u; ++i)
+      d[i] = (first_chunk + warp) * kChunk + 2u * lane + i < p.row_count ? softplus(raw[i] + bias) : 0.0f;
     sum[0] = d[0];
     sum[1] = d[0] + d[1];
     float through = sum[1], from = sum[1];  // sums up to and from this lane's tokens
@@ -509,16 +520,19 @@ __global__ void __launch_bounds__(kScanThreads) state_space_scan_kernel(StateSpa
     if (lane == 31) behind = 0.0f;
 #pragma unroll
     for (uint32_t i = 0; i < 2u; ++i) {
-      const uint32_t t = chunk * kChunk + 2u * lane + i;
+      const uint32_t t = warp * kChunk + 2u * lane + i;
       steps_all[t] = d[i];
       log_decay_all[t] = -rate * (before + sum[i]);
       // not a difference of the running sums: the last token's factor is exactly one
       to_end_all[t] = exp2f(-rate * (i == 0 ? behind + d[1] : behind)) * d[i];
     }
-  }
+  };
+  load_steps(0);
   for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
-    const uint32_t first = chunk * kChunk;
-    const float *log_decay = log_decay_all + first, *steps = steps_all + first, *to_end = to_end_all + first;
+    const uint32_t first = chunk * kChunk, kept = chunk % kStepChunks * kChunk;
+    const float *log_decay = log_decay_all + kept, *steps = steps_all + kept, *to_end = to_end_all + kept;
+    if (chunk % kStepChunks == 0) make_steps(chunk);  // the last chunk's use of them ended at its barrier
+    if (chunk % kStepChunks == kStepChunks - 1u) load_steps(chunk + 1u);
     cp_async_wait<0>();
     __syncthreads();  // this chunk's rows and steps are in place; the other stage is free
     if (chunk + 1u < chunks) issue(chunk + 1u);
@@ -708,6 +722,15 @@ __global__ void __launch_bounds__(kGroupThreads) grouped_norm_kernel(const float
 
 uint32_t column_tiles(const StateSpaceShape &s) { return (s.v_dim + kColumns - 1u) / kColumns; }
 
+// Two thread blocks fit an SM up to a state of 128, which pays where there are more of them than SMs; where there are not,
+// each asks for more than half of an SM, or two would share one beside an idle one: a 2048-token prompt through 14
+// scans of 128 thread blocks, 19.3 ms (two may share), 18.2 (alone).
+uint32_t scan_smem(const StateSpaceShape &s, uint32_t sm_count) {
+  constexpr uint32_t kAlone = 116u * 1024u;
+  const uint32_t bytes = ScanLayout(s).total;
+  return column_tiles(s) * s.heads <= sm_count && bytes < kAlone ? kAlone : bytes;
+}
+
 // Rows from which a block runs in chunks on the tensor pipe.
 constexpr uint32_t kScanMinRows = 16;
 
@@ -720,7 +743,7 @@ cudaError_t launch_block(cudaStream_t stream, const StateSpaceParams &p) {
   if (err != cudaSuccess) return err;
   if (sizeof(T) == 2u && p.row_count >= kScanMinRows)
     return launch_with_pdl(s.state <= 128u ? state_space_scan_kernel<1> : state_space_scan_kernel<2>,
-                           dim3(column_tiles(s), s.heads), dim3(kScanThreads), ScanLayout(s).total, stream, p.pdl != 0, p);
+                           dim3(column_tiles(s), s.heads), dim3(kScanThreads), scan_smem(s, p.sm_count), stream, p.pdl != 0, p);
   return launch_with_pdl(s.state <= 128u ? state_space_rows_kernel<T, 16> : state_space_rows_kernel<T, 32>,
                          dim3(column_tiles(s) * s.heads), dim3(kStepThreads), 0, stream, p.pdl != 0, p);
 }
@@ -737,8 +760,15 @@ cudaError_t configure_state_space() {
   cudaError_t err = cudaSuccess;
   for (const void *kernel : {reinterpret_cast<const void *>(state_space_scan_kernel<1>),
                              reinterpret_cast<const void *>(state_space_scan_kernel<2>)})
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024);  // beside the static steps
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   return err;
+}
+
+cudaError_t state_space_scan_blocks_per_sm(const StateSpaceShape &s, int *blocks) {
+  const cudaError_t err = configure_state_space();
+  if (err != cudaSuccess) return err;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      blocks, s.state <= 128u ? state_space_scan_kernel<1> : state_space_scan_kernel<2>, kScanThreads, ScanLayout(s).total);
 }
 
 cudaError_t launch_state_space_step(cudaStream_t stream, const StateSpaceParams &p) {
@@ -754,7 +784,7 @@ cudaError_t launch_state_space_step(cudaStream_t stream, const StateSpaceParams 
 }
 
 cudaError_t launch_state_space_block(cudaStream_t stream, const StateSpaceParams &p) {
-  if (!state_space_supported(p.s) || p.rows == nullptr || p.row_count == 0 || p.row_count > kScanMaxRows || p.convolved == nullptr)
+  if (!state_space_supported(p.s) || p.rows == nullptr || p.row_count == 0 || p.convolved == nullptr)
     return cudaErrorInvalidValue;
   return p.f32 != 0 ? launch_block<float>(stream, p) : launch_block<uint16_t>(stream, p);
 }

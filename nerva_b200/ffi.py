@@ -143,6 +143,7 @@ def _bind(L: C.CDLL, reference_abi_only: bool) -> C.CDLL:
         "nerva_b200_projection_sustained": [vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,
                                             C.c_uint32, P(C.c_uint64)],
         "nerva_b200_tensor_memory_launches": [vp, vp, C.c_uint32],
+        "nerva_b200_state_space_scan_blocks_per_sm": [C.c_uint32],
         "nerva_b200_gqa_decode_attention": [vp, vp, vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,
                                             C.c_uint32, C.c_uint32, C.c_uint32, P(C.c_uint64)],
         "nerva_b200_gqa_decode_attention_sustained": [vp, vp, vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32,

@@ -32,6 +32,10 @@ struct DeviceBuffers {
   }
 };
 
+// Copies and memsets on the null stream may still be queued when they return (of up to 64 KB, or behind the last staging
+// buffer), and the streams of the measurements below do not wait for it.
+cudaError_t inputs_arrived() { return cudaStreamSynchronize(nullptr); }
+
 struct Timing {
   cudaEvent_t a = nullptr, b = nullptr;
   ~Timing() {
@@ -218,6 +222,7 @@ extern "C" int nerva_b200_projection_sustained(const uint16_t *weight, const uin
   if (err == cudaSuccess)
     err = cudaMemset(d_tickets, 0, (static_cast<uint64_t>(gemm_tc_ticket_count(rows)) + 1u) * sizeof(uint32_t));
   if (err == cudaSuccess) err = cudaMemcpy(d_x, x, static_cast<uint64_t>(tokens) * cols * 2u, cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = inputs_arrived();
   if (err == cudaSuccess) err = t.init();
   cudaStream_t stream = nullptr;
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
@@ -259,7 +264,7 @@ extern "C" int nerva_b200_projection_sustained(const uint16_t *weight, const uin
   unsigned long long *d_stamps = nullptr;
   if (block && timeline_env != nullptr && timeline_env[0] == '1' && err == cudaSuccess) {
     err = buf.alloc(&d_stamps, uint64_t{2} * kTimelineSlots);
-    if (err == cudaSuccess) err = cudaMemset(d_stamps, 0, 2 * kTimelineSlots * sizeof(unsigned long long));
+    if (err == cudaSuccess) err = cudaMemsetAsync(d_stamps, 0, 2 * kTimelineSlots * sizeof(unsigned long long), stream);
   }
   for (uint32_t i = 0; err == cudaSuccess && i < warmup; ++i) err = launch(i);
   float ms = 0.0f;
@@ -385,6 +390,7 @@ extern "C" int nerva_cuda_projection_bench(const NervaCudaProjectionBenchRequest
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
   if (err == cudaSuccess) err = cudaMemcpy(d_w, h_w.data(), w_elems * 2u, cudaMemcpyHostToDevice);
   if (err == cudaSuccess) err = cudaMemcpy(d_x, h_x.data(), cols * 2u, cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = inputs_arrived();
   ProjectionParams p{};
   p.weight = d_w;
   p.rows = rows;
@@ -465,6 +471,7 @@ extern "C" int nerva_cuda_projection_bench(const NervaCudaProjectionBenchRequest
     if (err == cudaSuccess)
       err = cudaMemset(d_tickets, 0, (static_cast<uint64_t>(gemm_tc_ticket_count(rows)) + 1u) * sizeof(uint32_t));
     if (err == cudaSuccess) err = cudaMemcpy(d_xb, h_xb.data(), h_xb.size() * 2u, cudaMemcpyHostToDevice);
+    if (err == cudaSuccess) err = inputs_arrived();
     if (err == cudaSuccess) err = configure_gemm_tc_kernel();
     out->device_allocations += 4;
     GemmParams g{};
@@ -603,6 +610,7 @@ extern "C" int nerva_b200_gqa_decode_attention_sustained(const float *q, const u
   if (err == cudaSuccess) err = cudaMemcpy(d_q, q, q_elems * 4u, cudaMemcpyHostToDevice);
   if (err == cudaSuccess)
     err = cudaMemcpy(d_table, page_table, static_cast<uint64_t>(batch) * pages * 4u, cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = inputs_arrived();
   cudaStream_t stream = nullptr;
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
   AttentionParams p{};

@@ -453,6 +453,7 @@ cudaError_t allocate_comm(Session *s) {
   const CommLayout c = comm_layout(s->tp_world, s->dims.hidden);
   cudaError_t err = cudaMalloc(&s->comm_block, c.bytes);
   if (err == cudaSuccess) err = cudaMemset(s->comm_block, 0, c.bytes);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);  // before this session's stream or a peer writes there
   s->comm_bytes = c.bytes;
   return err;
 }
@@ -2742,10 +2743,12 @@ extern "C" int nerva_b200_session_set_kv_block_table(Session *s, const uint32_t 
     if (table[i] >= page_count || seen[table[i]]) return -1;  // must be a permutation
     seen[table[i]] = 1;
   }
-  if (cudaMemcpy(s->page_table, table, static_cast<uint64_t>(page_count) * 4u, cudaMemcpyHostToDevice) !=
-      cudaSuccess)
-    return -1;
-  return 0;
+  // on the session's stream: a copy on the null stream returns when it is staged, and this stream, which does not wait for
+  // that one, could begin the next request with the old table
+  return cudaMemcpyAsync(s->page_table, table, static_cast<uint64_t>(page_count) * 4u, cudaMemcpyHostToDevice, s->stream) ==
+                     cudaSuccess && cudaStreamSynchronize(s->stream) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 extern "C" int nerva_b200_session_get_kv_block_table(Session *s, uint32_t *table, uint32_t capacity) {
@@ -2827,6 +2830,6 @@ extern "C" int nerva_b200_session_read_phase_cycles(Session *s, uint64_t *cycles
   if (cudaStreamSynchronize(s->stream) != cudaSuccess) return -1;
   if (cudaMemcpy(cycles, s->phase_cycles, kPhaseCount * sizeof(uint64_t), cudaMemcpyDeviceToHost) != cudaSuccess)
     return -1;
-  if (cudaMemset(s->phase_cycles, 0, kPhaseCount * sizeof(uint64_t)) != cudaSuccess) return -1;
+  if (cudaMemsetAsync(s->phase_cycles, 0, kPhaseCount * sizeof(uint64_t), s->stream) != cudaSuccess) return -1;
   return static_cast<int>(kPhaseCount);
 }

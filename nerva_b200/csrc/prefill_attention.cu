@@ -382,10 +382,11 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
       float o[16], o1[16];
       tmem_load16(o_addr + c, o);
       tmem_load16(o_addr + D + c, o1);
-      if (!live) continue;
 #pragma unroll
       for (uint32_t i = 0; i < 16u; ++i) o[i] = ((w0 > 0.0f ? o[i] * w0 : 0.0f) + (w1 > 0.0f ? o1[i] * w1 : 0.0f)) * inv;
-      if (vector) {
+      if (!live) {
+        // nothing to store; the warp's next load wants all lanes
+      } else if (vector) {
 #pragma unroll
         for (uint32_t i = 0; i < 16u; i += 8u)
           *reinterpret_cast<uint4 *>(dst + c + i) = make_uint4(pack_bf16_hi(o[i], o[i + 1]), pack_bf16_hi(o[i + 2], o[i + 3]),
@@ -395,6 +396,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
         for (uint32_t i = 0; i < 16u; ++i)
           if (c + i < s.v_dim) dst[c + i] = f32_to_bf16_bits(o[i]);
       }
+      __syncwarp();
     }
   }
   // ---- teardown: nothing stays in flight ----

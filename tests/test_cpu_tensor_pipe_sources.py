@@ -69,3 +69,14 @@ def test_blocks_that_fit_on_an_sm_together_never_ask_for_more_tensor_memory_than
         return max((c + most_columns(room - s - reserved) for s, c in shapes if s + reserved <= room), default=0)
 
     assert most_columns(per_sm) <= 512
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_no_lane_leaves_a_loop_of_warp_wide_loads_on_its_own(name):
+    body = KERNELS[name]
+    for load in re.finditer(r"tmem_load\d+\(", body):
+        depth, at = 0, load.end()
+        while depth >= 0:  # to the end of the block that holds the load
+            depth += {"{": 1, "}": -1}.get(body[at], 0)
+            at += 1
+        assert "continue;" not in body[load.end():at], body[load.start():at]

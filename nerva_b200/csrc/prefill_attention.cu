@@ -53,6 +53,18 @@ struct AttentionShared {
   float m[2][kRows], l[2][kRows];  // the groups' softmax states
   uint32_t tmem_base;
   uint32_t abort;
+  uint32_t taken_out;  // values that are not finite were taken out of a tile
+};
+
+// What the rows of a block see: 0 <= pos - key, and pos - key < window or key < keep_first.
+struct Sight {
+  uint32_t pos_first, pos_last, window, keep_first;
+  __device__ __forceinline__ bool sees(uint32_t pos, uint32_t key) const {
+    return key <= pos && (pos - key < window || key < keep_first);
+  }
+  __device__ __forceinline__ bool edge(uint32_t first) const {  // some row does not see some key of the tile
+    return first + kKeys > pos_first + 1u || first < keep_first || pos_last - first >= window;
+  }
 };
 
 // 16-byte piece `piece` of row `row` of a tile whose 64-element column blocks follow each other.
@@ -103,6 +115,94 @@ __device__ __forceinline__ float exp2_ftz(float x) {
   return y;
 }
 
+// A block's rows: (position, head) pairs f0 .. f_end - 1 of its KV head, and the tiles of keys that they walk.
+template <bool EXTRAS>
+struct Extent {
+  uint32_t group, f0, f_end, base, kv_end, page_count;
+  const uint32_t *page_table;
+  uint32_t *error_word;
+  Sight sight;
+  TileWalk walk;
+  bool inside;
+  uint32_t tiles;
+  __device__ __forceinline__ explicit Extent(const WindowAttentionParams &p) : walk(0u, 0u, kKeys) {
+    const FusedAttentionRow &r0 = p.rows[0];
+    group = p.s.heads / p.s.kv_heads;
+    const uint32_t total_rows = p.row_count * group;
+    f0 = (gridDim.y - 1u - blockIdx.y) * kRows;  // the longest walks first
+    f_end = f0 + kRows < total_rows ? f0 + kRows : total_rows;
+    base = r0.position;
+    page_count = r0.page_count;
+    page_table = r0.page_table;
+    error_word = r0.error_word;
+    sight.pos_first = base + f0 / group;
+    sight.pos_last = base + (f_end - 1u) / group;
+    sight.window = p.s.window != 0 ? p.s.window : 0xffffffffu;
+    sight.keep_first = EXTRAS ? p.s.keep_first : 0u;
+    inside = sight.pos_last < r0.max_context;
+    const uint32_t window_lo = sight.pos_first + 1u > sight.window ? sight.pos_first + 1u - sight.window : 0u;  // of the first row
+    kv_end = sight.pos_last + 1u;
+    walk = TileWalk(sight.keep_first, window_lo, kKeys);
+    tiles = inside ? walk.count(kv_end, kKeys) : 0u;
+  }
+};
+
+// A probability of zero times a value that is not finite is not zero, and a tile at an edge holds values that some rows do
+// not see.  Such values are set to zero in the tile, and the rows that do see them get them at the end (put_back).  The last
+// page's rows behind the last query hold whatever the pool had: all zero.  By the MMA warp, which waits for the softmax of
+// the tile anyway: as a part of the softmax, 16 rows' pieces a thread, the same looks cost 3 % of a 512-token prompt.
+template <uint32_t D>
+__device__ __forceinline__ void clean_values(uint8_t *tile, uint32_t used, uint32_t *taken_out) {
+  constexpr uint32_t kPieces = D / 8u;
+  const uint32_t lane = threadIdx.x & 31u;
+  // all ones in the exponent carry into the sign's place, in both halves of a word
+  auto marks = [](uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; };
+  uint32_t any = 0;
+#pragma unroll 8
+  for (uint32_t i = lane; i < used * kPieces; i += 32u) {
+    const uint4 w = lds128(tile + swizzled(i / kPieces, i % kPieces));
+    any |= (marks(w.x) | marks(w.y)) | (marks(w.z) | marks(w.w));
+  }
+  const bool found = __any_sync(0xffffffffu, (any & 0x80008000u) != 0u);
+  if (found) {
+#pragma unroll 1
+    for (uint32_t i = lane; i < used * kPieces; i += 32u) {
+      uint4 *at = reinterpret_cast<uint4 *>(tile + swizzled(i / kPieces, i % kPieces));
+      auto clean = [&](uint32_t v) { return v & ~(((marks(v) & 0x80008000u) >> 15) * 0xffffu); };
+      const uint4 w = *at;
+      *at = make_uint4(clean(w.x), clean(w.y), clean(w.z), clean(w.w));
+    }
+    if (lane == 0) *taken_out = 1;
+  }
+  const uint32_t page_end = (used + kPageTokens - 1u) / kPageTokens * kPageTokens;
+  for (uint32_t i = used * kPieces + lane; i < page_end * kPieces; i += 32u)
+    *reinterpret_cast<uint4 *>(tile + swizzled(i / kPieces, i % kPieces)) = make_uint4(0u, 0u, 0u, 0u);
+  if (found || used < page_end) {
+    fence_proxy_async();
+    __syncwarp();
+  }
+}
+// What clean_values took out of `columns` values of a row's KV head (`values`: those of the first cached row) and the row
+// at `pos` sees: added to its output.
+__device__ __noinline__ void put_back(uint16_t *out, const uint16_t *values, uint32_t columns, uint64_t row_stride,
+                                      const uint32_t *page_table, uint32_t page_count, TileWalk walk, uint32_t tiles,
+                                      Sight sight, uint32_t pos) {
+  for (uint32_t c = 0; c < columns; ++c) {
+    float sum = 0.0f;
+    for (uint32_t j = 0; j < tiles; ++j) {
+      const uint32_t first = walk.tile(j) * kKeys;
+      if (!sight.edge(first)) continue;
+      for (uint32_t key = first; key < first + kKeys && key <= pos; ++key) {
+        const uint32_t page = page_table[key / kPageTokens];
+        if (!sight.sees(pos, key) || page >= page_count) continue;
+        const float v = bf16_bits_to_f32(values[(static_cast<uint64_t>(page) * kPageTokens + key % kPageTokens) * row_stride + c]);
+        if (!isfinite(v)) sum += v;
+      }
+    }
+    if (sum != 0.0f) out[c] = static_cast<uint16_t>(pack_bf16_hi(bf16_bits_to_f32(out[c]) + sum, 0.0f));
+  }
+}
+
 template <uint32_t D, bool EXTRAS>
 __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                const __grid_constant__ CUtensorMap map_v,
@@ -134,6 +234,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
     mbar_init(&sh.o_done, 1);
     mbar_init(&sh.drained, 1);
     sh.abort = 0;
+    sh.taken_out = 0;
     mbar_init_fence();
   }
   if (warp == kMmaWarp) {
@@ -143,22 +244,17 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();
-  const FusedAttentionRow &r0 = p.rows[0];
-  const uint32_t group = s.heads / s.kv_heads, kvh = blockIdx.x;
-  const uint32_t total_rows = p.row_count * group;
-  const uint32_t f0 = (gridDim.y - 1u - blockIdx.y) * kRows;  // the longest walks first
-  const uint32_t f_end = f0 + kRows < total_rows ? f0 + kRows : total_rows;
-  const uint32_t base = r0.position, page_count = r0.page_count;
-  const uint32_t *page_table = r0.page_table;
-  uint32_t *error_word = r0.error_word;
-  const uint32_t pos_first = base + f0 / group, pos_last = base + (f_end - 1u) / group;
-  const bool inside = pos_last < r0.max_context;
-  const uint32_t window = s.window != 0 ? s.window : 0xffffffffu;
-  const uint32_t keep_first = EXTRAS ? s.keep_first : 0u;
-  const uint32_t window_lo = pos_first + 1u > window ? pos_first + 1u - window : 0u;  // of the first row
-  const uint32_t kv_end = pos_last + 1u;
-  const TileWalk walk(keep_first, window_lo, kKeys);
-  const uint32_t tiles = inside ? walk.count(kv_end, kKeys) : 0u;
+  const uint32_t kvh = blockIdx.x;
+  const Extent<EXTRAS> e(p);
+  const uint32_t group = e.group, f0 = e.f0, f_end = e.f_end, base = e.base, kv_end = e.kv_end;
+  const uint32_t page_count = e.page_count;
+  const uint32_t *page_table = e.page_table;
+  uint32_t *error_word = e.error_word;
+  const Sight sight = e.sight;
+  const uint32_t pos_first = sight.pos_first, pos_last = sight.pos_last, window = sight.window, keep_first = sight.keep_first;
+  const TileWalk walk = e.walk;
+  const bool inside = e.inside;
+  const uint32_t tiles = e.tiles;
 
   // queries, scaled so that the softmax runs on exp2, as a bf16 rounding and its remainder
   if (inside) {
@@ -224,16 +320,9 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
       for (uint32_t j = 0; ok && j < tiles; ++j) {
         const uint32_t st = j % kStages;
         if (!warp_wait(&sh.v_full[st], (j / kStages) & 1u, abort, error_word)) break;
-        if (j + 1u == tiles && kv_end % kPageTokens != 0) {
-          // the last page's rows behind the last query hold whatever the pool had: a zero probability times a NaN
-          // would still be one
-          const uint32_t from = kv_end - walk.tile(j) * kKeys;
-          const uint32_t rows = kPageTokens - kv_end % kPageTokens;
-          for (uint32_t i = lane; i < rows * (D / 8u); i += 32u)
-            *reinterpret_cast<uint4 *>(v_ring + st * kTileBytes + swizzled(from + i / (D / 8u), i % (D / 8u))) = make_uint4(0, 0, 0, 0);
-          fence_proxy_async();
-          __syncwarp();
-        }
+        const uint32_t first = walk.tile(j) * kKeys;
+        if (sight.edge(first))
+          clean_values<D>(v_ring + st * kTileBytes, kv_end - first < kKeys ? kv_end - first : kKeys, &sh.taken_out);
         if (!warp_wait(&sh.p_full[j & 1u], (j >> 1) & 1u, abort, error_word)) break;
         tcgen05_fence_after();
         if (lane == 0) {
@@ -397,6 +486,13 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
           if (c + i < s.v_dim) dst[c + i] = f32_to_bf16_bits(o[i]);
       }
       __syncwarp();
+    }
+    if (sh.taken_out != 0u && live && half * (D / 2u) < s.v_dim) {
+      const Extent<EXTRAS> again(p);  // nothing of it stays in registers through the loops above
+      const uint32_t c = half * (D / 2u), columns = s.v_dim - c < D / 2u ? s.v_dim - c : D / 2u;
+      put_back(dst + c, static_cast<const uint16_t *>(p.values) + p.value_offset + kvh * D + c, columns,
+               static_cast<uint64_t>(s.kv_heads) * D, again.page_table, again.page_count, again.walk, again.tiles, again.sight,
+               again.base + f / group);
     }
   }
   // ---- teardown: nothing stays in flight ----

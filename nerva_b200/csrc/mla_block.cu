@@ -17,6 +17,8 @@
 // for 6 layers), 4 tokens 1.70 ms (steps 2.09), 64 tokens 2.6 ms (32.1).
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma_bf16.cuh"
@@ -306,7 +308,10 @@ __global__ void __launch_bounds__(512, 1) mla_block_attention_kernel(MlaBlockPar
         acc[mt][i][3] *= corr_b;
       }
     }
-#pragma unroll
+    // A zero probability times a value that is not finite is not zero: where a position of the block does not see every row
+    // of the tile, the rows it does not see are masked out of its product.
+    auto value_product = [&](auto masked) {
+#pragma unroll(masked ? 1 : kKeys / 16u)
     for (uint32_t ks = 0; ks < kKeys / 16u; ++ks) {
       const uint32_t row = ks * 16u + ((lane >> 3) & 1u) * 8u + (lane & 7u);
       uint32_t b[NT][2];
@@ -328,13 +333,24 @@ __global__ void __launch_bounds__(512, 1) mla_block_attention_kernel(MlaBlockPar
         const uint32_t at = (mt * 16u + (lane & 15u)) * kPStride + ks * 16u + (lane >> 4) * 8u;
         ldmatrix_x4(hi, smem_addr(p_hi + at));
         ldmatrix_x4(lo, smem_addr(p_lo + at));
+        uint32_t seen0 = 0xffffffffu, seen1 = 0xffffffffu;  // of rows 2 t, 2 t + 1 and of rows 2 t + 8, 2 t + 9
+        if constexpr (masked) {
+          const uint32_t key = token0 + ks * 16u + 2u * t, pos = pos0 + mt;
+          seen0 = (key <= pos ? 0xffffu : 0u) | (key + 1u <= pos ? 0xffff0000u : 0u);
+          seen1 = (key + 8u <= pos ? 0xffffu : 0u) | (key + 9u <= pos ? 0xffff0000u : 0u);
+        }
 #pragma unroll
         for (uint32_t i = 0; i < NT; ++i) {
-          mma_bf16(acc[mt][i], hi, b[i][0], b[i][1]);
-          mma_bf16(acc[mt][i], lo, b[i][0], b[i][1]);
+          mma_bf16(acc[mt][i], hi, b[i][0] & seen0, b[i][1] & seen1);
+          mma_bf16(acc[mt][i], lo, b[i][0] & seen0, b[i][1] & seen1);
         }
       }
     }
+    };
+    if (token0 + kKeys > pos0 + 1u)
+      value_product(std::true_type{});
+    else
+      value_product(std::false_type{});
   }
   if (lane == 0) {
 #pragma unroll

@@ -12,7 +12,7 @@ import pytest
 from nerva_b200 import ops, synth
 from nerva_b200.session import CudaHfDecodeSequenceSession, SmokeStatus
 from tests import vamidra_models as M
-from tests.test_gpu_sparse_prefill import MOE
+from tests.test_gpu_sparse_prefill import LATENT, LATENT_256, MOE
 
 pytestmark = pytest.mark.gpu
 
@@ -30,7 +30,8 @@ def _dense(name, **fields):
 
 DECODERS = {
     "128 wide": _dense("a"), "64 wide": _dense("b", head_dim=64), "a head per KV head": _dense("c", heads=4, kv_heads=4),
-    "experts": MOE,
+    "experts": MOE, "latent 128": LATENT, "latent 256": LATENT_256,
+    "latent 512": dataclasses.replace(LATENT, layers=2, heads=16, kv_heads=16, kv_lora_rank=512, qk_nope_head_dim=128, qk_rope_head_dim=64),
 }
 
 
@@ -41,9 +42,15 @@ def _overflowing(cfg):
     embed[BAD] = 0
     embed[BAD, 0] = ONE
     layer = ck.layers[0]
-    value = layer["w_v"].reshape(cfg.kv_heads, cfg.head_dim, cfg.hidden)
-    value[:, 3] = 0
-    value[:, 3, 0] = HUGE_BITS
+    if cfg.kv_lora_rank:
+        latent = layer["w_kv_a"].reshape(-1, cfg.hidden)
+        latent[3] = 0
+        latent[3, 0] = ONE
+        layer["kv_a_norm"][3] = HUGE_BITS
+    else:
+        value = layer["w_v"].reshape(cfg.kv_heads, cfg.head_dim, cfg.hidden)
+        value[:, 3] = 0
+        value[:, 3, 0] = HUGE_BITS
     return ck
 
 

@@ -648,14 +648,21 @@ cudaError_t allocate_block_workspace(NervaCudaHfDecodeSequenceSession *s) {
     const uint64_t fit = (64ull << 20) / (moe_widths(s).top_k * s->dims.hidden) / 64u * 64u;
     most = static_cast<uint32_t>(std::min<uint64_t>(most, std::max<uint64_t>(fit, 64u)));
   }
-  ws.max_rows = std::max(kBlockSampleRows, std::min(most, context_rows));
-  ws.part_rows = std::min(ws.max_rows, kBlockPartRows);
   ws.sample_rows = kBlockSampleRows;
-  StaticArena sizing(UINT64_MAX / 2);
-  if (!plan_workspace(s, &ws, sizing, nullptr)) return cudaErrorMemoryAllocation;
-  ws.bytes = sizing.used();
   ws.packed_steps = !s->has_moe && !s->dims.mla();
-  cudaError_t err = cudaMalloc(&ws.block, ws.bytes);
+  cudaError_t err = cudaSuccess;
+  for (;;) {
+    ws.max_rows = std::max(kBlockSampleRows, std::min(most, context_rows));
+    ws.part_rows = std::min(ws.max_rows, kBlockPartRows);
+    StaticArena sizing(UINT64_MAX / 2);
+    if (!plan_workspace(s, &ws, sizing, nullptr)) return cudaErrorMemoryAllocation;
+    ws.bytes = sizing.used();
+    err = cudaMalloc(&ws.block, ws.bytes);
+    if (err == cudaSuccess || ws.max_rows <= kBlockPartRows) break;
+    // a device with little room left: shorter chunks, which stream the weights more often, down to one MMA N
+    cudaGetLastError();
+    most = std::max(std::min(most, context_rows) / 2u, kBlockPartRows);
+  }
   if (err != cudaSuccess && !ws.packed_steps) {
     // sparse models and latent attention do without blocks, token by token
     cudaGetLastError();

@@ -47,6 +47,15 @@ struct WideTiles {
   uint32_t row_tiles, token_tiles, tile_tokens;  // of kPairRows weight rows, of tile_tokens tokens
 };
 
+// Timeline stamp of the first or the last pair, by a thread of the block that issues its MMAs.
+__device__ __forceinline__ void stamp_pair(unsigned long long *stamps, uint32_t slot, uint32_t pair, uint32_t pairs) {
+  if (stamps == nullptr || (pair != 0 && pair + 1u != pairs)) return;
+  unsigned long long now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+  if (pair == 0) stamps[slot] = now;
+  if (pair + 1u == pairs) stamps[4u + slot] = now;
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -105,6 +114,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
   pdl_trigger();
   if (threadIdx.x == 0) {
+    if (rank == 0) stamp_pair(p.stamps, kStampEntry, pair, pairs);
     for (uint32_t s = 0; s < p.stages; ++s) {
       mbar_init(&sh.full[s], 1);
       mbar_init(&sh.empty[s], 1);
@@ -159,6 +169,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     // ---------------- MMA issuer: the pair's first block ----------------
     if (rank == 0 && lane == 0) {
       const uint32_t idesc = pair_instr_desc(t.tile_tokens);
+      // (in front of the loop: a test inside it took 3 % of a 512-token prefill)
+      if (p.stamps != nullptr && abortable_wait(&sh.full[0], 0, abort, p.error_word)) stamp_pair(p.stamps, kStampAfterWait, pair, pairs);
       uint32_t consumed = 0, index = 0;
       bool ok = true;
       for (uint32_t tile = pair; ok && tile < tiles; tile += pairs, ++index) {
@@ -182,6 +194,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
         if (ok) pair_commit(&sh.acc_full[acc]);
       }
+      stamp_pair(p.stamps, kStampAfterPrologue, pair, pairs);
     }
   } else {
     // ---------------- epilogue (warps 2..5) ----------------
@@ -221,6 +234,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == 1) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemColumns) : "memory");
+    if (rank == 0 && lane == 0) stamp_pair(p.stamps, kStampExit, pair, pairs);
   }
 }
 

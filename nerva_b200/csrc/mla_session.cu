@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(512) mla_attention_kernel(MlaParams p) {
 }
 
 __global__ void __launch_bounds__(256) mla_output_kernel(MlaParams p, uint32_t slots) {
-  __shared__ float lat[kMlaMaxRank];
+  __shared__ __align__(16) float lat[kMlaMaxRank];  // written in pairs
   __shared__ float weight[kMlaMaxSplits];
   pdl_trigger();
   const uint32_t h = blockIdx.x;

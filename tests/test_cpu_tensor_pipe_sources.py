@@ -80,3 +80,14 @@ def test_no_lane_leaves_a_loop_of_warp_wide_loads_on_its_own(name):
             depth += {"{": 1, "}": -1}.get(body[at], 0)
             at += 1
         assert "continue;" not in body[load.end():at], body[load.start():at]
+
+
+def test_shared_arrays_that_are_accessed_in_wider_pieces_are_aligned():
+    """reinterpret_cast<float2 / float4 / uint2 / uint4 *> of a __shared__ array needs an alignment of its own."""
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = open(path).read()
+        for kernel in re.split(r"(?=__global__)", text):
+            arrays = {name: "__align__" in line
+                      for line in re.findall(r"__shared__[^;]*;", kernel) for name in re.findall(r"(\w+)\[", line)}
+            for name in re.findall(r"reinterpret_cast<(?:const )?(?:float|uint)[24] \*>\((\w+)", kernel):
+                assert arrays.get(name, True), (os.path.basename(path), name)

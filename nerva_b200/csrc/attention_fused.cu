@@ -56,7 +56,7 @@ struct FusedLayout {
 
 // ROWS: block-step form (one set of blocks per activation row, fields taken from p.rows[blockIdx.y]).
 template <uint32_t PER, bool ROWS>
-__global__ void fused_decode_attention_kernel(FusedAttentionParams p) {
+__device__ __forceinline__ void fused_decode_attention(FusedAttentionParams &p) {
   constexpr uint32_t D = PER * 32u;
   using Layout = FusedLayout<D>;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -422,6 +422,17 @@ __global__ void fused_decode_attention_kernel(FusedAttentionParams p) {
   stamp(p.stamps, kStampExit);
 }
 
+template <uint32_t PER, bool ROWS>
+__global__ void fused_decode_attention_kernel(FusedAttentionParams p) {
+  fused_decode_attention<PER, ROWS>(p);
+}
+// Eight query heads of 128 per KV head make 17 warps, which get registers in fours: 20 x 32 x 104 are more than an SM has.
+constexpr uint32_t kWideThreads = (2u * kFusedMaxGroup + 1u) * 32u;
+template <uint32_t PER, bool ROWS>
+__global__ void __launch_bounds__(kWideThreads) fused_decode_attention_wide_kernel(FusedAttentionParams p) {
+  fused_decode_attention<PER, ROWS>(p);
+}
+
 }  // namespace
 
 bool fused_attention_supported(uint32_t heads, uint32_t kv_heads, uint32_t head_dim) {
@@ -447,6 +458,8 @@ cudaError_t configure_fused_attention_kernel() {
   };
   set(fused_decode_attention_kernel<4, false>, FusedLayout<128>::bytes(kFusedMaxGroup));
   set(fused_decode_attention_kernel<4, true>, FusedLayout<128>::bytes(kFusedMaxGroup));
+  set(fused_decode_attention_wide_kernel<4, false>, FusedLayout<128>::bytes(kFusedMaxGroup));
+  set(fused_decode_attention_wide_kernel<4, true>, FusedLayout<128>::bytes(kFusedMaxGroup));
   set(fused_decode_attention_kernel<2, false>, FusedLayout<64>::bytes(kFusedMaxGroup));
   set(fused_decode_attention_kernel<2, true>, FusedLayout<64>::bytes(kFusedMaxGroup));
   return err;
@@ -463,14 +476,14 @@ cudaError_t launch_fused_attention(cudaStream_t stream, const FusedAttentionPara
     if (p.row_count == 0 || p.row_count > 65535u) return cudaErrorInvalidValue;
     const dim3 grid(blocks, p.row_count);
     if (p.head_dim == 128)
-      return launch_with_pdl(fused_decode_attention_kernel<4, true>, grid, dim3(threads),
-                             FusedLayout<128>::bytes(group), stream, p.pdl != 0, p);
+      return launch_with_pdl(group < kFusedMaxGroup ? fused_decode_attention_kernel<4, true> : fused_decode_attention_wide_kernel<4, true>,
+                             grid, dim3(threads), FusedLayout<128>::bytes(group), stream, p.pdl != 0, p);
     return launch_with_pdl(fused_decode_attention_kernel<2, true>, grid, dim3(threads), FusedLayout<64>::bytes(group),
                            stream, p.pdl != 0, p);
   }
   if (p.head_dim == 128) {
-    return launch_with_pdl(fused_decode_attention_kernel<4, false>, dim3(blocks), dim3(threads),
-                           FusedLayout<128>::bytes(group), stream, p.pdl != 0, p);
+    return launch_with_pdl(group < kFusedMaxGroup ? fused_decode_attention_kernel<4, false> : fused_decode_attention_wide_kernel<4, false>,
+                           dim3(blocks), dim3(threads), FusedLayout<128>::bytes(group), stream, p.pdl != 0, p);
   }
   return launch_with_pdl(fused_decode_attention_kernel<2, false>, dim3(blocks), dim3(threads),
                          FusedLayout<64>::bytes(group), stream, p.pdl != 0, p);

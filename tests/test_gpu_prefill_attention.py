@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 LOGIT_ATOL = 2e-2  # the stated bound of logits at this width and depth: both paths round the same values to bf16
 
-SHAPES = [(8, 2, 128), (6, 2, 64), (16, 1, 128), (4, 4, 64)]  # heads, KV heads, head size: 4, 3, 16 and 1 heads per KV head
+# heads, KV heads, head size: 4, 3, 8 and 1 heads per KV head (more than 8 keep a decoder off blocks)
+SHAPES = [(8, 2, 128), (6, 2, 64), (16, 2, 128), (4, 4, 64)]
 
 
 def _checkpoint(heads, kv_heads, dim):
@@ -39,6 +40,7 @@ def test_tile_prefill_matches_prefill_by_decode(built_lib, heads, kv_heads, dim)
         prompt = synth.uniform_u32(5, synth.T_PROMPT, tokens, cfg.vocab)
         want = _by_decode(ck, prompt, 512)
         s = CudaHfDecodeSequenceSession(ck, 512)
+        assert s.create_result.prefill_chunk_tokens > 1  # the prompt goes in blocks
         s.set_kv_block_table(synth.permutation(3, synth.T_PAGE_TABLE, 32))
         got = s.append(prompt, want=[tokens - 1], reset=True)[0]
         assert np.abs(got - want).max() <= LOGIT_ATOL, tokens
@@ -48,3 +50,18 @@ def test_tile_prefill_matches_prefill_by_decode(built_lib, heads, kv_heads, dim)
             again = s.append(prompt[101:], want=[tokens - 102])[0]
             assert np.abs(again - want).max() <= LOGIT_ATOL
         s.destroy()
+
+
+@pytest.mark.parametrize("heads,dim,mixer", [(16, 64, {}), (12, 128, {}), (24, 64, {"window": 90, "keep": 5, "cap": 6.0})])
+def test_many_query_heads_of_one_key_head(built_lib, heads, dim, mixer):
+    """More than 8 heads per KV head reach the tiles through the models described layer by layer."""
+    from tests import vamidra_models as M
+    from tests import vamidra_oracle as O
+    shape = {"window": 1000, "keep": 0, "cap": 0.0, **mixer}
+    cfg = M.config([M.attention(ff=0, heads=heads, kv_heads=1, dim=dim, vdim=dim, **shape)], width=128)
+    w = M.weights(cfg)
+    tokens = M.tokens(cfg, 200)
+    s = CudaHfDecodeSequenceSession(M.checkpoint(cfg, w), 208, compute="bfloat16")
+    got = s.append(tokens, range(200), reset=True)
+    assert M.worst_position(got, O.forward(cfg, w, tokens)) < 2 * M.TOLERANCE["bfloat16"]
+    s.destroy()

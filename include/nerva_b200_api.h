@@ -1055,6 +1055,16 @@ int nerva_b200_gqa_decode_attention_static_scratch(
     const uint32_t *page_table, float *out, uint32_t batch, uint32_t context, uint32_t heads,
     uint32_t kv_heads, uint32_t head_dim, void *stream);
 
+/* Output of one decode step's sparse MLP (without the residual) from the residual stream h[hidden], as rank `rank` of
+ * `world` computes it: all experts are routed over, those from expert_base on (expert_local of them) are held, and the
+ * partial sum goes to every rank's receive buffer, whose entries are checked.  gate_up [expert_local][2 * intermediate]
+ * [hidden], down [expert_local][hidden][intermediate]; shared: gate, up [shared_intermediate][hidden], down [hidden]
+ * [shared_intermediate] behind each other (the rank's slice), or NULL.  No peer is waited for.  Host pointers. */
+int nerva_b200_sparse_mlp_rank(const float *h, const uint16_t *norm, const uint16_t *router, const uint16_t *gate_up,
+                               const uint16_t *down, const uint16_t *shared, uint32_t hidden, uint32_t intermediate,
+                               uint32_t shared_intermediate, uint32_t num_experts, uint32_t top_k, uint32_t norm_topk,
+                               uint32_t expert_base, uint32_t expert_local, uint32_t rank, uint32_t world, float *out);
+
 /* Greedy argmax over f32 logits with the sampler's tie rule (lowest index,
  * non-finite values skipped).  Host pointers. */
 int nerva_b200_greedy_argmax(const float *logits, uint32_t count, uint32_t *token);

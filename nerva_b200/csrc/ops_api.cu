@@ -305,6 +305,109 @@ extern "C" int nerva_b200_projection_sustained(const uint16_t *weight, const uin
   return 0;
 }
 
+extern "C" int nerva_b200_sparse_mlp_rank(const float *h, const uint16_t *norm, const uint16_t *router, const uint16_t *gate_up,
+                                          const uint16_t *down, const uint16_t *shared, uint32_t hidden, uint32_t intermediate,
+                                          uint32_t shared_intermediate, uint32_t num_experts, uint32_t top_k, uint32_t norm_topk,
+                                          uint32_t expert_base, uint32_t expert_local, uint32_t rank, uint32_t world,
+                                          float *out) {
+  set_last_error("");
+  const uint64_t H = hidden, M = intermediate, S = shared != nullptr ? shared_intermediate : 0u;
+  if (h == nullptr || norm == nullptr || router == nullptr || gate_up == nullptr || down == nullptr || out == nullptr ||
+      expert_local == 0 || expert_base + expert_local > num_experts || world == 0 || world > kMaxTpWorld || rank >= world)
+    return -1;
+  uint32_t sms = 0;
+  cudaError_t err = device_sm_count(&sms, nullptr, nullptr, nullptr);
+  if (err == cudaSuccess) err = configure_moe_kernels();
+  DeviceBuffers buf;
+  auto upload = [&](auto **dst, const auto *src, uint64_t count) {
+    if (err == cudaSuccess) err = buf.alloc(dst, count);
+    if (err == cudaSuccess && src != nullptr) err = cudaMemcpy(*dst, src, count * sizeof(**dst), cudaMemcpyHostToDevice);
+  };
+  float *d_h = nullptr, *scratch = nullptr;
+  uint16_t *d_norm = nullptr, *d_router = nullptr, *d_gate_up = nullptr, *d_down = nullptr, *d_shared = nullptr;
+  uint32_t *words = nullptr;
+  unsigned long long *entries = nullptr;  // [world][world][hidden]: every rank's receive buffer, and the step counter
+  upload(&d_h, h, H);
+  upload(&d_norm, norm, H);
+  upload(&d_router, router, num_experts * H);
+  upload(&d_gate_up, gate_up, expert_local * 2u * M * H);
+  upload(&d_down, down, expert_local * H * M);
+  if (S != 0) upload(&d_shared, shared, 3u * S * H);
+  if (err == cudaSuccess) err = buf.alloc(&words, 32u);
+  const uint64_t route = 256u + 16u + 4u, activations = (top_k * M + S + 3u) & ~uint64_t{3};
+  if (err == cudaSuccess) err = buf.alloc(&scratch, route + activations + 3u * H);
+  const uint64_t entry_count = static_cast<uint64_t>(world) * world * H + 1u;
+  if (err == cudaSuccess) err = buf.alloc(&entries, entry_count);
+  if (err == cudaSuccess) err = cudaMemset(words, 0, 32u * sizeof(uint32_t));
+  if (err == cudaSuccess) err = cudaMemset(entries, 0, entry_count * sizeof(unsigned long long));
+  MoeExpertParams p{};
+  p.add_a = d_h;
+  p.norm_weight = d_norm;
+  p.eps = 1e-6f;
+  p.hidden = hidden;
+  p.moe_intermediate = intermediate;
+  p.shared_intermediate = static_cast<uint32_t>(S);
+  p.top_k = top_k;
+  p.w_expert_gate_up = d_gate_up;
+  p.expert_stride = 2u * M * H;
+  p.expert_up_offset = M * H;
+  p.w_expert_down = d_down;
+  if (S != 0) {
+    p.w_shared_gate = d_shared;
+    p.w_shared_up = d_shared + S * H;
+    p.w_shared_down = d_shared + 2u * S * H;
+  }
+  p.w_router = d_router;
+  p.num_experts = num_experts;
+  p.norm_topk_prob = norm_topk;
+  p.expert_ids = words;
+  p.error_word = words + 16;
+  p.router_logits = scratch;
+  p.route_weights = scratch + 256;
+  p.shared_gate = scratch + 272;
+  p.gate_up_out = scratch + route;
+  p.x_norm = scratch + route + activations;
+  p.out_f32 = p.x_norm + H;
+  p.resid_out = p.out_f32 + H;
+  p.expert_base = expert_base;
+  p.expert_local = expert_local;
+  if (world > 1) {
+    p.push.world = world;
+    p.push.rank = rank;
+    for (uint32_t q = 0; q < world; ++q) p.push.recv[q] = entries + q * world * H;
+    p.push.epoch = entries + entry_count - 1u;
+    p.push.per_epoch = 1;
+    p.push.offset = 1;
+  }
+  if (err == cudaSuccess) err = launch_moe_experts(nullptr, p, sms, true);
+  std::vector<unsigned long long> got(entry_count);
+  uint32_t device_error = 0;
+  if (err == cudaSuccess) err = cudaMemcpy(out, p.out_f32, H * sizeof(float), cudaMemcpyDeviceToHost);
+  if (err == cudaSuccess) err = cudaMemcpy(got.data(), entries, entry_count * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+  if (err == cudaSuccess) err = cudaMemcpy(&device_error, p.error_word, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+  if (err != cudaSuccess || device_error != 0) {
+    set_last_error(err != cudaSuccess ? cudaGetErrorString(err) : "sparse MLP kernel gave up a bounded wait");
+    return -1;
+  }
+  for (uint32_t q = 0; world > 1 && q < world; ++q) {
+    for (uint64_t i = 0; i < world * H; ++i) {
+      const unsigned long long entry = got[q * world * H + i];
+      const bool mine = i / H == rank;
+      if (entry >> 32 != (mine ? 1u : 0u) || (mine && entry != got[rank * H + i % H])) {
+        set_last_error("an entry of a receive buffer is missing, or in another rank's place");
+        return -1;
+      }
+    }
+  }
+  if (world > 1) {
+    for (uint64_t i = 0; i < H; ++i) {
+      const uint32_t bits = static_cast<uint32_t>(got[rank * H + i]);
+      memcpy(out + i, &bits, sizeof(bits));
+    }
+  }
+  return 0;
+}
+
 extern "C" int nerva_b200_tensor_memory_launches(uint32_t *smem_bytes, uint32_t *columns, uint32_t capacity) {
   std::vector<TensorMemoryLaunch> all;
   gemm_tc_launches(&all);

@@ -151,6 +151,7 @@ def _bind(L: C.CDLL, reference_abi_only: bool) -> C.CDLL:
                                                       P(C.c_uint64)],
         "nerva_b200_gqa_decode_attention_static_scratch": [vp, vp, vp, vp, vp, C.c_uint32, C.c_uint32,
                                                            C.c_uint32, C.c_uint32, C.c_uint32, vp],
+        "nerva_b200_sparse_mlp_rank": [vp] * 6 + [C.c_uint32] * 10 + [vp],
         "nerva_b200_greedy_argmax": [vp, C.c_uint32, P(C.c_uint32)],
         "nerva_b200_sample_token": [vp, C.c_uint32, C.c_uint32, C.c_float, C.c_float, C.c_uint32, C.c_uint64,
                                     P(C.c_uint32)],

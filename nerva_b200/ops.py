@@ -154,6 +154,27 @@ def deepseek_mla_decode(q_nope, q_pe, kv_c, k_pe, w_uk, w_uv, heads: int, tokens
     return rc, out_values, out
 
 
+def sparse_mlp_rank(h, norm, router, gate_up, down, shared=None, top_k: int = 1, norm_topk: bool = True, expert_base: int = 0,
+                    rank: int = 0, world: int = 1) -> np.ndarray:
+    """One rank's part of a decode step's sparse MLP (nerva_b200_sparse_mlp_rank): h [hidden] fp32, router [experts, hidden],
+    gate_up [held, 2, intermediate, hidden], down [held, hidden, intermediate] and shared = (gate, up, down) as bf16 bits."""
+    h = np.ascontiguousarray(h, dtype=np.float32)
+    norm, router, gate_up, down = (np.ascontiguousarray(a, dtype=np.uint16) for a in (norm, router, gate_up, down))
+    held, _, intermediate, hidden = gate_up.shape
+    assert h.shape == (hidden,) and router.shape[1] == hidden and down.shape == (held, hidden, intermediate)
+    packed, width = None, 0
+    if shared is not None:
+        width = shared[0].shape[0]
+        assert shared[1].shape == (width, hidden) and shared[2].shape == (hidden, width)
+        packed = np.concatenate([np.ascontiguousarray(a, dtype=np.uint16).reshape(-1) for a in shared])
+    out = np.empty(hidden, dtype=np.float32)
+    _check(ffi.lib().nerva_b200_sparse_mlp_rank(
+        h.ctypes.data, norm.ctypes.data, router.ctypes.data, gate_up.ctypes.data, down.ctypes.data,
+        packed.ctypes.data if packed is not None else None, hidden, intermediate, width, router.shape[0], top_k, int(norm_topk),
+        expert_base, held, rank, world, out.ctypes.data), "sparse_mlp_rank")
+    return out
+
+
 def deepseek_moe_forward(x, expert_ids, expert_weights, w_gate, w_up, w_down, hidden: int, intermediate: int,
                          num_experts: int, clamp_swiglu: bool = False, swiglu_limit: float = 0.0):
     """fp32 expert MLP of one token over already routed experts.  Returns (return code, out, result)."""

@@ -40,7 +40,8 @@ def _row_distance_in_steps(a: np.ndarray, b: np.ndarray) -> float:
 
 @pytest.mark.parametrize("prompt_tokens", [2, 17, 64, 255, 256, 257, 300])
 def test_chunked_prefill_matches_prefill_by_decode(built_lib, oracle_mod, tiny_checkpoint, prompt_tokens):
-    """Prompt lengths around the 16-token page and the 256-token chunk: same first token and same
+    """Prompt lengths around the 16-token page, the 64 rows from which attention runs on tiles and the 256 tokens from
+    which the projections run on pairs of SMs, all in one block (several: test_gpu_long_prompts.py): same first token and same
     continuation as the token-by-token prefill, first-token logits within the stated bound of the
     oracle, cached K/V rows within one bf16 rounding step (at the row's magnitude) of the rows the
     decode step writes: the two prefills differ in the fp32 summation order of the QKV projection."""
@@ -86,7 +87,7 @@ def test_chunked_prefill_on_the_golden_prompt(built_lib, tiny_checkpoint, tiny_g
 
 
 def test_chunked_prefill_on_qwen3_8b_layer_shapes(built_lib, oracle_mod):
-    """Two full-width layers, a 300-token prompt (two chunks): first-token logits against the oracle."""
+    """Two full-width layers, a 300-token prompt (one block): first-token logits against the oracle."""
     import dataclasses
     from tests.conftest import contract_self_distance
     cfg = dataclasses.replace(synth.QWEN3_8B, layers=2, prompt_tokens=300, decode_tokens=4)

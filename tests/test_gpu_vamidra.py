@@ -211,7 +211,8 @@ def test_first_tokens(built_lib, full, count, dtype):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_prompts_of_several_blocks(built_lib, dtype):
-    """More positions than one block step carries, more wanted places than one head launch does."""
+    """More positions than one block step carries in fp32 (in bf16: test_gpu_long_prompts.py), more wanted places than one
+    head launch does."""
     cfg = M.config([M.attention(window=300, keep=5), M.space(heads=2, groups=1, norm_groups=2),
                     M.attention(window=70, heads=6, kv_heads=3)], loop=(0, 2, 2))
     w = M.weights(cfg)

@@ -6,11 +6,13 @@
 //     projection.cu:192-262 one skinny GEMM per projection);
 //   * the chunked prefill of session_start — up to 2048 prompt positions of one session at a time
 //     (reference: session_decode_prefill.inc.cu:1879-2245, prefill_kernels.cu:66-170).
-// Per layer: RMSNorm of the block -> QKV block projection -> (prefill: q/k-norm + RoPE + paged KV
-// publish for all rows) -> split attention, one set of blocks per row -> O block projection with
-// the residual add in its epilogue -> RMSNorm -> gate/up block projection with SwiGLU in its
-// epilogue -> down block projection with the residual add.  The projections are the tcgen05 block
-// kernel (gemm_tc.cu); attention is the session's own fused kernel in its row form.
+// Per layer: RMSNorm of the block -> QKV block projection -> q/k-norm + RoPE + paged KV publish for
+// all rows -> attention -> O block projection with the residual add in its epilogue -> RMSNorm ->
+// gate/up block projection with SwiGLU in its epilogue -> down block projection with the residual
+// add, or the sparse MLP of a block (moe_block.cu).  The projections are the tcgen05 block kernels
+// (gemm_tc.cu; gemm_wide.cu where the tokens are many); attention runs on 128-row tiles
+// (prefill_attention.cu) in a prefill of many rows, row by row on the paged kernel (attention.cu) or
+// the fused kernel's row form otherwise, and as mla_block.cu on latent caches.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -394,8 +396,9 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
                        ws.x_bf16, d.hidden, kEpilogueStore, nullptr, ws.qkv, nullptr);
     n += 2;
     const bool tiles = b.publish && ws.tile_prefill && b.rows >= kTilePrefillMinRows;
-    // Sparse models keep short blocks on the fused kernel's row form: it adds in the decode step's order, so hardly a
-    // rounding differs from the token-by-token prefill, and with it hardly a router's choice between near equals.
+    // Sparse models keep short blocks on the fused kernel's row form, whose attention adds in the decode step's order: the
+    // paged kernel takes the same time, and the more roundings differ from the token-by-token prefill, the more often a
+    // router chooses differently between near equals.
     const bool paged = !tiles && !b.k_maps.empty() && !s->has_moe;
     if (err == cudaSuccess && d.mla()) {
       MlaBlockParams mp{};
@@ -456,10 +459,10 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       n += 1;
       if (err != cudaSuccess) break;
     } else if (paged) {
-      // every row's K/V (its own newest row included) is in its cache and its queries are prepared
-      for (uint32_t at = 0; err == cudaSuccess && at < b.rows; at += ws.part_rows) {
+      // every row's K/V (its own newest row included) is in its cache and its queries are prepared; blocks of more rows
+      // than have partials (part_rows) are prefill blocks on tiles
       AttentionParams ap{};
-      ap.batch = std::min(ws.part_rows, b.rows - at);
+      ap.batch = b.rows;
       ap.heads = d.heads;
       ap.kv_heads = d.kv_heads;
       ap.head_dim = d.head_dim;
@@ -467,13 +470,12 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       ap.partial_acc = ws.partial_acc;
       ap.partial_m = ws.partial_m;
       ap.partial_l = ws.partial_l;
-      ap.out_bf16 = ws.attn + static_cast<uint64_t>(at) * ah;
+      ap.out_bf16 = ws.attn;
       ap.error_word = s->device_error;
-      ap.rows = ws.attn_rows + at;
+      ap.rows = ws.attn_rows;
       ap.layer = l;
       err = launch_attention_rows(b.stream, ap, b.k_maps.data(), b.v_maps.data(), static_cast<uint32_t>(b.k_maps.size()));
       n += 2;
-      }
       if (err != cudaSuccess) break;
     } else {
     FusedAttentionParams fp{};

@@ -518,7 +518,7 @@ cudaError_t launch_window_publish(cudaStream_t stream, const WindowAttentionPara
 // One token per row: the lone decode step (rows == nullptr: prepares q and appends K/V itself) or block rows.
 cudaError_t launch_window_attention(cudaStream_t stream, const WindowAttentionParams &p);
 // Consecutive positions of one session on the tensor pipe (bf16 cache only): prefill_attention.cu where it takes the
-// shape and the rows fill it, mma.sync tiles otherwise.
+// shape, mma.sync tiles otherwise.
 cudaError_t launch_window_prefill(cudaStream_t stream, const WindowAttentionParams &p);
 bool prefill_attention_supported(const WindowAttentionShape &s);
 cudaError_t configure_prefill_attention();

@@ -9,9 +9,10 @@
 //                             a shared expert runs through the same kernel as a group of all rows
 //   moe_block_combine_kernel  residual + the row's slots in rank order + the shared expert
 //
-// Arithmetic is that of the decode step (moe.cu): fp32 normalised rows and fp32 SwiGLU outputs enter the projections
-// unrounded, here as two bf16 parts (the product loses 2^-17 of an element), two MMAs into one fp32 accumulator; router
-// logits are the same fp32 sums in the same order; contributions are added in rank order, the shared expert last.
+// Arithmetic is that of the decode step (moe.cu) up to roundings: fp32 normalised rows and fp32 SwiGLU outputs enter the
+// projections as two bf16 parts (2^-17 of an element is lost), two MMAs into one fp32 accumulator.  Sums run in another
+// order than there: a router logit is added by the lanes of a warp (there by a block of 256 threads), a row's contributions
+// in rank order with the shared expert last (there per lane before the lanes are added).
 //
 // What bounds the projections: the expert weights out of HBM while an expert has up to about 128 tokens, the tensor
 // pipe beyond.  A block therefore takes a pair of 128-row weight tiles (gate and up rows of the same index, or 256 rows

@@ -66,10 +66,7 @@ __device__ __noinline__ void gather_prologue(const ProjectionParams &p, uint16_t
 // about 1 % slower; holding a slot back ahead of the plain vector copy of O/down too: no gain).
 // The tensor-parallel gather prologue polls its entries behind the same queue and gains the same
 // way (its held-back slot is issued by the first stream_fill of stream_consume).
-#ifndef NERVA_PREWAIT_SLOTS
-#define NERVA_PREWAIT_SLOTS (NERVA_STREAM_SLOTS - 1)
-#endif
-constexpr uint32_t kPrewaitSlots = NERVA_PREWAIT_SLOTS;
+constexpr uint32_t kPrewaitSlots = kStreamSlots - 1u;
 constexpr uint32_t kPlainL2PrefetchBytes = 16384;  // per warp, after the plain vector copy
 
 template <uint32_t EPI, bool TP>

@@ -28,19 +28,10 @@
 
 namespace nb {
 
-#ifndef NERVA_STREAM_WARPS
-#define NERVA_STREAM_WARPS 8
-#endif
-#ifndef NERVA_STREAM_SLOTS
-#define NERVA_STREAM_SLOTS 3
-#endif
-#ifndef NERVA_CHUNK_BYTES
-#define NERVA_CHUNK_BYTES 8192
-#endif
-constexpr uint32_t kStreamWarps = NERVA_STREAM_WARPS;
+constexpr uint32_t kStreamWarps = 8;
 constexpr uint32_t kStreamThreads = kStreamWarps * 32;
-constexpr uint32_t kStreamSlots = NERVA_STREAM_SLOTS;
-constexpr uint32_t kChunkBytes = NERVA_CHUNK_BYTES;
+constexpr uint32_t kStreamSlots = 3;
+constexpr uint32_t kChunkBytes = 8192;
 constexpr uint32_t kRingBytes = kStreamWarps * kStreamSlots * kChunkBytes;
 constexpr uint32_t kSweepBytes = 512;  // 32 lanes x 16 bytes
 static_assert(kChunkBytes % (4 * kSweepBytes) == 0, "a chunk is a whole number of 4-sweep steps");

@@ -9,24 +9,25 @@
 // Queries and probabilities are fp32 values; each enters as a bf16 rounding and its remainder, two MMAs into the same
 // accumulator, so a product loses only the rounding of the cached row (the contract of the other attention kernels).
 //
-// What bounds it: the tensor pipe, 4 x 512 MMA cycles per tile (two parts of Q, two of P), as long as the softmax of a
-// tile (about 8 instructions and one exponential for each of a thread's 128 scores) fits beside it.  S has two
-// buffers: S(j+1) is computed while the softmax works on S(j).  The output accumulator is rescaled only when a row's
-// maximum has grown by more than 2^8 since the reference it uses (the probabilities stay below 2^8, the sums exact
-// to fp32): after the first tiles that almost never happens.
-// One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), but two
+// What bounds it: the softmax.  The MMAs of a tile are 4 x 512 cycles (two parts of Q, two of P), but a tile takes about
+// 6800 (75 and 150 us a layer for the two chunks of a 3001-token prompt, 32 heads: 9200 tiles on 148 SMs), because a
+// tile's chain of scores out of tensor memory, maximum, 128 exponentials a thread, two packs and the stores back runs by
+// itself: the tensor pipe works for less than a third of the time.  S has two buffers: S(j+1) is computed while the
+// softmax works on S(j).  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since
+// the reference it uses (the probabilities stay below 2^8, the sums exact to fp32): after the first tiles that almost
+// never happens.
+// One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), and two
 // groups of softmax warps, each with every second tile, a running maximum, a sum and an output accumulator of its own,
-// added at the end: a tile's softmax is a chain of about 6000 cycles for one warp per scheduler, which one group could
-// not hide behind 2048 cycles of MMA (2048 tokens, 32 heads: 117 us with one group).
+// added at the end.  The second group gives little: 2048 tokens, 32 heads, 117 us with one group, 114 with two.
 //
-// Measured (whole prefill, 8B shapes, 8 layers; row by row through the decode kernel before): 3001 tokens 19.5 ms
-// (33.1), 12000 tokens 101.6 ms (279.1); vuvolix 1.7b, window 1024, 2048 tokens 18.6 ms (23.0 with mma.sync tiles).
+// Measured (whole prefill, 8B shapes, 8 layers and head; row by row through the decode kernel before): 512 tokens 3.2 ms
+// (5.5), 3001 tokens 13.2 (40.5), projections on pairs of SMs included; vuvolix 1.7b, window 1024, 2048 tokens 12.8 (38.4).
 //
 // Roles (320 threads): warps 0..3 and 4..7 softmax, rescaling and the output (warp w reads tensor-memory lanes
-// 32 (w % 4) ..), warp 8 brings K and V (one 2-D TMA box per page and 64 columns, 128-byte swizzle), warp 9 issues the MMAs.  (cp.async by
-// two warps instead of TMA: their 1800 instructions per tile took 10,700 cycles, five times the MMAs.)  Tiles outside
-// every row's window are never loaded.  Every wait is bounded; one that gives up sets the error word and the block's
-// abort flag, and all roles leave.
+// 32 (w % 4) ..), warp 8 brings K and V (one 2-D TMA box per page and 64 columns, 128-byte swizzle), warp 9 issues the
+// MMAs and cleans the values of tiles at an edge.  (cp.async by two warps instead of TMA: their 1800 instructions per
+// tile took 10,700 cycles, five times the MMAs.)  Tiles outside every row's window are never loaded.
+// Every wait is bounded; one that gives up sets the error word and the block's abort flag, and all roles leave.
 #include "gemm_device.cuh"
 #include "mma_bf16.cuh"
 #include "window_device.cuh"

@@ -29,9 +29,10 @@ namespace {
 
 typedef NervaCudaHfDecodeSequenceSession Session;
 
-// Rows of a prefill block from which on its attention runs on 128-row tiles (prefill_attention.cu) and not row by row:
-// 8B shapes, 33 rows 1.49 (row by row 1.41), 128 rows 2.12 (2.21), 3001 rows 19.5 (33.1) ms for 8 layers and head.
-constexpr uint32_t kTilePrefillMinRows = 64;
+// Rows of a sparse model's prefill block from which on its attention runs on 128-row tiles and not row by row in the fused
+// kernel: 6 layers of 64 experts, 64 rows 1.62 ms (row by row 1.61), 96 rows 1.71 (1.79).  Behind a long context tiles would
+// pay from 16 rows on; short blocks stay with the step's order of sums all the same (below).
+constexpr uint32_t kSparseTileMinRows = 64;
 constexpr uint32_t kNormThreads = 256;  // the thread count the single-token prologue normalises with
 
 __device__ __forceinline__ uint32_t row_token(const BlockTokenRow &r) {
@@ -395,7 +396,7 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       err = block_gemm(b, s->weights->qkv_packed + static_cast<uint64_t>(l) * qkv_rows * d.hidden, qkv_rows, d.hidden,
                        ws.x_bf16, d.hidden, kEpilogueStore, nullptr, ws.qkv, nullptr);
     n += 2;
-    const bool tiles = b.publish && ws.tile_prefill && b.rows >= kTilePrefillMinRows;
+    const bool tiles = b.publish && ws.tile_prefill && (s->has_moe ? b.rows >= kSparseTileMinRows : prefill_tiles_pay(b.rows, b.longest));
     // Sparse models keep short blocks on the fused kernel's row form, whose attention adds in the decode step's order: the
     // paged kernel takes the same time, and the more roundings differ from the token-by-token prefill, the more often a
     // router chooses differently between near equals.
@@ -428,7 +429,7 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       // few rows: a head per warp; many: all heads of a row in one block
       const uint32_t query_heads = tiles || paged ? d.heads : 0u;
       const uint32_t groups = (d.kv_heads + query_heads + kPublishWarps - 1u) / kPublishWarps;
-      const dim3 grid(b.rows >= kTilePrefillMinRows ? 1u : groups, b.rows);
+      const dim3 grid(tiles ? 1u : groups, b.rows);
       auto publish = d.head_dim == 128 ? block_kv_publish_kernel<4> : block_kv_publish_kernel<2>;
       err = launch_with_pdl(publish, grid, dim3(kPublishWarps * 32), 0, b.stream, b.pdl, ws.attn_rows, l, d.heads,
                             query_heads, d.kv_heads, arena_at(s, L.k_bias), arena_at(s, L.v_bias), arena_at(s, L.k_norm),

@@ -521,6 +521,15 @@ cudaError_t launch_window_attention(cudaStream_t stream, const WindowAttentionPa
 // shape, mma.sync tiles otherwise.
 cudaError_t launch_window_prefill(cudaStream_t stream, const WindowAttentionParams &p);
 bool prefill_attention_supported(const WindowAttentionShape &s);
+// Whether a prefill block's attention is quicker on 128-row tiles than row by row.  A tile walks its keys alone, a chain of
+// a few us per 128 of them however few its rows; row by row, every row reads its keys and its blocks share the GPU.  So
+// tiles want rows, and fewer of them the more keys there are.  Whole appends in ms, tiles against rows: 8B layers, 64 / 72 /
+// 80 rows of a new prompt 1.49 1.44, 1.80 1.79, 1.81 1.82; 32 / 40 / 48 rows behind 1000 tokens 1.60 1.48, 1.58 1.60, 1.59
+// 1.62; vuvolix, 64 / 80 / 96 new rows 2.36 2.10, 2.71 2.62, 2.83 2.78; 32 / 48 behind 400 2.38 2.24, 2.37 2.69; 32 / 40
+// behind 2000 2.67 2.61, 2.73 3.25.
+inline bool prefill_tiles_pay(uint32_t rows, uint32_t keys) {
+  return rows >= (keys <= 80u ? 80u : keys >= 400u ? 40u : 90u - keys / 8u);
+}
 cudaError_t configure_prefill_attention();
 // p.keys, p.values and p.page_count name the session's cache, as for one token.
 cudaError_t launch_prefill_attention(cudaStream_t stream, const WindowAttentionParams &p);

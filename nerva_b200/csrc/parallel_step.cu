@@ -113,10 +113,6 @@ WindowAttentionParams layer_attention(const ParallelPlan &plan, const ParallelLa
   return p;
 }
 
-// Rows below which a block's attention is one query per thread block: a tile of the tensor-pipe kernel
-// would be mostly empty and walk its keys alone.
-constexpr uint32_t kPrefillTileMinRows = 8;
-
 // Checks a layer's attention and fills its part of the plan; why it is refused, or null.
 const char *plan_attention(const NervaB200ParallelLayer &in, bool f32, float eps, ParallelPlan *plan, ParallelLayerPlan *out) {
   ParallelLayerPlan &l = *out;
@@ -405,7 +401,8 @@ cudaError_t enqueue_block_attention(Session *s, const ParallelBlock &b, const Pa
   *launches += 2;
   const cudaError_t err = launch_window_publish(b.stream, a);
   if (err != cudaSuccess) return err;
-  if (b.one_session && b.rows >= kPrefillTileMinRows && !plan.f32) return launch_window_prefill(b.stream, a);
+  const uint32_t keys = a.s.window != 0 ? std::min(b.longest, a.s.window + a.s.keep_first) : b.longest;
+  if (b.one_session && !plan.f32 && prefill_tiles_pay(b.rows, keys)) return launch_window_prefill(b.stream, a);
   a.splits = window_rows_splits(l.shape, b.rows, b.longest, s->sm_count);
   return launch_window_attention(b.stream, a);
 }

@@ -65,3 +65,30 @@ def test_many_query_heads_of_one_key_head(built_lib, heads, dim, mixer):
     got = s.append(tokens, range(200), reset=True)
     assert M.worst_position(got, O.forward(cfg, w, tokens)) < 2 * M.TOLERANCE["bfloat16"]
     s.destroy()
+
+
+@pytest.mark.parametrize("first,sizes", [(0, (64, 79, 80, 81, 96)), (120, (64, 65, 75, 76)), (420, (16, 39, 40, 41))])
+def test_rows_around_where_tiles_begin(built_lib, first, sizes):
+    """Portions of fewer rows go row by row, the more keys there are the fewer: 80 of a new prompt, 40 behind 400 keys."""
+    from tests import vamidra_models as M
+    from tests import vamidra_oracle as O
+    cfg, ck = _checkpoint(8, 2, 128)
+    windowed = M.config([M.attention(ff=0, dim=64, vdim=64, window=450, keep=3, cap=0.0), M.attention(ff=0, dim=128, vdim=128, window=300)],
+                        width=128)
+    w = M.weights(windowed)
+    dense = CudaHfDecodeSequenceSession(ck, 512)
+    layers = CudaHfDecodeSequenceSession(M.checkpoint(windowed, w), 512, compute="bfloat16")
+    longest = first + max(sizes)
+    prompt, tokens = synth.uniform_u32(5, synth.T_PROMPT, longest, cfg.vocab), M.tokens(windowed, longest)
+    oracle = O.forward(windowed, w, tokens)
+    for rows in sizes:
+        want = _by_decode(ck, prompt[:first + rows], 512)
+        if first:
+            dense.append(prompt[:first], reset=True)
+            layers.append(tokens[:first], reset=True)
+        got = dense.append(prompt[first:first + rows], want=[rows - 1], reset=first == 0)[0]
+        assert np.abs(got - want).max() <= LOGIT_ATOL, rows
+        got = layers.append(tokens[first:first + rows], range(rows), reset=first == 0)
+        assert M.worst_position(got, oracle[first:first + rows]) < 2 * M.TOLERANCE["bfloat16"], rows
+    dense.destroy()
+    layers.destroy()

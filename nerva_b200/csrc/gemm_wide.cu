@@ -13,7 +13,8 @@
 // split: there is no workspace and no second launch.  Tokens per tile: choose_tile_tokens below.
 //
 // Measured alone with cold caches, launch included (and as chunks of 256 tokens in gemm_tc.cu): 2048 tokens x
-// 24576 x 4096 363 us, 1135 TFLOP/s (8 x 115); 4096 x 12288 188 us (8 x 50); 6144 x 4096 118 us (8 x 40).
+// 24576 x 4096 363 us, 1135 TFLOP/s (8 x 115); 4096 x 12288 188 us (8 x 50); 6144 x 4096 118 us (8 x 40).  Among the
+// launches of a prefill, with the SwiGLU and residual epilogues: 425, 200 and 108 us, the tensor pipe active 51 to 61 %.
 //
 // Roles inside a block (192 threads), as in gemm_tc.cu: warp 0 issues the TMA copies into the block's own ring,
 // warp 1 of the pair's first block issues the MMAs for both (its `full` barriers count the bytes of both blocks),

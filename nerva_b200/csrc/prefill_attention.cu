@@ -10,15 +10,15 @@
 // accumulator, so a product loses only the rounding of the cached row (the contract of the other attention kernels).
 //
 // What bounds it: the softmax.  The MMAs of a tile are 4 x 512 cycles (two parts of Q, two of P), but a tile takes about
-// 6800 (75 and 150 us a layer for the two chunks of a 3001-token prompt, 32 heads: 9200 tiles on 148 SMs), because a
-// tile's chain of scores out of tensor memory, maximum, 128 exponentials a thread, two packs and the stores back runs by
-// itself: the tensor pipe works for less than a third of the time.  S has two buffers: S(j+1) is computed while the
+// 7300 (2048 tokens, 32 heads: 4352 tiles on 148 SMs in 122 us), because a tile's chain of scores out of tensor memory,
+// maximum, 128 exponentials a thread, two packs and the stores back runs by itself: the tensor pipe is active 31 % of the
+// time.  S has two buffers: S(j+1) is computed while the
 // softmax works on S(j).  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since
 // the reference it uses (the probabilities stay below 2^8, the sums exact to fp32): after the first tiles that almost
 // never happens.
 // One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), and two
 // groups of softmax warps, each with every second tile, a running maximum, a sum and an output accumulator of its own,
-// added at the end.  The second group gives little: 2048 tokens, 32 heads, 117 us with one group, 114 with two.
+// added at the end.  The second group gives little: 2048 tokens, 32 heads, 117 us with one group, 114 with two when it was added.
 //
 // Measured (whole prefill, 8B shapes, 8 layers and head; row by row through the decode kernel before): 512 tokens 3.2 ms
 // (5.5), 3001 tokens 13.2 (40.5), projections on pairs of SMs included; vuvolix 1.7b, window 1024, 2048 tokens 12.8 (38.4).

@@ -2,39 +2,47 @@
 //
 // A projection y[n] = sum_k W[n][k] * x[k] at one token is pure HBM streaming:
 // every weight byte is read once and used once.  The rows of a projection are
-// dealt to thread blocks as equal contiguous row ranges, and inside a block the
-// BYTES of that range are dealt to the warps as equal contiguous byte ranges
-// (cut at 512-byte lane sweeps, not at row boundaries), so every warp of the
+// dealt to thread blocks as equal contiguous row ranges, and inside a block two rows
+// are taken together: the sweeps (512 bytes of each row) of the block's row pairs are
+// dealt to the warps in equal runs, cut anywhere in a row, so every warp of the
 // grid streams the same amount of memory whatever the shape.  Each warp owns a
 // private ring of shared-memory slots that it keeps filled with pieces ("chunks",
-// at most kChunkBytes, never crossing a row end) of its range through 1-D bulk
-// TMA copies, and drains them with 128-bit shared loads and fp32 FMAs.  There is
+// at most kChunkBytes, never crossing the rows' ends) of its run through 1-D bulk
+// TMA copies, one per row.  There is
 // no block-level synchronisation in the loop: a warp waits only on the mbarrier
 // of the slot it is about to read and refills that slot as soon as it has read it.
+//
+// The arithmetic is on the tensor pipe (mma.sync, see sweep_mma), not for its rate: a launch
+// begins with a full ring, and what the stream loses is the time until the ring has been
+// worked off.  With unpacking and FMAs a sweep of one row took 26 instructions and a block went through its ring
+// at 25 bytes per cycle, hardly more than its share of HBM (22); with two MMAs and three loads for a sweep of two
+// rows it is bound by shared memory, 85 bytes per cycle.  Steps before and after, us: vamidra 1.7b widths (28 layer
+// runs) 1376 and 1249, vuvolix 1016 and 991, 8 layers of the 8B shapes 784 and 762, the 4-layer hidden-512 model 118 and 99.
 //
 // The chunk list runs ACROSS projections (a job list): weights do not depend on
 // activations, so the issue side of a ring runs ahead into the next projection
 // while the block is still normalising, attending or waiting at a grid barrier.
 //
-// A row that lies inside one warp's range is reduced by that warp and its total
-// goes to the block's row-total buffer in shared memory.  A row cut by a range
-// boundary leaves one partial per warp in that warp's two "edge" records.  After
-// the block has synchronised, stream_finish() adds the edge partials to the
+// A pair that lies inside one warp's range is reduced by that warp and its totals
+// go to the block's row-total buffer in shared memory.  A pair cut by a range
+// boundary leaves one partial per row and warp in that warp's two "edge" records.  After
+// the block has synchronised, stream_row_total() adds the edge partials to the
 // totals in ascending warp order, so results do not depend on timing and are
 // bit-identical run to run.
 #pragma once
 
-#include "common.cuh"
+#include "mma_bf16.cuh"
 
 namespace nb {
 
 constexpr uint32_t kStreamWarps = 8;
 constexpr uint32_t kStreamThreads = kStreamWarps * 32;
 constexpr uint32_t kStreamSlots = 3;
-constexpr uint32_t kChunkBytes = 8192;
+constexpr uint32_t kChunkBytes = 8192;               // of both rows of a pair
+constexpr uint32_t kChunkRowBytes = kChunkBytes / 2u;
 constexpr uint32_t kRingBytes = kStreamWarps * kStreamSlots * kChunkBytes;
 constexpr uint32_t kSweepBytes = 512;  // 32 lanes x 16 bytes
-static_assert(kChunkBytes % (4 * kSweepBytes) == 0, "a chunk is a whole number of 4-sweep steps");
+static_assert(kChunkRowBytes % (4 * kSweepBytes) == 0, "a chunk is a whole number of 4-sweep steps");
 constexpr uint32_t kNoRow = 0xffffffffu;
 
 struct JobDesc {
@@ -57,11 +65,12 @@ __host__ __device__ inline uint32_t max_rows_per_block(uint32_t rows, uint32_t u
   return ((units + blocks - 1) / blocks) * unit;
 }
 
-// One warp's share of one job: bytes [begin, end) of the block's row range,
-// offsets relative to the first byte of the block's first row.
+// One warp's share of one job.  Positions count the bytes of ONE row of each pair (pair p, column byte c: p * row_bytes
+// + c); the range [begin, end) is the warp's.
 struct WarpJob {
-  const uint8_t *base;   // first byte of the block's first row
+  const uint8_t *base;  // first byte of the block's first row
   uint32_t row_bytes;
+  uint32_t rows;        // the block's; the last pair of an odd number has one
   uint32_t begin, end;
 };
 
@@ -71,55 +80,55 @@ __device__ __forceinline__ WarpJob warp_job(const JobDesc &d) {
   WarpJob j;
   j.row_bytes = d.cols * 2u;
   j.base = reinterpret_cast<const uint8_t *>(d.weight) + static_cast<uint64_t>(row_begin) * j.row_bytes;
-  const uint32_t warp = threadIdx.x >> 5;
+  j.rows = row_end - row_begin;
+  const uint32_t warp = threadIdx.x >> 5, pairs = (j.rows + 1u) / 2u;
   if (j.row_bytes % kSweepBytes == 0) {
-    // cut the block's bytes into equal runs of whole 512-byte lane sweeps
-    const uint32_t sweeps = (row_end - row_begin) * (j.row_bytes / kSweepBytes);
+    // cut the block's pairs into equal runs of whole 512-byte lane sweeps
+    const uint32_t sweeps = pairs * (j.row_bytes / kSweepBytes);
     j.begin = static_cast<uint32_t>(static_cast<uint64_t>(sweeps) * warp / kStreamWarps) * kSweepBytes;
     j.end = static_cast<uint32_t>(static_cast<uint64_t>(sweeps) * (warp + 1) / kStreamWarps) * kSweepBytes;
   } else {
-    // rows that are not a whole number of sweeps are dealt whole
-    const uint32_t rows = row_end - row_begin;
-    j.begin = static_cast<uint32_t>(static_cast<uint64_t>(rows) * warp / kStreamWarps) * j.row_bytes;
-    j.end = static_cast<uint32_t>(static_cast<uint64_t>(rows) * (warp + 1) / kStreamWarps) * j.row_bytes;
+    // rows that are not a whole number of sweeps are dealt in whole pairs
+    j.begin = static_cast<uint32_t>(static_cast<uint64_t>(pairs) * warp / kStreamWarps) * j.row_bytes;
+    j.end = static_cast<uint32_t>(static_cast<uint64_t>(pairs) * (warp + 1) / kStreamWarps) * j.row_bytes;
   }
   return j;
 }
 
 // A cursor walks a WarpJob chunk by chunk.
 struct StreamCursor {
-  uint32_t pos;      // byte offset of the next chunk
-  uint32_t row_end;  // end byte of the row that contains pos
-  uint32_t row;      // block-local index of that row
+  uint32_t pos;      // position of the next chunk
+  uint32_t row_end;  // end position of the pair that contains pos
+  uint32_t pair;     // block-local index of that pair
 };
 __device__ __forceinline__ StreamCursor cursor_at_start(const WarpJob &j) {
   StreamCursor c;
   c.pos = j.begin;
-  c.row = j.begin / j.row_bytes;
-  c.row_end = (c.row + 1u) * j.row_bytes;
+  c.pair = j.begin / j.row_bytes;
+  c.row_end = (c.pair + 1u) * j.row_bytes;
   return c;
 }
-// Length of the chunk at the cursor, its position, the end of its row and the row's index;
+// Length of the chunk at the cursor in each row, its position, the end of its pair and the pair's index;
 // advances the cursor.
 __device__ __forceinline__ uint32_t cursor_next(const WarpJob &j, StreamCursor &c, uint32_t *pos,
-                                                uint32_t *row_end, uint32_t *row = nullptr) {
-  uint32_t len = kChunkBytes;
+                                                uint32_t *row_end, uint32_t *pair) {
+  uint32_t len = kChunkRowBytes;
   if (c.row_end - c.pos < len) len = c.row_end - c.pos;
   if (j.end - c.pos < len) len = j.end - c.pos;
   *pos = c.pos;
   *row_end = c.row_end;
-  if (row != nullptr) *row = c.row;
+  *pair = c.pair;
   c.pos += len;
   if (c.pos == c.row_end) {
     c.row_end += j.row_bytes;
-    c.row += 1u;
+    c.pair += 1u;
   }
   return len;
 }
 
 struct EdgeRecord {
-  uint32_t row;  // block-local row, kNoRow when unused
-  float value;
+  uint32_t pair;  // block-local pair, kNoRow when unused
+  float value[2];
 };
 
 // Shared-memory bookkeeping of a block's streams.
@@ -181,42 +190,35 @@ __device__ __forceinline__ void stream_fill(RowStream &rs, uint32_t depth = SLOT
       }
       continue;
     }
-    uint32_t pos, row_end;
-    const uint32_t len = cursor_next(rs.issue, rs.issue_cursor, &pos, &row_end);
+    uint32_t pos, row_end, pair;
+    const uint32_t len = cursor_next(rs.issue, rs.issue_cursor, &pos, &row_end, &pair);
     const uint32_t slot = rs.issued % SLOTS;
     if ((threadIdx.x & 31u) == 0) {
-      mbar_arrive_expect_tx(&rs.bars[slot], len);
-      tma_load_1d_hint(rs.ring + slot * kChunkBytes, rs.issue.base + pos, len, &rs.bars[slot], rs.policy);
+      const bool both = 2u * pair + 1u < rs.issue.rows;
+      const uint8_t *src = rs.issue.base + pos + static_cast<uint64_t>(pair) * rs.issue.row_bytes;
+      mbar_arrive_expect_tx(&rs.bars[slot], both ? 2u * len : len);
+      tma_load_1d_hint(rs.ring + slot * kChunkBytes, src, len, &rs.bars[slot], rs.policy);
+      if (both)
+        tma_load_1d_hint(rs.ring + slot * kChunkBytes + kChunkRowBytes, src + rs.issue.row_bytes, len, &rs.bars[slot], rs.policy);
     }
     rs.issued += 1;
   }
 }
 
-// Asks L2 for the `bytes` that follow the chunks already issued (the warp's own span of the
-// current job only): the ring cannot hold more, but HBM can keep working while the block is
-// busy with its prologue.
+// Asks L2 for the `bytes` that follow the chunks already issued, half of them in each row of the pair (the warp's own
+// range of the current job only): the ring cannot hold more, but HBM can keep working while the block is busy with its
+// prologue.
 __device__ __forceinline__ void stream_prefetch_l2(const RowStream &rs, uint32_t bytes) {
-  if (rs.dead || bytes == 0 || rs.issue_job >= rs.job_count || (threadIdx.x & 31u) != 0) return;
-  const uint32_t pos = rs.issue_cursor.pos;
-  if (pos >= rs.issue.end) return;
-  uint32_t size = rs.issue.end - pos;
-  if (size > bytes) size = bytes;
+  const uint32_t lane = threadIdx.x & 31u;
+  if (rs.dead || bytes == 0 || rs.issue_job >= rs.job_count || lane > 1u) return;
+  const StreamCursor &c = rs.issue_cursor;
+  if (c.pos >= rs.issue.end || 2u * c.pair + lane >= rs.issue.rows) return;
+  uint32_t size = (rs.issue.end < c.row_end ? rs.issue.end : c.row_end) - c.pos;
+  if (size > bytes / 2u) size = bytes / 2u;
   size &= ~15u;
   if (size == 0) return;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rs.issue.base + pos), "r"(size) : "memory");
-}
-
-// dot of 8 bf16 weights with 8 bf16 activations, fp32.
-__device__ __forceinline__ float dot8(const uint4 &w, const uint4 &x, float acc) {
-  acc = fmaf(bf16x2_lo(w.x), bf16x2_lo(x.x), acc);
-  acc = fmaf(bf16x2_hi(w.x), bf16x2_hi(x.x), acc);
-  acc = fmaf(bf16x2_lo(w.y), bf16x2_lo(x.y), acc);
-  acc = fmaf(bf16x2_hi(w.y), bf16x2_hi(x.y), acc);
-  acc = fmaf(bf16x2_lo(w.z), bf16x2_lo(x.z), acc);
-  acc = fmaf(bf16x2_hi(w.z), bf16x2_hi(x.z), acc);
-  acc = fmaf(bf16x2_lo(w.w), bf16x2_lo(x.w), acc);
-  acc = fmaf(bf16x2_hi(w.w), bf16x2_hi(x.w), acc);
-  return acc;
+  const uint8_t *src = rs.issue.base + c.pos + static_cast<uint64_t>(c.pair + lane) * rs.issue.row_bytes;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(size) : "memory");
 }
 
 // Packed fp32 multiply-add (two lanes per instruction).
@@ -252,11 +254,21 @@ __device__ __forceinline__ float dot8_f32(const uint4 &w, const float4 &xa, cons
   acc = fmaf(bf16x2_hi(w.w), xb.w, acc);
   return acc;
 }
+
+// One lane sweep of a pair: 512 bytes of each row times the same 512 bytes of x.  A lane's 16 bytes are eight
+// columns of 64-byte slab lane / 4; the fragments of the MMA take the slabs of the first row as rows 0..7 of A, those
+// of the second as rows 8..15, and those of x as the columns of B, so the products of like slabs are the diagonals of
+// the two halves of the accumulator.  What stands beside the diagonals is never read.
+__device__ __forceinline__ void sweep_mma(float (&acc)[4], const uint4 &w0, const uint4 &w1, const uint4 &x) {
+  mma_bf16(acc, {w0.x, w1.x, w0.y, w1.y}, x.x, x.y);
+  mma_bf16(acc, {w0.z, w1.z, w0.w, w1.w}, x.z, x.w);
+}
+
 // Consumes job `index` (jobs are consumed in order, each exactly once, by every
 // warp of the block).  `x` is the bf16 activation vector in shared memory;
 // row_total[r] (shared, one float per block-local row, zeroed by the caller
-// before the block's previous synchronisation) receives the total of every row
-// that lies wholly inside this warp's range; partial rows go to sh.edge.
+// before the block's previous synchronisation) receives the totals of every pair
+// that lies wholly inside this warp's range; partial sums go to sh.edge.
 template <uint32_t SLOTS = kStreamSlots>
 __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, uint32_t index,
                                                const void *x, float *row_total,
@@ -265,15 +277,16 @@ __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, 
   const WarpJob job = warp_job(rs.jobs[index]);
   StreamCursor cur = cursor_at_start(job);
   if (lane == 0) {
-    sh.edge[warp][0].row = kNoRow;
-    sh.edge[warp][1].row = kNoRow;
+    sh.edge[warp][0].pair = kNoRow;
+    sh.edge[warp][1].pair = kNoRow;
   }
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const bool odd_slab = (lane & 4u) != 0, diagonal = (lane & 3u) == lane >> 3;  // column lane / 4 is in c[odd_slab] of lane % 4 == lane / 8
+  float sum0 = 0.0f, sum1 = 0.0f;
   uint32_t edges = 0;
-  bool row_from_start = job.begin % job.row_bytes == 0;  // this warp has seen the current row from byte 0
+  bool row_from_start = job.begin % job.row_bytes == 0;  // this warp has seen the current pair from its first column
   while (cur.pos < job.end) {
-    uint32_t pos, row_end, row;
-    const uint32_t len = cursor_next(job, cur, &pos, &row_end, &row);
+    uint32_t pos, row_end, pair;
+    const uint32_t len = cursor_next(job, cur, &pos, &row_end, &pair);
     stream_fill<SLOTS>(rs);
     const uint32_t slot = rs.consumed % SLOTS;
     const uint32_t parity = (rs.consumed / SLOTS) & 1u;
@@ -286,49 +299,60 @@ __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, 
     const uint8_t *wp = rs.ring + slot * kChunkBytes + lane * 16u;
     const uint32_t row_offset = pos - (row_end - job.row_bytes);  // bytes into the row
     const uint8_t *xp = reinterpret_cast<const uint8_t *>(x) + row_offset + lane * 16u;
-    if (len == kChunkBytes) {
+    // four accumulators, zeroed per chunk: chains of four MMAs, whose sums meet in fp32 adds
+    float acc[4][4];
 #pragma unroll
-      for (uint32_t i = 0; i < kChunkBytes / kSweepBytes; i += 4) {
-        const uint4 w0 = lds128(wp + (i + 0) * kSweepBytes), x0 = lds128(xp + (i + 0) * kSweepBytes);
-        const uint4 w1 = lds128(wp + (i + 1) * kSweepBytes), x1 = lds128(xp + (i + 1) * kSweepBytes);
-        const uint4 w2 = lds128(wp + (i + 2) * kSweepBytes), x2 = lds128(xp + (i + 2) * kSweepBytes);
-        const uint4 w3 = lds128(wp + (i + 3) * kSweepBytes), x3 = lds128(xp + (i + 3) * kSweepBytes);
-        acc[0] = dot8(w0, x0, acc[0]);
-        acc[1] = dot8(w1, x1, acc[1]);
-        acc[2] = dot8(w2, x2, acc[2]);
-        acc[3] = dot8(w3, x3, acc[3]);
-      }
+    for (uint32_t i = 0; i < 4u; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+    if (len == kChunkRowBytes) {
+#pragma unroll
+      for (uint32_t i = 0; i < kChunkRowBytes / kSweepBytes; ++i)
+        sweep_mma(acc[i & 3u], lds128(wp + i * kSweepBytes), lds128(wp + kChunkRowBytes + i * kSweepBytes), lds128(xp + i * kSweepBytes));
     } else {
       uint32_t off = 0;
-      for (; off + 4u * kSweepBytes <= len; off += 4u * kSweepBytes) {
-        const uint4 w0 = lds128(wp + off), x0 = lds128(xp + off);
-        const uint4 w1 = lds128(wp + off + kSweepBytes), x1 = lds128(xp + off + kSweepBytes);
-        const uint4 w2 = lds128(wp + off + 2u * kSweepBytes), x2 = lds128(xp + off + 2u * kSweepBytes);
-        const uint4 w3 = lds128(wp + off + 3u * kSweepBytes), x3 = lds128(xp + off + 3u * kSweepBytes);
-        acc[0] = dot8(w0, x0, acc[0]);
-        acc[1] = dot8(w1, x1, acc[1]);
-        acc[2] = dot8(w2, x2, acc[2]);
-        acc[3] = dot8(w3, x3, acc[3]);
+      for (; off + 2u * kSweepBytes <= len; off += 2u * kSweepBytes) {
+#pragma unroll
+        for (uint32_t i = 0; i < 2u; ++i)
+          sweep_mma(acc[i], lds128(wp + off + i * kSweepBytes), lds128(wp + kChunkRowBytes + off + i * kSweepBytes),
+                    lds128(xp + off + i * kSweepBytes));
       }
-      // tail: whole sweeps, then (rows that are not a multiple of 512 bytes) the lanes that still have data
-      for (; off + lane * 16u < len; off += kSweepBytes) {
-        acc[0] = dot8(lds128(wp + off), lds128(xp + off), acc[0]);
+      // a last sweep: whole, or (rows that are not a multiple of 512 bytes) of the lanes that still have data
+      for (; off < len; off += kSweepBytes) {
+        uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w1 = w0, xv = w0;
+        if (off + lane * 16u < len) {
+          w0 = lds128(wp + off);
+          w1 = lds128(wp + kChunkRowBytes + off);
+          xv = lds128(xp + off);
+        }
+        __syncwarp();
+        sweep_mma(acc[2], w0, w1, xv);
       }
+    }
+    if (odd_slab) {
+      sum0 += (acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1]);
+      sum1 += (acc[0][3] + acc[1][3]) + (acc[2][3] + acc[3][3]);
+    } else {
+      sum0 += (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
+      sum1 += (acc[0][2] + acc[1][2]) + (acc[2][2] + acc[3][2]);
     }
     const bool row_done = pos + len == row_end;
     const bool range_done = pos + len == job.end;
     if (row_done || range_done) {
-      const float total = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-      if (lane == 0) {
-        if (row_done && row_from_start) {
+      // the first row's total to the lower half of the warp, the second's to the upper
+      const float mine = diagonal ? (lane < 16u ? sum0 : sum1) : 0.0f, theirs = diagonal ? (lane < 16u ? sum1 : sum0) : 0.0f;
+      float total = mine + __shfl_xor_sync(0xffffffffu, theirs, 16);
+#pragma unroll
+      for (int offset = 8; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
+      if ((lane & 15u) == 0) {
+        const uint32_t row = 2u * pair + (lane >> 4);
+        if (!(row_done && row_from_start)) {
+          sh.edge[warp][edges].pair = pair;
+          sh.edge[warp][edges].value[lane >> 4] = total;
+        } else if (row < job.rows) {
           row_total[row] = total;
-        } else {
-          sh.edge[warp][edges].row = row;
-          sh.edge[warp][edges].value = total;
         }
       }
       if (!(row_done && row_from_start)) edges += 1;
-      acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+      sum0 = sum1 = 0.0f;
       row_from_start = true;
     }
     __syncwarp();
@@ -339,14 +363,14 @@ __device__ __forceinline__ void stream_consume(RowStream &rs, StreamShared &sh, 
 }
 
 // After the block has synchronised behind stream_consume: row r's total with
-// the partials of cut rows added in ascending warp order.
+// the partials of cut pairs added in ascending warp order.
 __device__ __forceinline__ float stream_row_total(const StreamShared &sh, const float *row_total,
                                                   uint32_t r) {
   float total = row_total[r];
 #pragma unroll
   for (uint32_t w = 0; w < kStreamWarps; ++w) {
-    if (sh.edge[w][0].row == r) total += sh.edge[w][0].value;
-    if (sh.edge[w][1].row == r) total += sh.edge[w][1].value;
+    if (sh.edge[w][0].pair == r >> 1) total += sh.edge[w][0].value[r & 1u];
+    if (sh.edge[w][1].pair == r >> 1) total += sh.edge[w][1].value[r & 1u];
   }
   return total;
 }

@@ -141,3 +141,14 @@ def test_projection_bench_entry_point(built_lib):
     assert rc == 0 and out.status == 0 and out.mismatch_count == 0
     assert out.custom_avg_ns > 0 and out.custom_graph_avg_ns > 0 and out.hot_path_allocations == 0
     assert out.matrix_bytes == 4096 * 4096 * 2
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 37, 147, 149, 297, 2049])
+@pytest.mark.parametrize("cols", [8, 64, 248, 256, 264, 768, 2048, 2056, 4096, 12288])
+def test_projection_of_row_pairs_at_their_edges(built_lib, rows, cols):
+    """Odd rows, ranges cut inside a pair, last sweeps that are not whole.  The inputs are multiples of 2^-14 (products)
+    of at most 2^-2: up to 4096 columns every partial sum is below 2^10 and exact in fp32, in any order; beyond, each of the
+    additions loses at most half of 2^-12 (sums below 2^12), and a row goes through 64 of them and a few more."""
+    rc, out = ops.projection_bench(rows, cols, iterations=1, warmup=1)
+    assert rc == 0 and out.status == 0 and out.mismatch_count == 0
+    assert out.max_abs_diff <= (0.0 if cols <= 4096 else 72 * 2.0 ** -13)

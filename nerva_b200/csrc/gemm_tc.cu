@@ -159,6 +159,8 @@ __global__ void __launch_bounds__(4 * kTileRows) gemm_fixup_kernel(GemmKernelPar
   const uint32_t m0 = blockIdx.y * kGroup + 4u * threadIdx.y;
   const uint64_t slot_floats = static_cast<uint64_t>(p.n_pad) * kTileRows;
   const float *base = p.workspace + static_cast<uint64_t>(m0) * kTileRows + row_in_tile;
+  float resid[4];
+  row_residual<4>(p, resid, tile * kTileRows + row_in_tile, m0);  // in flight with the partials
   float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   for (uint32_t q = 0; q < count; q += kFixupBatch) {
     float4 x[kFixupBatch];
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(4 * kTileRows) gemm_fixup_kernel(GemmKernelPar
     }
   }
   const float vals[4] = {v.x, v.y, v.z, v.w};
-  row_epilogue<4>(p, vals, tile * kTileRows + row_in_tile, m0, threadIdx.x & 31u);
+  row_epilogue<4>(p, vals, resid, tile * kTileRows + row_in_tile, m0, threadIdx.x & 31u);
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 2)
@@ -333,10 +335,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
       } else {
         const uint32_t row = seg.tile * kTileRows + row_in_tile;
+        float resid[kGroup];
+        row_residual<kGroup>(p, resid, row, 0);
         for (uint32_t g = 0; g < p.n_pad; g += kGroup) {
-          float v[kGroup];
+          float v[kGroup], next[kGroup];
           tmem_load16(taddr + g, v);
-          row_epilogue<kGroup>(p, v, row, g, lane);
+          row_residual<kGroup>(p, next, row, g + kGroup);  // zeros behind the last token
+          row_epilogue<kGroup>(p, v, resid, row, g, lane);
+#pragma unroll
+          for (uint32_t j = 0; j < kGroup; ++j) resid[j] = next[j];
         }
       }
       tcgen05_fence_before();

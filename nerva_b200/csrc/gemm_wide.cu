@@ -12,13 +12,17 @@
 // weight tiles (each read from HBM once) and all token tiles (which stay in L2).  The inner dimension is never
 // split: there is no workspace and no second launch.  Tokens per tile: choose_tile_tokens below.
 //
-// Measured alone with cold caches, launch included (and as chunks of 256 tokens in gemm_tc.cu): 2048 tokens x
-// 24576 x 4096 363 us, 1135 TFLOP/s (8 x 115); 4096 x 12288 188 us (8 x 50); 6144 x 4096 118 us (8 x 40).  Among the
-// launches of a prefill, with the SwiGLU and residual epilogues: 425, 200 and 108 us, the tensor pipe active 51 to 61 %.
+// The epilogue runs under the MMAs of the next tile, but a tile's has to be shorter than a tile's MMAs (17 us at 4096
+// columns), and the last one is not hidden: hence eight warps, values without branches and residuals a group ahead
+// (row_epilogue, row_residual).
 //
-// Roles inside a block (192 threads), as in gemm_tc.cu: warp 0 issues the TMA copies into the block's own ring,
+// Measured back to back, other weights each time, 2048 tokens (four warps and a branch per value before): 24576 x 4096
+// with SwiGLU 311 us, 1325 TFLOP/s (394), 281 without an epilogue; 4096 x 12288 with residual 158 (178); 6144 x 4096 89 (96);
+// 4096 x 4096 with residual 62 (85).  Loads alone would take 205 us of the first, MMAs alone 275.
+//
+// Roles inside a block (320 threads), as in gemm_tc.cu: warp 0 issues the TMA copies into the block's own ring,
 // warp 1 of the pair's first block issues the MMAs for both (its `full` barriers count the bytes of both blocks),
-// warps 2..5 read the accumulator and run the epilogue.  Commits of the MMAs are signalled to both blocks.  Two
+// warps 2..9 read the accumulator and run the epilogue, four of them every second group of tokens.  Commits of the MMAs are signalled to both blocks.  Two
 // accumulator buffers of 256 columns let the epilogue of one tile run under the MMAs of the next.  Every wait is
 // bounded; a wait that gives up sets the error word and the block's abort flag, the block drains and the pair
 // leaves together.  No copy is multicast.
@@ -31,8 +35,8 @@ constexpr uint32_t kPairRows = 2u * kTileRows;  // MMA M over the pair
 constexpr uint32_t kMinTileTokens = 64, kMaxTileTokens = 256;  // MMA N
 constexpr uint32_t kTokenStep = 32;             // tile sizes: whole 8-row swizzle atoms in each half, N a multiple of 16
 constexpr uint32_t kMaxStages = 8;
-constexpr uint32_t kThreads = 192;
-constexpr uint32_t kEpilogueWarps = 4;
+constexpr uint32_t kThreads = 320;
+constexpr uint32_t kEpilogueWarps = 8;
 constexpr uint32_t kTmemColumns = 512, kAccStride = 256;
 constexpr uint32_t kLeaderMask = 0xfeffffffu;   // clears the bit of a shared::cluster address that names the pair's second block
 
@@ -198,22 +202,27 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       stamp_pair(p.stamps, kStampAfterPrologue, pair, pairs);
     }
   } else {
-    // ---------------- epilogue (warps 2..5) ----------------
+    // ---------------- epilogue (warps 2..9) ----------------
     pdl_wait();
-    const uint32_t quarter = warp & 3u;
+    const uint32_t quarter = warp & 3u, from = ((warp - 2u) >> 2) * kGroup;
     uint32_t index = 0;
     for (uint32_t tile = pair; tile < tiles; tile += pairs, ++index) {
       const uint32_t acc = index & 1u;
-      if (!warp_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, p.error_word)) break;
-      tcgen05_fence_after();
       const uint32_t taddr = tmem_base + acc * kAccStride + ((quarter * 32u) << 16);
       const uint32_t row = (tile / t.token_tiles) * kPairRows + rank * kTileRows + quarter * 32u + lane;
       const uint32_t m0 = (tile % t.token_tiles) * t.tile_tokens;
       const uint32_t count = p.tokens - m0 < t.tile_tokens ? p.tokens - m0 : t.tile_tokens;
-      for (uint32_t g = 0; g < count; g += kGroup) {
-        float v[kGroup];
+      float resid[kGroup];
+      row_residual<kGroup>(p, resid, row, m0 + from);
+      if (!warp_wait(&sh.acc_full[acc], (index >> 1) & 1u, abort, p.error_word)) break;
+      tcgen05_fence_after();
+      for (uint32_t g = from; g < count; g += 2u * kGroup) {
+        float v[kGroup], next[kGroup];
         tmem_load16(taddr + g, v);
-        row_epilogue<kGroup>(p, v, row, m0 + g, lane);
+        row_residual<kGroup>(p, next, row, m0 + g + 2u * kGroup);
+        row_epilogue<kGroup>(p, v, resid, row, m0 + g, lane);
+#pragma unroll
+        for (uint32_t j = 0; j < kGroup; ++j) resid[j] = next[j];
       }
       tcgen05_fence_before();
       __syncwarp();

@@ -61,12 +61,10 @@ __host__ __device__ inline uint32_t round128(uint32_t v) { return (v + 127u) & ~
 
 // The sandwich prologue: x (shared memory) from the residual stream and a pending sublayer output.
 template <uint32_t KIND, class Fill>
-__device__ __forceinline__ void sandwich_norm(const ParallelProjectionParams &p, uint16_t *x, float *scratch, Fill fill) {
+__device__ __forceinline__ void sandwich_norm(const ParallelProjectionParams &p, const NormWeightRegs &weights,
+                                              const NormWeightRegs &after, uint16_t *x, float *scratch, Fill fill) {
   constexpr bool kJoin = KIND == kSandwichJoin;
   const uint32_t cols = kJoin ? p.cols0 / 2u : p.cols0, vecs = cols / 4u;
-  NormWeightRegs weights, after;
-  if (!kJoin) norm_weights_preload(weights, p.norm, cols);
-  if (p.pending != nullptr) norm_weights_preload(after, p.after, cols);
   pdl_wait();
   NormValueRegs h, y;
   norm_single_load(h, p.h, cols);
@@ -116,10 +114,9 @@ __device__ __forceinline__ void sandwich_norm(const ParallelProjectionParams &p,
 
 // x (shared memory) = grouped RMS norm of p.x_f32.  A warp's 128 values of one iteration lie in one part.
 template <class Fill>
-__device__ __forceinline__ void grouped_norm(const ParallelProjectionParams &p, uint16_t *x, float *scratch, Fill fill) {
+__device__ __forceinline__ void grouped_norm(const ParallelProjectionParams &p, const NormWeightRegs &weights, uint16_t *x,
+                                             float *scratch, Fill fill) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, vecs = p.cols0 / 4u;
-  NormWeightRegs weights;
-  norm_weights_preload(weights, p.norm, p.cols0);
   pdl_wait();
   NormValueRegs y;
   norm_single_load(y, p.x_f32, p.cols0);
@@ -171,11 +168,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
     sh.jobs[0] = JobDesc{gate_pairs(KIND) ? p.w1 : p.w0, rows_all, p.cols0, unit, 0};
     sh.jobs[1] = JobDesc{p.w1, p.rows1, p.cols1, 1, 0};
   }
+  // What does not depend on the previous kernel comes in front of the ring's copies, behind which it would wait for them:
+  // the weights of the prologue's norms and, beside the attention, the stream itself (late blocks of kParallelGate waited
+  // 5 us for it).  28 layer runs, us a step: vuvolix 1.7b widths 1017 and 970 to 1010, vamidra 1286 and 1255.
+  NormWeightRegs weights, other;  // other: of the pending output's norm, or the pass vector
+  NormValueRegs values;
+  const uint32_t norm_cols = KIND == kSandwichJoin ? p.cols0 / 2u : p.cols0;
+  if (KIND != kParallelOut && KIND != kSandwichJoin && (KIND != kSandwichOut || p.groups != 0)) norm_weights_preload(weights, p.norm, norm_cols);
+  if (sandwich_prologue(KIND) && p.pending != nullptr) norm_weights_preload(other, p.after, norm_cols);
+  if ((KIND == kParallelIn || KIND == kParallelGate || KIND == kParallelHead) && p.step != nullptr) norm_weights_preload(other, p.step, norm_cols);
+  if (KIND == kParallelGate) norm_single_load(values, p.h, norm_cols);
   __syncthreads();
   RowStream rs;
   stream_init<SLOTS>(rs, ring, sh.first, sh.jobs, second ? 2u : 1u);
   // ahead of a norm prologue one slot is held back: the activation loads would queue behind a whole ring
-  stream_fill<SLOTS>(rs, KIND == kParallelOut ? SLOTS : SLOTS - 1u);
+  stream_fill<SLOTS>(rs, KIND == kParallelOut || KIND == kParallelGate ? SLOTS : SLOTS - 1u);
 
   uint32_t begin0, end0, begin1 = 0, end1 = 0;
   block_row_range(rows_all, unit, blockIdx.x, gridDim.x, &begin0, &end0);
@@ -187,10 +194,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
   float resid_first = 0.0f;
   auto fill = [&]() { stream_fill<SLOTS>(rs); };  // the ring slot held back, behind the activation loads
   if (sandwich_prologue(KIND)) {
-    sandwich_norm<KIND>(p, x0, sh.scratch, fill);
+    sandwich_norm<KIND>(p, weights, other, x0, sh.scratch, fill);
   } else if (KIND == kSandwichOut) {
     if (p.groups != 0) {
-      grouped_norm(p, x0, sh.scratch, fill);
+      grouped_norm(p, weights, x0, sh.scratch, fill);
     } else {
       pdl_wait();
       const uint4 *src0 = reinterpret_cast<const uint4 *>(p.x0);
@@ -209,21 +216,19 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
     }
     stream_prefetch_l2(rs, kPlainL2PrefetchBytes);
   } else {
-    NormWeightRegs weights, step;
-    norm_weights_preload(weights, p.norm, p.cols0);
-    if (p.step != nullptr) norm_weights_preload(step, p.step, p.cols0);
     if (KIND != kParallelGate) pdl_wait();
     if (KIND == kParallelIn) pdl_trigger();  // whoever runs after this knows that h is complete
-    NormValueRegs values;
-    norm_single_load(values, p.h, p.cols0);
-    stream_fill<SLOTS>(rs);  // the ring slot held back, now behind the activation loads
+    if (KIND != kParallelGate) {
+      norm_single_load(values, p.h, p.cols0);
+      stream_fill<SLOTS>(rs);  // the ring slot held back, now behind the activation loads
+    }
     if (p.step != nullptr) {
 #pragma unroll
       for (uint32_t k = 0; k < kNormRegIters; ++k) {
-        values.v[k].x += bf16x2_lo(step.w[k].x);
-        values.v[k].y += bf16x2_hi(step.w[k].x);
-        values.v[k].z += bf16x2_lo(step.w[k].y);
-        values.v[k].w += bf16x2_hi(step.w[k].y);
+        values.v[k].x += bf16x2_lo(other.w[k].x);
+        values.v[k].y += bf16x2_hi(other.w[k].x);
+        values.v[k].z += bf16x2_lo(other.w[k].y);
+        values.v[k].w += bf16x2_hi(other.w[k].y);
       }
     }
     norm_single_finish(x0, values, weights, p.eps, p.cols0, sh.scratch, p.width);

@@ -88,6 +88,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(Pr
   const bool norm_single = p.prologue == kPrologueAddNorm && p.add_b == nullptr && p.add_bias == nullptr &&
                            p.resid_out == nullptr && !(TP && p.gather.world > 1) &&
                            norm_single_eligible(p.add_a, p.norm_weight, p.cols);
+  // What does not depend on the previous kernel comes first: behind the ring's copies it would wait for them (with the
+  // range arithmetic in 32 bits a step of 8 layers of the 8B shapes 768 and 761 us).
+  NormWeightRegs norm_regs;
+  if (norm_single) norm_weights_preload(norm_regs, p.norm_weight, p.cols);
   RowStream rs;
   stream_init(rs, ring, sh.stream, &sh.job, 1);
   // Weights do not depend on the activations: start streaming before the prologue.  Ahead of a
@@ -100,8 +104,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(Pr
   block_row_range(p.rows, unit, blockIdx.x, gridDim.x, &row_begin, &row_end);
   const uint32_t rows_local = row_end - row_begin;
   for (uint32_t r = threadIdx.x; r < rows_local; r += blockDim.x) row_total[r] = 0.0f;
-  NormWeightRegs norm_regs;
-  if (norm_single) norm_weights_preload(norm_regs, p.norm_weight, p.cols);
 
   // Everything above is independent of the previous kernel; its output is read below.
   pdl_wait();

@@ -56,9 +56,10 @@ struct JobDesc {
 // Rows [begin, end) of block `block` out of `blocks`, in units of `unit` rows.
 __host__ __device__ inline void block_row_range(uint32_t rows, uint32_t unit, uint32_t block,
                                                 uint32_t blocks, uint32_t *begin, uint32_t *end) {
-  const uint64_t units = rows / unit;
-  *begin = static_cast<uint32_t>(units * block / blocks) * unit;
-  *end = static_cast<uint32_t>(units * (block + 1) / blocks) * unit;
+  // units * block / blocks without 64-bit divisions, which a launch would wait for before its first copy
+  const uint32_t units = rows / unit, each = units / blocks, rest = units % blocks;
+  *begin = (each * block + rest * block / blocks) * unit;
+  *end = (each * (block + 1u) + rest * (block + 1u) / blocks) * unit;
 }
 __host__ __device__ inline uint32_t max_rows_per_block(uint32_t rows, uint32_t unit, uint32_t blocks) {
   const uint32_t units = rows / unit;

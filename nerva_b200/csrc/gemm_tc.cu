@@ -246,7 +246,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   if (warp == 0) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (elected()) {
       const uint64_t w_policy = l2_evict_first_policy();  // weights are read once
       const uint64_t x_policy = l2_evict_last_policy();   // every block re-reads the activation block
       SegmentWalk walk{run_begin, run_end, part.slices};
@@ -273,7 +273,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     pdl_wait();
-    if (lane == 0) {
+    if (elected()) {
       const uint32_t idesc = instr_desc_bf16(p.n_pad);
       SegmentWalk walk{run_begin, run_end, part.slices};
       Segment seg;
@@ -356,7 +356,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   __syncthreads();
   if (sh.abort != 0u) {
     if (threadIdx.x == 0) drain_copies(sh.full, p.stages);
-    if (warp == 1 && lane == 0) drain_mmas(&sh.drained);
+    if (warp == 1 && elected()) drain_mmas(&sh.drained);
   }
   __syncthreads();
   if (warp == 1) {

@@ -16,9 +16,9 @@
 // columns), and the last one is not hidden: hence eight warps, values without branches and residuals a group ahead
 // (row_epilogue, row_residual).
 //
-// Measured back to back, other weights each time, 2048 tokens (four warps and a branch per value before): 24576 x 4096
-// with SwiGLU 311 us, 1325 TFLOP/s (394), 281 without an epilogue; 4096 x 12288 with residual 158 (178); 6144 x 4096 89 (96);
-// 4096 x 4096 with residual 62 (85).  Loads alone would take 205 us of the first, MMAs alone 275.
+// Measured back to back, other weights each time, 2048 tokens, with four warps and a branch per value, with this epilogue, and
+// with it and issuing threads chosen by elect.sync: 24576 x 4096 with SwiGLU 394, 311, 260 us, 1586 TFLOP/s of the last; 4096 x 12288 with residual
+// 178, 158, 140; 6144 x 4096 96, 89, 71; 4096 x 4096 with residual 85, 62, 52.
 //
 // Roles inside a block (320 threads), as in gemm_tc.cu: warp 0 issues the TMA copies into the block's own ring,
 // warp 1 of the pair's first block issues the MMAs for both (its `full` barriers count the bytes of both blocks),
@@ -145,7 +145,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
   if (warp == 0) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (elected()) {
       const uint64_t w_policy = l2_evict_first_policy();  // a weight tile's readers run together
       const uint64_t x_policy = l2_evict_last_policy();
       bool ok = true, waited = false;
@@ -172,7 +172,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer: the pair's first block ----------------
-    if (rank == 0 && lane == 0) {
+    if (rank == 0 && elected()) {
       const uint32_t idesc = pair_instr_desc(t.tile_tokens);
       // (in front of the loop: a test inside it took 3 % of a 512-token prefill)
       if (p.stamps != nullptr && abortable_wait(&sh.full[0], 0, abort, p.error_word)) stamp_pair(p.stamps, kStampAfterWait, pair, pairs);
@@ -234,7 +234,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   __syncthreads();
   if (sh.abort != 0u && rank == 0) {  // the first block counts the copies of both and issues the MMAs
     if (threadIdx.x == 0) drain_copies(sh.full, p.stages);
-    if (warp == 1 && lane == 0) {
+    if (warp == 1 && elected()) {
       pair_commit(&sh.drained, 1);
       mbar_wait_bounded(&sh.drained, 0);
     }

@@ -330,7 +330,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const uint32_t tiles = sh.first_tile[g.groups];
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elected()) {
       const uint64_t w_policy = l2_evict_first_policy(), x_policy = l2_evict_last_policy();
       uint32_t issued = 0;
       bool ok = true;
@@ -353,7 +353,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elected()) {
       uint32_t consumed = 0, index = 0;
       bool ok = true;
       for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++index) {
@@ -435,7 +435,7 @@ moe_block_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   __syncthreads();
   if (sh.abort != 0u) {
     if (threadIdx.x == 0) drain_copies(sh.full, g.stages);
-    if (warp == 1 && lane == 0) drain_mmas(&sh.drained);
+    if (warp == 1 && elected()) drain_mmas(&sh.drained);
   }
   __syncthreads();
   if (warp == 1) {

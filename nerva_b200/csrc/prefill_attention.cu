@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
         if (!warp_wait(&sh.k_full[st], (j / kStages) & 1u, abort, error_word)) return false;
         if (j >= 2u && !warp_wait(&sh.pv_done[j & 1u], ((j >> 1) & 1u) ^ 1u, abort, error_word)) return false;
         tcgen05_fence_after();
-        if (lane != 0) return true;
+        if (!elected()) return true;
         const uint8_t *k = k_ring + st * kTileBytes;
 #pragma unroll
         for (uint32_t part = 0; part < 2u; ++part) {
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
           clean_values<D>(v_ring + st * kTileBytes, kv_end - first < kKeys ? kv_end - first : kKeys, &sh.taken_out);
         if (!warp_wait(&sh.p_full[j & 1u], (j >> 1) & 1u, abort, error_word)) break;
         tcgen05_fence_after();
-        if (lane == 0) {
+        if (elected()) {
           const uint64_t v = mn_major_sw128_desc(v_ring + st * kTileBytes);
 #pragma unroll
           for (uint32_t part = 0; part < 2u; ++part) {
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   if (sh.abort != 0u) {
     if (threadIdx.x == 0) drain_copies(sh.k_full, kStages);
     if (threadIdx.x == 32) drain_copies(sh.v_full, kStages);
-    if (warp == kMmaWarp && lane == 0) drain_mmas(&sh.drained);
+    if (warp == kMmaWarp && elected()) drain_mmas(&sh.drained);
   }
   __syncthreads();
   if (warp == kMmaWarp) {

@@ -396,6 +396,10 @@ __global__ void gqa_merge_kernel(AttentionParams p) {
   const uint32_t d = p.head_dim, S = p.splits;
   const uint64_t slot0 = (static_cast<uint64_t>(b) * p.heads + head) * S;
   const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
+  if (p.host_error != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
+    const uint32_t error = __ldcg(p.error_word);
+    if (error != 0u) *reinterpret_cast<volatile uint32_t *>(p.host_error) = error;
+  }
   if (tid < 32u) {
     const uint32_t lane = tid;
     float m = -INFINITY;

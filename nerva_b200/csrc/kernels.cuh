@@ -205,6 +205,7 @@ struct AttentionParams {
   float *out_f32;              // [batch][heads*d] optional
   uint16_t *out_bf16;          // optional
   uint32_t *error_word;
+  uint32_t *host_error;        // optional, mapped host memory: the merge launch hands a non-zero error word on to it
   // Row form (launch_attention_rows): sequence b of the batch is row b of a block step; its q
   // (normalised, rotated, fp32, at the start of the row's projection output), cache, page table
   // and context (position + 1) come from rows[b], q / key_pages / value_pages / page_table /

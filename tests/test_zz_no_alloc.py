@@ -105,3 +105,17 @@ def test_static_scratch_attention_rejects_oversize(built_lib):
     with pytest.raises(RuntimeError, match="static scratch too small"):
         ops.gqa_decode_attention_static_scratch(dummy.data_ptr(), dummy.data_ptr(), dummy.data_ptr(),
                                                 dummy.data_ptr(), dummy.data_ptr(), 64, 16, 128, 8, 128)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (32, 8, 128), (4, 4, 48)])
+def test_page_index_outside_the_table_is_reported_and_forgotten(built_lib, heads, kv_heads, head_dim):
+    """The kernels check the index and read page 0 instead; the call after it is a clean one."""
+    q, k, v, table = _inputs(1, 500, heads, kv_heads, head_dim, 7)
+    good = _static_scratch(q, k, v, table, 1, 500, heads, kv_heads, head_dim)
+    bad = table.copy()
+    bad[0, 3] = table.shape[1]
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="page index"):
+            _static_scratch(q, k, v, bad, 1, 500, heads, kv_heads, head_dim)
+    again = _static_scratch(q, k, v, table, 1, 500, heads, kv_heads, head_dim)
+    assert np.array_equal(again, good)

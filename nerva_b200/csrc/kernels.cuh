@@ -151,6 +151,7 @@ bool encode_bf16_map_2d(void *map, const uint16_t *base, uint64_t inner, uint64_
                         uint32_t box_outer);
 cudaError_t configure_gemm_tc_kernel();  // and gemm_wide.cu's
 cudaError_t configure_gemm_wide_kernel();
+uint32_t gemm_wide_waves(uint32_t rows, uint32_t tokens, uint32_t sm_count);  // tiles that the busiest pair of SMs takes
 // launch_gemm_tc takes any number of tokens: above kGemmMaxTokens it is launch_gemm_wide.
 cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);

@@ -797,8 +797,6 @@ cudaError_t enqueue_chunked_prefill(NervaCudaHfDecodeSequenceSession *s, uint32_
       // the last position's residual stream becomes the session's own, where the head expects it
       err = cudaMemcpyAsync(s->h_b, ws.h_b + static_cast<uint64_t>(rows - 1u) * width, width * sizeof(float),
                             cudaMemcpyDeviceToDevice, s->stream);
-      // (a model with sparse layers adds the last sublayer's output in the head: it is in the stream already)
-      if (err == cudaSuccess && s->has_moe) err = cudaMemsetAsync(s->down, 0, width * sizeof(float), s->stream);
     }
     // the wanted positions of this chunk, up to sample_rows of them per head launch
     std::vector<uint32_t> place, row;

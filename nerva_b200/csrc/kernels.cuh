@@ -340,6 +340,7 @@ struct MoeExpertParams {
   const uint16_t *w_router;          // [num_experts][hidden]
   uint32_t num_experts, norm_topk_prob;
   float *resid_out;
+  const float *resid_in;             // optional [hidden]: out_f32 becomes MLP output + resid_in (not with push)
   float *router_logits;              // [num_experts] scratch
   float *x_norm;                     // [hidden] scratch: the normalised row
   uint32_t *expert_ids;              // [top_k] scratch: the routing result

@@ -473,6 +473,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_down_kernel(MoeExpertParam
     __syncthreads();
     for (uint32_t r = row_begin + warp; r < row_end; r += kMoeWarps) {
       float sum = 0.0f, shared = 0.0f;  // of this lane
+      const float resid = p.resid_in != nullptr && m1 == matrices && lane == 0 ? __ldcg(p.resid_in + r) : 0.0f;
       for (uint32_t m = m0; m < m1; ++m) {
         const uint32_t cols = m == 0 ? si : mi;
         const float4 *xa = reinterpret_cast<const float4 *>(x) + (m == 0 ? routed_floats : (m - 1u - routed_from) * mi) / 8u + lane;
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_down_kernel(MoeExpertParam
         for (uint32_t q = 0; q < p.push.world; ++q)
           asm volatile("st.volatile.global.u64 [%0], %1;" ::"l"(p.push.recv[q] + at), "l"(entry) : "memory");
       } else {
-        p.out_f32[r] = sum;
+        p.out_f32[r] = p.resid_in != nullptr ? sum + resid : sum;
       }
     }
     if (m1 >= matrices) break;

@@ -314,6 +314,12 @@ __device__ __forceinline__ void gqa_decode_block(const CUtensorMap *map_k_all, c
       }
     }
     const uint64_t slot = (static_cast<uint64_t>(b) * p.heads + kvh * G + gg) * p.splits + split;
+    if (ROWS && p.splits == 1u) {  // the only span: what the merge would make of it, without the launch
+      const float y = a * (l > 0.0f ? 1.0f / l : 0.0f);
+      if (p.out_f32 != nullptr) p.out_f32[slot * D + d] = y;
+      if (p.out_bf16 != nullptr) p.out_bf16[slot * D + d] = f32_to_bf16_bits(y);
+      continue;
+    }
     p.partial_acc[slot * D + d] = a;
     if (d == 0) {
       p.partial_m[slot] = m;
@@ -558,7 +564,7 @@ cudaError_t launch_attention_rows(cudaStream_t stream, const AttentionParams &p,
   else
     err = launch_with_pdl(gqa_decode_rows_kernel<64>, grid, dim3(kAttnWarps * 32), paged_smem_bytes<64>(), stream, true,
                           maps, p);
-  if (err != cudaSuccess) return err;
+  if (err != cudaSuccess || p.splits == 1u) return err;
   return launch_with_pdl(gqa_merge_kernel, dim3(p.heads, p.batch), merge_block(p.head_dim, p.splits), 0, stream, true, p);
 }
 

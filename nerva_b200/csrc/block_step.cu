@@ -476,7 +476,7 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       ap.rows = ws.attn_rows;
       ap.layer = l;
       err = launch_attention_rows(b.stream, ap, b.k_maps.data(), b.v_maps.data(), static_cast<uint32_t>(b.k_maps.size()));
-      n += 2;
+      n += ap.splits == 1u ? 1 : 2;
       if (err != cudaSuccess) break;
     } else {
     FusedAttentionParams fp{};

@@ -169,7 +169,7 @@ struct WarpRing {
     slot_bytes = bytes;
     base = ring + warp * slots * slot_bytes;
     bars = all_bars + warp * kMaxSlots;
-    if ((threadIdx.x & 31u) == 0) {
+    if (elected()) {
       for (uint32_t i = 0; i < slots; ++i) mbar_init(&bars[i], 1);
       mbar_init_fence();
     }
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_gate_up_kernel(MoeExpertPa
 
   auto issue = [&](PairCursor &c, uint64_t up_offset) {
     const uint32_t bytes = hidden - c.col < kPieceCols ? (hidden - c.col) * 2u : kPieceBytes;
-    if (lane == 0) {
+    if (elected()) {
       uint64_t *bar = &ring.bars[ring.issue_slot];
       uint8_t *dst = ring.base + ring.issue_slot * ring.slot_bytes;
       const uint16_t *src = c.gate + c.col;
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_down_kernel(MoeExpertParam
     while (ring.room() && row < row_end && matrix < known) {
       const uint32_t cols = matrix == 0 ? si : mi;
       const uint32_t bytes = cols - col < kPieceCols ? (cols - col) * 2u : kPieceBytes;
-      if (lane == 0) {
+      if (elected()) {
         const uint16_t *src = matrix == 0 ? p.w_shared_down + static_cast<uint64_t>(row) * si
                                           : p.w_expert_down + (static_cast<uint64_t>(sh.ids[matrix - 1u]) * p.hidden + row) * mi;
         uint64_t *bar = &ring.bars[ring.issue_slot];

@@ -171,7 +171,7 @@ __device__ inline void stream_init(RowStream &rs, uint8_t *ring_base, StreamShar
     rs.issue = warp_job(jobs[0]);
     rs.issue_cursor = cursor_at_start(rs.issue);
   }
-  if ((threadIdx.x & 31u) == 0) {
+  if (elected()) {
     for (uint32_t s = 0; s < SLOTS; ++s) mbar_init(&rs.bars[s], 1);
     mbar_init_fence();
   }
@@ -194,7 +194,7 @@ __device__ __forceinline__ void stream_fill(RowStream &rs, uint32_t depth = SLOT
     uint32_t pos, row_end, pair;
     const uint32_t len = cursor_next(rs.issue, rs.issue_cursor, &pos, &row_end, &pair);
     const uint32_t slot = rs.issued % SLOTS;
-    if ((threadIdx.x & 31u) == 0) {
+    if (elected()) {
       const bool both = 2u * pair + 1u < rs.issue.rows;
       const uint8_t *src = rs.issue.base + pos + static_cast<uint64_t>(pair) * rs.issue.row_bytes;
       mbar_arrive_expect_tx(&rs.bars[slot], both ? 2u * len : len);

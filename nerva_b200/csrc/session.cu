@@ -683,9 +683,10 @@ cudaError_t enqueue_step(Session *s, uint32_t splits, uint32_t sample, uint64_t 
     if (sample == 2) return cudaErrorNotSupported;  // the one-kernel engine only has the arg-max sampler
     return enqueue_step_kernel(s, splits, sample);
   }
-  // Single-GPU models without an O bias: O and down (of sparse layers too: a step of the 64-expert model 377 and 367 us, latent 437 and 425) add the residual stream to their
+  // Single-GPU models without an O bias: O and down add the residual stream to their
   // own output (row by row, by the row's owner), so the next prologue reads one summed vector.
-  // The sum is the same two-operand add the prologue would have done.
+  // The sum is the same two-operand add the prologue would have done.  (Sparse layers' down too: a step of
+  // 6 layers of 64 experts 377 and 367 us, with latent attention 437 and 425.)
   bool fused_resid = !tp && !ep_on;
   for (const LayerLayout &L : s->layout.layers) fused_resid = fused_resid && arena_at(s, L.o_bias) == nullptr;
   profile_mark(s, prof, kBucketEmbed);
@@ -2614,12 +2615,26 @@ extern "C" int nerva_b200_session_append(Session *s, const uint32_t *tokens, uin
   s->started = false;
   s->prompt_count = end;
   if (chunked) {
-    const WantedLogits wanted{want, want_count, logits};
+    bool last_logits = false;
+    const WantedLogits wanted{want, want_count, logits, &last_logits};
     if (err == cudaSuccess) err = enqueue_chunked_prefill(s, begin, end, wanted, nullptr);
     const uint32_t last = end - 1u;
     if (err == cudaSuccess)
       err = cudaMemcpyAsync(s->device_cursor, &last, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
-    if (err == cudaSuccess) err = enqueue_step(s, splits_for(s, end), s->sample_kind, nullptr, nullptr, true);
+    if (last_logits) {
+      // the last token's logits were wanted and stand in s->logits: sampled from, without another pass over the head (40 tokens
+      // through 8 layers of the 8B shapes 1.30 and 1.12 ms)
+      const BlockWorkspace &ws = s->weights->block_ws;
+      if (err == cudaSuccess && s->sample_kind == 2u) {
+        err = launch_sample_general(s->stream, step_state(s), s->logits, s->device_sampler, s->use_pdl);
+      } else if (err == cudaSuccess) {
+        err = launch_argmax_partials(s->stream, s->logits, s->dims.vocab, 1, kBlockArgmaxChunks, ws.best_value, ws.best_index, s->use_pdl);
+        if (err == cudaSuccess)
+          err = launch_sample_greedy(s->stream, step_state(s), ws.best_value, ws.best_index, kBlockArgmaxChunks, s->sample_kind, s->use_pdl, nullptr);
+      }
+    } else if (err == cudaSuccess) {
+      err = enqueue_step(s, splits_for(s, end), s->sample_kind, nullptr, nullptr, true);
+    }
   } else {
     for (uint32_t i = 0; err == cudaSuccess && i < count; ++i) {
       bool sampled = i + 1u == count;

@@ -222,3 +222,24 @@ def test_file_backed_upload_reports_what_went_wrong(built_lib, tiny_checkpoint, 
         f.truncate(1 << 20)
     short = CudaHfDecodeSequenceSession(tiny_checkpoint, 64, weight_file=path)
     assert short.status == SmokeStatus.FAILED and "short read" in short.error
+
+
+@pytest.mark.parametrize("count,places", [(2, [1]), (40, [39]), (40, [39, 3, 39]), (70, list(range(70)))])
+def test_append_samples_from_the_last_tokens_wanted_logits(built_lib, tiny_checkpoint, count, places):
+    """With the last token's logits wanted there is no second pass over the head: the session holds those very logits, and
+    the token sampled behind them is their arg-max; without them the same token comes from the session's own pass."""
+    tokens = synth.uniform_u32(3, synth.T_PROMPT, count, synth.TINY_QWEN3.vocab)
+    s = CudaHfDecodeSequenceSession(tiny_checkpoint, 128)
+    assert s.status == SmokeStatus.OK, s.error
+    logits = s.append(tokens, want=places, reset=True)
+    last = logits[places.index(count - 1)]
+    assert np.array_equal(s.read_logits(), last)
+    first = CudaHfDecodeSequenceLoop(s).advance(2).tokens
+    assert first[0] == int(last.argmax())
+    s.append(tokens, reset=True)
+    own = s.read_logits()
+    assert np.abs(own - last).max() <= LOGIT_ATOL
+    top = np.sort(last)[-2:]
+    if top[1] - top[0] > 2 * LOGIT_ATOL:
+        assert CudaHfDecodeSequenceLoop(s).advance(2).tokens == first
+    s.destroy()

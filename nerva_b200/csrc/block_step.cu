@@ -64,18 +64,26 @@ __global__ void block_embed_kernel(const BlockTokenRow *rows, const uint16_t *em
 // summation order of the single-token prologue (step_device.cuh norm_single_*), so a token
 // normalises to the same bits whichever path carries it.  row_index (optional): block i takes row
 // row_index[i] of h.
+// ITERS: float4 per thread, the fewest that hold a row: with registers for 8192 columns three blocks fit an SM where six do
+// (2048 rows of 4096: 15.4 and 9.5 us, cold).
+template <uint32_t ITERS>
 __global__ void __launch_bounds__(kNormThreads) block_norm_kernel(const float *h, const uint16_t *w, float eps,
                                                                   uint32_t cols, uint16_t *x, uint32_t x_stride,
                                                                   const uint32_t *row_index) {
   __shared__ float scratch[40];
   pdl_trigger();
-  NormWeightRegs weights;
+  NormWeights<ITERS> weights;
   norm_weights_preload(weights, w, cols);
   pdl_wait();
-  NormValueRegs values;
+  NormValues<ITERS> values;
   const uint32_t source = row_index != nullptr ? row_index[blockIdx.x] : blockIdx.x;
   norm_single_load(values, h + static_cast<uint64_t>(source) * cols, cols);
   norm_single_finish(x + static_cast<uint64_t>(blockIdx.x) * x_stride, values, weights, eps, cols, scratch);
+}
+
+using BlockNorm = void (*)(const float *, const uint16_t *, float, uint32_t, uint16_t *, uint32_t, const uint32_t *);
+BlockNorm block_norm(uint32_t cols) {
+  return cols <= 8u * kNormThreads ? block_norm_kernel<2> : cols <= 16u * kNormThreads ? block_norm_kernel<4> : block_norm_kernel<kNormRegIters>;
 }
 
 // K (k-norm + RoPE) and V of every row of the block, rounded to bf16, into the row's page: the same functions, in the
@@ -109,8 +117,21 @@ block_kv_publish_kernel(const FusedAttentionRow *rows, uint32_t layer, uint32_t 
   const uint32_t page = r.page_table[r.position / NERVA_KV_CACHE_BLOCK_TOKENS];
   const bool cached = page < r.page_count;
   if (!cached) report_error(r.error_word, kErrPageOutOfRange);
-  for (uint32_t unit = blockIdx.x * kPublishWarps + (threadIdx.x >> 5); unit < kv_heads + query_heads;
-       unit += gridDim.x * kPublishWarps) {
+  // a unit's values (of a KV head, its K) are asked for while the one before it is at work: a round trip to L2 each, five of them
+  // for 32 + 8 heads (2048 rows: 24.6 us in turn, 22.1)
+  const uint32_t first = blockIdx.x * kPublishWarps + (threadIdx.x >> 5), stride = gridDim.x * kPublishWarps;
+  auto ask = [&](float (&v)[PER], uint32_t unit) {
+    const float *src = unit >= kv_heads ? r.qkv + (unit - kv_heads) * D : r.qkv + attention_hidden + unit * D;
+#pragma unroll
+    for (uint32_t k = 0; k < PER; ++k) v[k] = unit < kv_heads + query_heads ? __ldcg(src + lane + 32u * k) : 0.0f;
+  };
+  float ahead[PER];
+  ask(ahead, first);
+  for (uint32_t unit = first; unit < kv_heads + query_heads; unit += stride) {
+    float now[PER];
+#pragma unroll
+    for (uint32_t k = 0; k < PER; ++k) now[k] = ahead[k];
+    ask(ahead, unit + stride);
     if (unit >= kv_heads) {
       const uint32_t h = unit - kv_heads;
       float *q = const_cast<float *>(r.qkv) + h * D;  // the row's projection output is scratch of the block step
@@ -118,7 +139,7 @@ block_kv_publish_kernel(const FusedAttentionRow *rows, uint32_t layer, uint32_t 
 #pragma unroll
       for (uint32_t k = 0; k < PER; ++k) {
         const uint32_t e = lane + 32u * k;
-        qn[k] = __ldcg(q + e);
+        qn[k] = now[k];
         if (q_bias != nullptr) qn[k] += bf16_bits_to_f32(q_bias[h * D + e]);
       }
       head_norm_rope_pre<PER>(qn, q_norm != nullptr, q_norm_w, eps, rope);
@@ -131,7 +152,7 @@ block_kv_publish_kernel(const FusedAttentionRow *rows, uint32_t layer, uint32_t 
 #pragma unroll
     for (uint32_t k = 0; k < PER; ++k) {
       const uint32_t e = lane + 32u * k;
-      kn[k] = __ldcg(r.qkv + attention_hidden + kvh * D + e);
+      kn[k] = now[k];
       vn[k] = __ldcg(r.qkv + attention_hidden + kv_hidden + kvh * D + e);
       if (k_bias != nullptr) kn[k] += bf16_bits_to_f32(k_bias[kvh * D + e]);
       if (v_bias != nullptr) vn[k] += bf16_bits_to_f32(v_bias[kvh * D + e]);
@@ -390,7 +411,7 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
   for (uint32_t l = 0; err == cudaSuccess && l < d.layers; ++l) {
     const LayerLayout &L = s->layout.layers[l];
     // attention half
-    err = launch_with_pdl(block_norm_kernel, dim3(b.rows), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_b,
+    err = launch_with_pdl(block_norm(d.hidden), dim3(b.rows), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_b,
                           arena_at(s, L.rms_attn), s->rms_eps, d.hidden, ws.x_bf16, d.hidden, nullptr);
     if (err == cudaSuccess)
       err = block_gemm(b, s->weights->qkv_packed + static_cast<uint64_t>(l) * qkv_rows * d.hidden, qkv_rows, d.hidden,
@@ -516,7 +537,7 @@ cudaError_t enqueue_block_layers(const BlockPlan &b, uint64_t *launches) {
       continue;
     }
     if (err == cudaSuccess)
-      err = launch_with_pdl(block_norm_kernel, dim3(b.rows), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_a,
+      err = launch_with_pdl(block_norm(d.hidden), dim3(b.rows), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_a,
                             arena_at(s, L.rms_mlp), s->rms_eps, d.hidden, ws.x_bf16, d.hidden, nullptr);
     if (err == cudaSuccess)
       err = block_gemm(b, s->weights->gate_up_packed + gate_up_packed_offset(s, l),
@@ -540,7 +561,7 @@ cudaError_t enqueue_block_head(const BlockPlan &b, uint32_t count, const uint32_
   if (s->parallel) return enqueue_parallel_block_head(s, b.stream, count, row_index, launches);
   BlockPlan head = b;
   head.rows = count;
-  cudaError_t err = launch_with_pdl(block_norm_kernel, dim3(count), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_b,
+  cudaError_t err = launch_with_pdl(block_norm(d.hidden), dim3(count), dim3(kNormThreads), 0, b.stream, b.pdl, ws.h_b,
                                     arena_at(s, s->layout.final_norm), s->rms_eps, d.hidden, ws.x_bf16, d.hidden,
                                     row_index);
   if (err == cudaSuccess)

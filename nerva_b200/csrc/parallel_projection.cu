@@ -342,6 +342,14 @@ __device__ __forceinline__ float2 load_pair(const uint16_t *x) {
 }
 __device__ __forceinline__ void store_act(float *out, float v) { *out = v; }
 __device__ __forceinline__ void store_act(uint16_t *out, float v) { *out = f32_to_bf16_bits(v); }
+// Four consecutive values, the first at a multiple of four.
+__device__ __forceinline__ void store_act4(float *out, float a, float b, float c, float d) {
+  *reinterpret_cast<float4 *>(out) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void store_act4(uint16_t *out, float a, float b, float c, float d) {
+  *reinterpret_cast<uint2 *>(out) = make_uint2(f32_to_bf16_bits(a) | static_cast<uint32_t>(f32_to_bf16_bits(b)) << 16,
+                                               f32_to_bf16_bits(c) | static_cast<uint32_t>(f32_to_bf16_bits(d)) << 16);
+}
 
 template <class X>
 __device__ __forceinline__ void plain_dots(const uint16_t *w, const X *x, uint32_t cols, uint32_t tokens,
@@ -469,10 +477,8 @@ __device__ __forceinline__ void norm_in_registers(const StreamNormParams &p, flo
     const uint32_t i = threadIdx.x + k * kNormThreads;
     if (i < vecs) {
       const uint2 w = reinterpret_cast<const uint2 *>(p.norm)[i];
-      store_act(out + 4u * i, (h.v[k].x - m.mean) * m.scale * bf16x2_lo(w.x));
-      store_act(out + 4u * i + 1u, (h.v[k].y - m.mean) * m.scale * bf16x2_hi(w.x));
-      store_act(out + 4u * i + 2u, (h.v[k].z - m.mean) * m.scale * bf16x2_lo(w.y));
-      store_act(out + 4u * i + 3u, (h.v[k].w - m.mean) * m.scale * bf16x2_hi(w.y));
+      store_act4(out + 4u * i, (h.v[k].x - m.mean) * m.scale * bf16x2_lo(w.x), (h.v[k].y - m.mean) * m.scale * bf16x2_hi(w.x),
+                 (h.v[k].z - m.mean) * m.scale * bf16x2_lo(w.y), (h.v[k].w - m.mean) * m.scale * bf16x2_hi(w.y));
     }
   }
 }
@@ -521,12 +527,8 @@ __global__ void __launch_bounds__(kNormThreads) stream_norm_kernel(StreamNormPar
     for (uint32_t i = threadIdx.x * 4u; i < p.padded; i += kNormThreads * 4u) {
       const float4 v = *reinterpret_cast<const float4 *>(row + i);
       const float4 f = *reinterpret_cast<const float4 *>(first + i);
-      const float a[4] = {v.x, v.y, v.z, v.w}, b[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-      for (uint32_t j = 0; j < 4u; ++j) {
-        store_act(out + i + j, a[j]);
-        store_act(out + p.padded + i + j, b[j]);
-      }
+      store_act4(out + i, v.x, v.y, v.z, v.w);
+      store_act4(out + p.padded + i, f.x, f.y, f.z, f.w);
     }
     return;
   }
@@ -535,10 +537,8 @@ __global__ void __launch_bounds__(kNormThreads) stream_norm_kernel(StreamNormPar
   for (uint32_t i = threadIdx.x * 4u; i < p.padded; i += kNormThreads * 4u) {
     const float4 v = *reinterpret_cast<const float4 *>(row + i);
     const uint2 w = *reinterpret_cast<const uint2 *>(p.norm + i);
-    store_act(out + i, (v.x - m.mean) * m.scale * bf16x2_lo(w.x));
-    store_act(out + i + 1u, (v.y - m.mean) * m.scale * bf16x2_hi(w.x));
-    store_act(out + i + 2u, (v.z - m.mean) * m.scale * bf16x2_lo(w.y));
-    store_act(out + i + 3u, (v.w - m.mean) * m.scale * bf16x2_hi(w.y));
+    store_act4(out + i, (v.x - m.mean) * m.scale * bf16x2_lo(w.x), (v.y - m.mean) * m.scale * bf16x2_hi(w.x),
+               (v.z - m.mean) * m.scale * bf16x2_lo(w.y), (v.w - m.mean) * m.scale * bf16x2_hi(w.y));
   }
 }
 

@@ -9,11 +9,11 @@
 // Queries and probabilities are fp32 values; each enters as a bf16 rounding and its remainder, two MMAs into the same
 // accumulator, so a product loses only the rounding of the cached row (the contract of the other attention kernels).
 //
-// What bounds it: the softmax.  The MMAs of a tile are 4 x 512 cycles (two parts of Q, two of P), but a tile takes about
-// 7300 (2048 tokens, 32 heads: 4352 tiles on 148 SMs in 122 us), because a tile's chain of scores out of tensor memory,
-// maximum, 128 exponentials a thread, two packs and the stores back runs by itself: the tensor pipe is active 31 % of the
-// time.  S has two buffers: S(j+1) is computed while the
-// softmax works on S(j).  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since
+// What bounds it: the MMAs, 4 x 512 cycles a tile (two parts of Q, two of P), and the hand-overs between them.  With probes a
+// tile of a long walk takes 3500 cycles, 2090 of them issuing MMAs (2680 of 3920 while a lane's number chose the issuing
+// thread); the softmax warps wait 64 % of the time: a tile of theirs is 120 cycles of loads, 320 for the maximum, 1700 for 128
+// exponentials a thread, their sums and two packs.  S has two buffers: S(j+1) is computed while the
+// softmax works on S(j), but S(j+2) goes where P(j) is and waits for its PV.  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since
 // the reference it uses (the probabilities stay below 2^8, the sums exact to fp32): after the first tiles that almost
 // never happens.
 // One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), and two

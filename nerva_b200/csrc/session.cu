@@ -2623,7 +2623,7 @@ extern "C" int nerva_b200_session_append(Session *s, const uint32_t *tokens, uin
       err = cudaMemcpyAsync(s->device_cursor, &last, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
     if (last_logits) {
       // the last token's logits were wanted and stand in s->logits: sampled from, without another pass over the head (40 tokens
-      // through 8 layers of the 8B shapes 1.30 and 1.12 ms)
+      // through 8 layers of the 8B shapes 1.30 and 1.13 ms)
       const BlockWorkspace &ws = s->weights->block_ws;
       if (err == cudaSuccess && s->sample_kind == 2u) {
         err = launch_sample_general(s->stream, step_state(s), s->logits, s->device_sampler, s->use_pdl);

@@ -91,17 +91,21 @@ __device__ __forceinline__ void add_norm_to_smem(uint16_t *x, const float *a, co
 // added its output to it): x = bf16(a * rsqrt(mean(a^2) + eps) * w).  The norm weights do not
 // depend on the previous kernel, so norm_weights_preload fetches them before the dependency
 // wait and the wait is followed by one 16-byte load per thread and iteration.
-struct NormWeightRegs {
-  uint2 w[kNormRegIters];
+// N: float4 per thread; a kernel that knows its rows to be shorter takes fewer registers than kNormRegIters want.
+template <uint32_t N>
+struct NormWeights {
+  uint2 w[N];
 };
+using NormWeightRegs = NormWeights<kNormRegIters>;
 __device__ __forceinline__ bool norm_single_eligible(const float *a, const uint16_t *w, uint32_t cols) {
   return cols % 4u == 0 && cols / 4u <= kNormRegIters * blockDim.x && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 &&
          (reinterpret_cast<uintptr_t>(w) & 7u) == 0;
 }
-__device__ __forceinline__ void norm_weights_preload(NormWeightRegs &regs, const uint16_t *w, uint32_t cols) {
+template <uint32_t N>
+__device__ __forceinline__ void norm_weights_preload(NormWeights<N> &regs, const uint16_t *w, uint32_t cols) {
   const uint32_t vecs = cols / 4u;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t i = threadIdx.x + k * blockDim.x;
     regs.w[k] = i < vecs ? reinterpret_cast<const uint2 *>(w)[i] : make_uint2(0u, 0u);
   }
@@ -109,25 +113,29 @@ __device__ __forceinline__ void norm_weights_preload(NormWeightRegs &regs, const
 // Two halves, so that the caller can issue other memory traffic (the rest of its weight ring)
 // behind the activation loads instead of in front of them: norm_single_load issues the loads,
 // norm_single_finish consumes them.
-struct NormValueRegs {
-  float4 v[kNormRegIters];
+template <uint32_t N>
+struct NormValues {
+  float4 v[N];
 };
-__device__ __forceinline__ void norm_single_load(NormValueRegs &r, const float *a, uint32_t cols) {
+using NormValueRegs = NormValues<kNormRegIters>;
+template <uint32_t N>
+__device__ __forceinline__ void norm_single_load(NormValues<N> &r, const float *a, uint32_t cols) {
   const uint32_t vecs = cols / 4u;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t i = threadIdx.x + k * blockDim.x;
     r.v[k] = i < vecs ? __ldcg(reinterpret_cast<const float4 *>(a) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 // mean_count: elements the mean is taken over, when the vector is padded with zeros up to cols (0: cols).
-__device__ __forceinline__ void norm_single_finish(uint16_t *x, const NormValueRegs &loaded, const NormWeightRegs &regs,
+template <uint32_t N>
+__device__ __forceinline__ void norm_single_finish(uint16_t *x, const NormValues<N> &loaded, const NormWeights<N> &regs,
                                                    float eps, uint32_t cols, float *scratch, uint32_t mean_count = 0) {
   const uint32_t vecs = cols / 4u;
   const float4 *r = loaded.v;
   float sumsq = 0.0f;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t i = threadIdx.x + k * blockDim.x;
     if (i < vecs) {
       const float4 v = r[k];
@@ -137,7 +145,7 @@ __device__ __forceinline__ void norm_single_finish(uint16_t *x, const NormValueR
   const float total = block_sum(sumsq, scratch);
   const float scale = rsqrtf(total / static_cast<float>(mean_count != 0 ? mean_count : cols) + eps);
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t i = threadIdx.x + k * blockDim.x;
     if (i < vecs) {
       const float4 v = r[k];

@@ -447,17 +447,18 @@ __device__ __forceinline__ NormMoments row_moments(const float *row, const Strea
 }
 
 // A row's pending output and norm with every value read once: the sandwich prologue for a block of rows.
-template <class X>
+// N: float4 per thread.
+template <class X, uint32_t N>
 __device__ __forceinline__ void norm_in_registers(const StreamNormParams &p, float *row, uint32_t source) {
   __shared__ float scratch[2u * kMomentsScratch];
   const uint32_t vecs = p.padded / 4u;
-  NormValueRegs h, y;
+  NormValues<N> h, y;
   norm_single_load(h, row, p.padded);
   if (p.pending != nullptr) {
     norm_single_load(y, p.pending + static_cast<uint64_t>(source) * p.padded, p.padded);
     const NormMoments m = norm_moments(y.v, p.width, p.layer_norm, p.eps, scratch);
 #pragma unroll
-    for (uint32_t k = 0; k < kNormRegIters; ++k) {
+    for (uint32_t k = 0; k < N; ++k) {
       const uint32_t i = threadIdx.x + k * kNormThreads;
       if (i < vecs) {
         const uint2 w = reinterpret_cast<const uint2 *>(p.after)[i];
@@ -473,7 +474,7 @@ __device__ __forceinline__ void norm_in_registers(const StreamNormParams &p, flo
   const NormMoments m = norm_moments(h.v, p.width, p.layer_norm, p.eps, scratch + kMomentsScratch);
   X *out = reinterpret_cast<X *>(p.x) + static_cast<uint64_t>(blockIdx.x) * p.padded;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t i = threadIdx.x + k * kNormThreads;
     if (i < vecs) {
       const uint2 w = reinterpret_cast<const uint2 *>(p.norm)[i];
@@ -483,17 +484,48 @@ __device__ __forceinline__ void norm_in_registers(const StreamNormParams &p, flo
   }
 }
 
-// One block per row.
-template <class X>
+// A row's RMS norm with every value read once, in the order of row_moments.
+template <class X, uint32_t N>
+__device__ __forceinline__ void rms_in_registers(const StreamNormParams &p, const float *row, float *scratch) {
+  const uint32_t vecs = p.padded / 4u;
+  NormValues<N> h;
+  NormWeights<N> w;
+  norm_single_load(h, row, p.padded);
+  norm_weights_preload(w, p.norm, p.padded);
+  float sumsq = 0.0f;
+#pragma unroll
+  for (uint32_t k = 0; k < N; ++k)
+    sumsq += h.v[k].x * h.v[k].x + h.v[k].y * h.v[k].y + h.v[k].z * h.v[k].z + h.v[k].w * h.v[k].w;
+  const float scale = 1.0f / sqrtf(block_sum(sumsq, scratch) / static_cast<float>(p.width) + p.eps);
+  X *out = reinterpret_cast<X *>(p.x) + static_cast<uint64_t>(blockIdx.x) * p.padded;
+#pragma unroll
+  for (uint32_t k = 0; k < N; ++k) {
+    const uint32_t i = threadIdx.x + k * kNormThreads;
+    if (i < vecs)
+      store_act4(out + 4u * i, h.v[k].x * scale * bf16x2_lo(w.w[k].x), h.v[k].y * scale * bf16x2_hi(w.w[k].x),
+                 h.v[k].z * scale * bf16x2_lo(w.w[k].y), h.v[k].w * scale * bf16x2_hi(w.w[k].y));
+  }
+}
+
+// One block per row.  N: float4 per thread of the rows that fit registers, the fewest: with room for 8192 columns three blocks
+// of 256 threads fit an SM (2048 rows of 2048 columns, cold: layer norm of a pending output and of the sum 26.3 and 16.6 us, RMS
+// norm, its values from L1 twice, 15.9 and 8.6).
+template <class X, uint32_t N>
 __global__ void __launch_bounds__(kNormThreads) stream_norm_kernel(StreamNormParams p) {
   __shared__ float scratch[40];
   pdl_trigger();
   pdl_wait();
   const uint32_t source = p.row_index != nullptr ? p.row_index[blockIdx.x] : blockIdx.x;
   float *row = p.h + static_cast<uint64_t>(source) * p.padded;
-  if (p.layer_norm != 0 && p.step == nullptr && p.first == nullptr && p.padded <= 4u * kNormRegIters * kNormThreads) {
-    norm_in_registers<X>(p, row, source);
-    return;
+  if (p.step == nullptr && p.first == nullptr && p.padded <= 4u * N * kNormThreads) {
+    if (p.layer_norm != 0) {
+      norm_in_registers<X, N>(p, row, source);
+      return;
+    }
+    if (p.pending == nullptr && p.x != nullptr) {
+      rms_in_registers<X, N>(p, row, scratch);
+      return;
+    }
   }
   if (p.step != nullptr) {
     for (uint32_t i = threadIdx.x * 4u; i < p.padded; i += kNormThreads * 4u) {
@@ -625,8 +657,13 @@ cudaError_t launch_parallel_projection_plain(cudaStream_t stream, uint32_t kind,
 cudaError_t launch_stream_norm(cudaStream_t stream, const StreamNormParams &p, bool f32, uint32_t rows, bool pdl) {
   if (rows == 0 || p.padded % 4u != 0 || (p.row_index != nullptr && (p.step != nullptr || p.pending != nullptr)))
     return cudaErrorInvalidValue;
-  return launch_with_pdl(f32 ? stream_norm_kernel<float> : stream_norm_kernel<uint16_t>, dim3(rows), dim3(kNormThreads), 0,
-                         stream, pdl, p);
+  const bool two = p.padded <= 8u * kNormThreads, four = p.padded <= 16u * kNormThreads;
+  void (*kernel)(StreamNormParams);
+  if (f32)
+    kernel = two ? stream_norm_kernel<float, 2> : four ? stream_norm_kernel<float, 4> : stream_norm_kernel<float, kNormRegIters>;
+  else
+    kernel = two ? stream_norm_kernel<uint16_t, 2> : four ? stream_norm_kernel<uint16_t, 4> : stream_norm_kernel<uint16_t, kNormRegIters>;
+  return launch_with_pdl(kernel, dim3(rows), dim3(kNormThreads), 0, stream, pdl, p);
 }
 
 }  // namespace nb

@@ -168,13 +168,14 @@ struct NormMoments {
   float mean, scale;
 };
 constexpr uint32_t kMomentsScratch = 3u * 32u;
-__device__ __forceinline__ NormMoments norm_moments(const float4 (&v)[kNormRegIters], uint32_t width, uint32_t layer_norm,
+template <uint32_t N>
+__device__ __forceinline__ NormMoments norm_moments(const float4 (&v)[N], uint32_t width, uint32_t layer_norm,
                                                     float eps, float *scratch) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   float sum = 0.0f;
   uint32_t count = 0;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t first = 4u * (threadIdx.x + k * blockDim.x);
     sum += (v[k].x + v[k].y) + (v[k].z + v[k].w);
     count += first >= width ? 0u : (width - first < 4u ? width - first : 4u);
@@ -183,7 +184,7 @@ __device__ __forceinline__ NormMoments norm_moments(const float4 (&v)[kNormRegIt
   const float mean_w = layer_norm != 0 && n > 0.0f ? warp_sum(sum) / n : 0.0f;
   float square = 0.0f;
 #pragma unroll
-  for (uint32_t k = 0; k < kNormRegIters; ++k) {
+  for (uint32_t k = 0; k < N; ++k) {
     const uint32_t first = 4u * (threadIdx.x + k * blockDim.x);
     const float d[4] = {v[k].x - mean_w, v[k].y - mean_w, v[k].z - mean_w, v[k].w - mean_w};
 #pragma unroll

@@ -198,7 +198,7 @@ __device__ __forceinline__ void put(uint16_t *dst, float v) { *dst = f32_to_bf16
 __device__ __forceinline__ float get(const float *src) { return __ldcg(src); }
 __device__ __forceinline__ float get(const uint16_t *src) { return bf16_bits_to_f32(__ldcg(src)); }
 
-constexpr uint32_t kConvThreads = 128, kConvRows = 16;
+constexpr uint32_t kConvThreads = 128, kConvRows = 16, kConvBatch = 8;
 
 // Channel of column j of a convolved row; channels(): padding.
 __device__ __forceinline__ uint32_t padded_channel(const StateSpaceShape &s, uint32_t j) {
@@ -248,14 +248,24 @@ __global__ void __launch_bounds__(kConvThreads) state_space_conv_kernel(StateSpa
       u[k - 1u] = row0 >= k ? __ldcg(in + static_cast<uint64_t>(row0 - k) * p.in_stride)
                             : __ldcg(history + static_cast<uint64_t>((base + row0 - k) % s.taps) * channels);
   }
-  for (uint32_t r = row0; r < row_end; ++r) {
+  // a batch of rows is asked for before the first store, behind which the compiler keeps later loads: a round trip each
+  // (2048 rows of 6144 channels, cold: 50.3 us one by one, 30.2)
+  for (uint32_t r = row0; r < row_end; r += kConvBatch) {
+    float next[kConvBatch];
 #pragma unroll
-    for (uint32_t k = TAPS - 1u; k > 0; --k) u[k] = u[k - 1u];
-    u[0] = __ldcg(in + static_cast<uint64_t>(r) * p.in_stride);
-    float v = bias;
+    for (uint32_t q = 0; q < kConvBatch; ++q)
+      next[q] = r + q < row_end ? __ldcg(in + static_cast<uint64_t>(r + q) * p.in_stride) : 0.0f;
 #pragma unroll
-    for (uint32_t k = 0; k < TAPS; ++k) v = fmaf(w[k], u[k], v);
-    put(out + static_cast<uint64_t>(r) * width, silu(v));
+    for (uint32_t q = 0; q < kConvBatch; ++q) {
+      if (r + q >= row_end) break;
+#pragma unroll
+      for (uint32_t k = TAPS - 1u; k > 0; --k) u[k] = u[k - 1u];
+      u[0] = next[q];
+      float v = bias;
+#pragma unroll
+      for (uint32_t k = 0; k < TAPS; ++k) v = fmaf(w[k], u[k], v);
+      put(out + static_cast<uint64_t>(r + q) * width, silu(v));
+    }
   }
 }
 

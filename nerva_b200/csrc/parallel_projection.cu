@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
   RowStream rs;
   stream_init<SLOTS>(rs, ring, sh.first, sh.jobs, second ? 2u : 1u);
   // ahead of a norm prologue one slot is held back: the activation loads would queue behind a whole ring
-  stream_fill<SLOTS>(rs, KIND == kParallelOut || KIND == kParallelGate ? SLOTS : SLOTS - 1u);
+  stream_fill<SLOTS, kCompact>(rs, KIND == kParallelOut || KIND == kParallelGate ? SLOTS : SLOTS - 1u);
 
   uint32_t begin0, end0, begin1 = 0, end1 = 0;
   block_row_range(rows_all, unit, blockIdx.x, gridDim.x, &begin0, &end0);
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
   for (uint32_t r = threadIdx.x; r < rows0 + rows1; r += blockDim.x) total0[r] = 0.0f;
 
   float resid_first = 0.0f;
-  auto fill = [&]() { stream_fill<SLOTS>(rs); };  // the ring slot held back, behind the activation loads
+  auto fill = [&]() { stream_fill<SLOTS, kCompact>(rs); };  // the ring slot held back, behind the activation loads
   if (sandwich_prologue(KIND)) {
     sandwich_norm<KIND>(p, weights, other, x0, sh.scratch, fill);
   } else if (KIND == kSandwichOut) {
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
     if (KIND == kParallelIn) pdl_trigger();  // whoever runs after this knows that h is complete
     if (KIND != kParallelGate) {
       norm_single_load(values, p.h, p.cols0);
-      stream_fill<SLOTS>(rs);  // the ring slot held back, now behind the activation loads
+      stream_fill<SLOTS, kCompact>(rs);  // the ring slot held back, now behind the activation loads
     }
     if (p.step != nullptr) {
 #pragma unroll
@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) parallel_stream_kernel(Para
   }
   __syncthreads();
 
-  stream_consume<SLOTS>(rs, sh.first, 0, x0, total0, p.error_word);
-  if (second) stream_consume<SLOTS>(rs, sh.second, 1, x1, total1, p.error_word);
+  stream_consume<SLOTS, kCompact>(rs, sh.first, 0, x0, total0, p.error_word);
+  if (second) stream_consume<SLOTS, kCompact>(rs, sh.second, 1, x1, total1, p.error_word);
   __syncthreads();
 
   if (KIND == kParallelIn || KIND == kSandwichIn || KIND == kSandwichOut) {

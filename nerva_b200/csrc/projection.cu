@@ -69,7 +69,7 @@ __device__ __noinline__ void gather_prologue(const ProjectionParams &p, uint16_t
 constexpr uint32_t kPrewaitSlots = kStreamSlots - 1u;
 constexpr uint32_t kPlainL2PrefetchBytes = 16384;  // per warp, after the plain vector copy
 
-template <uint32_t EPI, bool TP>
+template <uint32_t EPI, bool TP, StreamForm FORM>
 __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(ProjectionParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t *ring = smem;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(Pr
   // norm prologue the last ring slot is held back until the activation loads have been issued:
   // they would otherwise queue behind a whole ring of bulk copies.
   const bool gathers = TP && p.prologue == kPrologueAddNorm && p.gather.world > 1 && p.add_b != nullptr;
-  stream_fill(rs, norm_single || gathers ? kPrewaitSlots : kStreamSlots);
+  stream_fill<kStreamSlots, FORM>(rs, norm_single || gathers ? kPrewaitSlots : kStreamSlots);
 
   uint32_t row_begin, row_end;
   block_row_range(p.rows, unit, blockIdx.x, gridDim.x, &row_begin, &row_end);
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(Pr
     } else if (norm_single) {
       NormValueRegs loaded;
       norm_single_load(loaded, p.add_a, p.cols);
-      stream_fill(rs);  // the slot held back above, now behind the activation loads
+      stream_fill<kStreamSlots, FORM>(rs);  // the slot held back above, now behind the activation loads
       norm_single_finish(x, loaded, norm_regs, p.eps, p.cols, sh.scratch);
     } else {
       add_norm_to_smem(x, p.add_a, p.add_b, p.add_bias, p.norm_weight, p.eps, p.cols,
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) projection_stream_kernel(Pr
   __syncthreads();
   stamp(p.stamps, kStampAfterPrologue);
 
-  stream_consume(rs, sh.stream, 0, x, row_total, p.error_word);
+  stream_consume<kStreamSlots, FORM>(rs, sh.stream, 0, x, row_total, p.error_word);
   __syncthreads();
 
   // Epilogue over the block's rows, coalesced.
@@ -315,6 +315,14 @@ bool stream_eligible(const ProjectionParams &p, uint32_t sm_count) {
 
 }  // namespace
 
+// Rows that can share a chunk go to kernels of their own (measured at StreamForm): with both forms in one kernel long rows
+// lose 1 to 3 %.
+template <uint32_t EPI>
+static void (*stream_kernel(bool tp, bool short_rows))(ProjectionParams) {
+  if (short_rows) return tp ? projection_stream_kernel<EPI, true, kShortRows> : projection_stream_kernel<EPI, false, kShortRows>;
+  return tp ? projection_stream_kernel<EPI, true, kLongRows> : projection_stream_kernel<EPI, false, kLongRows>;
+}
+
 cudaError_t configure_projection_kernels() {
   const int max_smem = 227 * 1024;
   cudaError_t err = cudaSuccess;
@@ -322,12 +330,12 @@ cudaError_t configure_projection_kernels() {
     if (err == cudaSuccess)
       err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   };
-  set(projection_stream_kernel<kEpilogueStore, false>);
-  set(projection_stream_kernel<kEpilogueSwiglu, false>);
-  set(projection_stream_kernel<kEpilogueArgmax, false>);
-  set(projection_stream_kernel<kEpilogueStore, true>);
-  set(projection_stream_kernel<kEpilogueSwiglu, true>);
-  set(projection_stream_kernel<kEpilogueArgmax, true>);
+  for (uint32_t i = 0; i < 4u; ++i) {
+    const bool tp = (i & 1u) != 0, short_rows = (i & 2u) != 0;
+    set(stream_kernel<kEpilogueStore>(tp, short_rows));
+    set(stream_kernel<kEpilogueSwiglu>(tp, short_rows));
+    set(stream_kernel<kEpilogueArgmax>(tp, short_rows));
+  }
   return err;
 }
 
@@ -344,14 +352,10 @@ cudaError_t launch_projection(cudaStream_t stream, const ProjectionParams &p, ui
     const uint32_t smem = stream_smem_bytes(p, blocks);
     const bool pdl = p.pdl != 0;
     const bool tp = p.push.world > 1 || p.gather.world > 1;
-    void (*kernel)(ProjectionParams) = nullptr;
-    if (p.epilogue == kEpilogueStore) {
-      kernel = tp ? projection_stream_kernel<kEpilogueStore, true> : projection_stream_kernel<kEpilogueStore, false>;
-    } else if (p.epilogue == kEpilogueSwiglu) {
-      kernel = tp ? projection_stream_kernel<kEpilogueSwiglu, true> : projection_stream_kernel<kEpilogueSwiglu, false>;
-    } else {
-      kernel = tp ? projection_stream_kernel<kEpilogueArgmax, true> : projection_stream_kernel<kEpilogueArgmax, false>;
-    }
+    const bool short_rows = p.cols * 2u <= kPairRowBytes;
+    auto *kernel = p.epilogue == kEpilogueStore    ? stream_kernel<kEpilogueStore>(tp, short_rows)
+                   : p.epilogue == kEpilogueSwiglu ? stream_kernel<kEpilogueSwiglu>(tp, short_rows)
+                                                   : stream_kernel<kEpilogueArgmax>(tp, short_rows);
     return launch_with_pdl(kernel, dim3(blocks), dim3(kStreamThreads), smem, stream, pdl, p);
   }
   if (p.push.world > 1 || p.gather.world > 1) return cudaErrorNotSupported;  // exchange: streaming path only

@@ -152,3 +152,26 @@ def test_projection_of_row_pairs_at_their_edges(built_lib, rows, cols):
     rc, out = ops.projection_bench(rows, cols, iterations=1, warmup=1)
     assert rc == 0 and out.status == 0 and out.mismatch_count == 0
     assert out.max_abs_diff <= (0.0 if cols <= 4096 else 72 * 2.0 ** -13)
+
+
+@pytest.mark.parametrize("rows,cols", [(4097, 512), (2049, 1032), (4096, 2048), (4097, 4096), (3001, 12288), (18992, 4096)])
+def test_single_token_sums_are_those_of_fp32(built_lib, rows, cols):
+    """Against the 64-bit product of the same operands.  A row's sum goes through at most cols / 32 + 24 roundings to nearest
+    (a lane's products, four accumulators, the warp, the warps of a row), each of half a unit of the sum so far.  They fall on
+    either side: the mean over thousands of rows of one sign is 1e-9 of the sum, and a sum that is cut off towards zero,
+    as the tensor pipe's, is 3e-8 to 9e-8 too small.  Odd rows: the last one of a block has no partner."""
+    rng = np.random.default_rng(rows + cols)
+    for sign in (False, True):
+        w = rng.standard_normal((rows, cols)) * cols ** -0.5
+        x = rng.standard_normal(cols)
+        if sign:
+            w, x = np.abs(w), np.abs(x)
+        wb, xb = synth.f32_to_bf16(w.astype(np.float32)), synth.f32_to_bf16(x.astype(np.float32))
+        y, _ = ops.projection(wb, xb, rows, cols)
+        wv, xv = synth.bf16_to_f32(wb).astype(np.float64).reshape(rows, cols), synth.bf16_to_f32(xb).astype(np.float64)
+        error = y[0] - wv @ xv
+        size = np.abs(wv) @ np.abs(xv)
+        assert np.isfinite(y).all()
+        assert (np.abs(error) <= (cols / 32 + 24) * 2.0 ** -24 * size).all()
+        if sign:
+            assert abs((error / size).mean()) <= 1e-8

@@ -473,17 +473,16 @@ cudaError_t configure_gemm_tc_kernel() {
   return err == cudaSuccess ? configure_gemm_wide_kernel() : err;
 }
 
-// From kSmallBlockTokens tokens on a block here is alone on its SM, and what it leaves to the fix-up launch grows with rows and
-// tokens; tiles on pairs of SMs (gemm_wide.cu) leave nothing, but have all slices of the inner dimension to go through.
-// Both as lines through measurements at 70 to 256 tokens, us, here and there: 4096 x 4096 17 to 27, 19 to 20; 4096 x 12288
-// 27 to 38, 49; 6144 x 4096 18 to 31, 19 to 21; 24576 x 4096 57 to 70, 44 to 53; 2048 x 2048 12 to 17, 11.5; 4096 x 2048 13 to 23,
-// 12 to 12.6; 12288 x 2048 21 to 38, 13 to 18.5; 2048 x 6144 15 to 22, 26.
+// With more than kSmallBlockTokens tokens a block here is alone on its SM and its runs come in two waves of their own
+// start and end.  Matrices whose 256-row tiles occupy most pairs of SMs go to gemm_wide.cu then: 24576 x 4096, 70 to 256 tokens
+// 44 to 53 us, here 57 to 70.  Fewer rows leave pairs idle there (4096 x 12288 49 us, here 27 to 38), and where they are
+// faster all the same (256 tokens: 4096 x 4096 20 us, here 27; 6144 x 4096 21 and 31) they lose precision: the tensor pipe cuts its
+// sums off towards zero, and a tile there has the whole inner dimension for one sum, which here is cut into the runs of
+// several blocks (4096 x 4096: about nine) that meet in fp32.  Relative error against 64 bits, 128 tokens: 4096 x 4096 4.0e-7 here and 4.4e-6, 6144 x 4096 6.0e-7 and 4.4e-6,
+// 2048 x 2048 1.4e-7 and 2.1e-6.  Of 24576 rows no tile is cut here: 4.4e-6 on either path.
 static bool wide_from_65_tokens(const GemmParams &g, uint32_t sm_count) {
-  if (g.tokens <= kSmallBlockTokens || g.tokens > kGemmMaxTokens || !gemm_shape_ok(g)) return false;
-  const uint64_t bytes = static_cast<uint64_t>(g.rows) * g.cols * 2u;
-  const uint64_t here = 8000u + bytes / 6400u + static_cast<uint64_t>(g.tokens) * g.rows / 80u;  // ns
-  const uint64_t there = 4000u + 235ull * (g.cols / kSliceK) * gemm_wide_waves(g.rows, g.tokens, sm_count);
-  return there < here;
+  return g.tokens > kSmallBlockTokens && g.tokens <= kGemmMaxTokens && gemm_shape_ok(g) &&
+         (g.rows + 2u * kTileRows - 1u) / (2u * kTileRows) >= sm_count / 2u * 3u / 4u;
 }
 
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count) {

@@ -290,11 +290,6 @@ void gemm_wide_launches(std::vector<TensorMemoryLaunch> *out) {
   for (uint32_t n = kMinTileTokens; n <= kMaxTileTokens; n += kTokenStep) out->push_back({wide_smem_bytes(n), kTmemColumns});
 }
 
-uint32_t gemm_wide_waves(uint32_t rows, uint32_t tokens, uint32_t sm_count) {
-  const uint32_t pairs = sm_count / 2u, n = choose_tile_tokens(rows, tokens, pairs);
-  return ((rows + kPairRows - 1u) / kPairRows * ((tokens + n - 1u) / n) + pairs - 1u) / pairs;
-}
-
 cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t sm_count) {
   const uint32_t pairs = sm_count / 2u;
   WideTiles t{};

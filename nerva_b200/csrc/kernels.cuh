@@ -132,7 +132,7 @@ struct GemmParams {
   const float *resid_in;   // optional [tokens][rows]; may be out_f32
   float *out_f32;          // [tokens][rows]
   uint16_t *out_bf16;      // [tokens][rows/2]
-  float *workspace;        // gemm_tc_workspace_bytes(tokens, sm_count); unused above kGemmMaxTokens
+  float *workspace;        // gemm_tc_workspace_bytes(tokens, sm_count); unused by launch_gemm_wide
   uint32_t *tickets;       // unused (kept so that callers' buffer plans stay as they are)
   uint32_t *error_word;
   uint32_t pdl;
@@ -151,8 +151,8 @@ bool encode_bf16_map_2d(void *map, const uint16_t *base, uint64_t inner, uint64_
                         uint32_t box_outer);
 cudaError_t configure_gemm_tc_kernel();  // and gemm_wide.cu's
 cudaError_t configure_gemm_wide_kernel();
-uint32_t gemm_wide_waves(uint32_t rows, uint32_t tokens, uint32_t sm_count);  // tiles that the busiest pair of SMs takes
-// launch_gemm_tc takes any number of tokens: above kGemmMaxTokens it is launch_gemm_wide.
+// launch_gemm_tc takes any number of tokens: above kGemmMaxTokens, and from 65 on where a matrix has rows for most pairs of SMs,
+// it is launch_gemm_wide.
 cudaError_t launch_gemm_wide(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);
 cudaError_t launch_gemm_tc(cudaStream_t stream, const GemmParams &g, uint32_t sm_count);
 

@@ -84,3 +84,17 @@ def test_reference_projection_bench_entry_point_with_a_block(built_lib):
     assert out.custom_avg_ns > 0 and out.block_cublaslt_avg_ns > 0 and out.block_cublaslt_graph_avg_ns > 0
     # eight tokens for less than eight single-token passes over the weights
     assert out.block_cublaslt_graph_avg_ns < 8 * out.custom_graph_avg_ns
+
+
+@pytest.mark.parametrize("rows,cols,counts", [(4096, 4096, (70, 128, 256)), (6144, 4096, (65, 200)), (2048, 2048, (129, 241)),
+                                              (2048, 6144, (129, 241, 256)), (4096, 12288, (113, 256)), (13824, 128, (65, 100))])
+def test_a_split_rows_sum_is_as_good_in_a_block_of_up_to_256_tokens(built_lib, rows, cols, counts):
+    """Where a matrix has fewer rows than fill the pairs of SMs its inner dimension is split up to 256 tokens, and the parts of
+    a sum meet in fp32: what the tensor pipe cuts off grows with the length of a part.  The cut is the matrix's alone, so the
+    sums of a token are the same bits in a block of any such length."""
+    w, x = _weights(rows, cols), _acts(cols, max(counts))
+    few, _ = ops.projection(w, x[:40 * cols], rows, cols, tokens=40)
+    for tokens in counts:
+        y, _ = ops.projection(w, x[:tokens * cols], rows, cols, tokens=tokens)
+        assert np.isfinite(y).all()
+        assert np.array_equal(y[:40], few), tokens

@@ -1005,6 +1005,12 @@ int nerva_b200_session_read_timeline(NervaCudaHfDecodeSequenceSession *session, 
 int nerva_b200_projection(const uint16_t *weight, const uint16_t *x, float *y, uint32_t rows,
                           uint32_t cols, uint32_t tokens, uint32_t warmup, uint32_t iterations,
                           uint64_t *avg_ns);
+/* Isolated block projection (2 tokens or more, cols a multiple of 64) with the epilogues of the block steps.  Rows below
+ * split_row, a multiple of 32, are stored: out[token][split_row] += y.  Rows from split_row on are interleaved (gate, up)
+ * pairs: gated[token][(rows - split_row) / 2] = bf16(act(gate) * up), act 0 SiLU or 1 tanh GELU.  HOST memory; an output
+ * that has no rows may be NULL. */
+int nerva_b200_block_projection(const uint16_t *weight, const uint16_t *x, float *out, uint16_t *gated, uint32_t rows,
+                                uint32_t cols, uint32_t tokens, uint32_t split_row, uint32_t activation);
 /* Sustained form of the same measurement (no counterpart in the reference): `copies` device copies
  * of the matrix, together larger than the L2, are projected back to back, each launch allowed to
  * start while its predecessor drains, as the projections of consecutive layers follow each other

@@ -188,6 +188,63 @@ extern "C" int nerva_b200_projection(const uint16_t *weight, const uint16_t *x, 
   return 0;
 }
 
+extern "C" int nerva_b200_block_projection(const uint16_t *weight, const uint16_t *x, float *out, uint16_t *gated, uint32_t rows,
+                                           uint32_t cols, uint32_t tokens, uint32_t split_row, uint32_t activation) {
+  set_last_error("");
+  if (weight == nullptr || x == nullptr || rows == 0 || cols == 0 || tokens < 2 || split_row > rows ||
+      (split_row != 0 && out == nullptr) || (split_row != rows && gated == nullptr) || activation > 1u)
+    return -1;
+  uint32_t sms = 0;
+  cudaError_t err = device_sm_count(&sms, nullptr, nullptr, nullptr);
+  if (err == cudaSuccess) err = configure_gemm_tc_kernel();
+  DeviceBuffers buf;
+  uint16_t *d_w = nullptr, *d_x = nullptr, *d_gated = nullptr;
+  float *d_out = nullptr, *d_ws = nullptr;
+  uint32_t *d_error = nullptr;
+  const uint64_t w_elems = static_cast<uint64_t>(rows) * cols, x_elems = static_cast<uint64_t>(tokens) * cols;
+  const uint64_t out_elems = static_cast<uint64_t>(tokens) * split_row, gated_elems = static_cast<uint64_t>(tokens) * ((rows - split_row) / 2u);
+  const uint32_t split_tokens = tokens < kGemmMaxTokens ? tokens : kGemmMaxTokens;  // more are never split
+  if (err == cudaSuccess) err = buf.alloc(&d_w, w_elems);
+  if (err == cudaSuccess) err = buf.alloc(&d_x, x_elems);
+  if (err == cudaSuccess && out_elems != 0) err = buf.alloc(&d_out, out_elems);
+  if (err == cudaSuccess && gated_elems != 0) err = buf.alloc(&d_gated, gated_elems);
+  if (err == cudaSuccess) err = buf.alloc(&d_ws, gemm_tc_workspace_bytes(split_tokens, sms) / sizeof(float));
+  if (err == cudaSuccess) err = buf.alloc(&d_error, 1);
+  if (err == cudaSuccess) err = cudaMemset(d_error, 0, sizeof(uint32_t));
+  if (err == cudaSuccess) err = cudaMemcpy(d_w, weight, w_elems * 2u, cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = cudaMemcpy(d_x, x, x_elems * 2u, cudaMemcpyHostToDevice);
+  if (err == cudaSuccess && out_elems != 0) err = cudaMemcpy(d_out, out, out_elems * 4u, cudaMemcpyHostToDevice);
+  GemmParams g{};
+  g.weight = d_w;
+  g.rows = rows;
+  g.cols = cols;
+  g.x = d_x;
+  g.tokens = tokens;
+  g.epilogue = split_row == rows ? kEpilogueStore : split_row == 0 ? kEpilogueSwiglu : kEpilogueStoreSwiglu;
+  g.split_row = split_row;
+  g.activation = activation;
+  g.resid_in = d_out;
+  g.out_f32 = d_out;
+  g.out_bf16 = d_gated;
+  g.workspace = d_ws;
+  g.error_word = d_error;
+  if (err == cudaSuccess && !gemm_tc_eligible(g) && !gemm_wide_eligible(g)) err = cudaErrorNotSupported;
+  if (err == cudaSuccess) err = launch_gemm_tc(nullptr, g, sms);
+  if (err == cudaSuccess && out_elems != 0) err = cudaMemcpy(out, d_out, out_elems * 4u, cudaMemcpyDeviceToHost);
+  if (err == cudaSuccess && gated_elems != 0) err = cudaMemcpy(gated, d_gated, gated_elems * 2u, cudaMemcpyDeviceToHost);
+  uint32_t device_error = 0;
+  if (err == cudaSuccess) err = cudaMemcpy(&device_error, d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+  if (err != cudaSuccess) {
+    set_last_error(cudaGetErrorString(err));
+    return -1;
+  }
+  if (device_error != 0) {
+    set_last_error("block projection kernel gave up a bounded wait (device error code " + std::to_string(device_error) + ")");
+    return -1;
+  }
+  return 0;
+}
+
 // Sustained form of the same measurement: `copies` device copies of the matrix (together larger
 // than the L2, so no launch finds its weights cached) are projected back to back, each launch
 // allowed to start while its predecessor drains (programmatic dependent launch), the way the

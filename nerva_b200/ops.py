@@ -26,6 +26,21 @@ def projection(weight_bits: np.ndarray, x_bits: np.ndarray, rows: int, cols: int
     return y, ns.value
 
 
+def block_projection(weight_bits: np.ndarray, x_bits: np.ndarray, rows: int, cols: int, tokens: int, residual=None,
+                     activation: int = 0):
+    """A block step's projection with its epilogues: the first residual.shape[1] rows are added to residual [tokens, n] (in
+    place on the device), the others are interleaved (gate, up) pairs.  Returns (residual + y, bf16 bits of act(gate) * up)."""
+    w = np.ascontiguousarray(weight_bits, dtype=np.uint16)
+    x = np.ascontiguousarray(x_bits, dtype=np.uint16)
+    out = np.array(residual, dtype=np.float32) if residual is not None else np.empty((tokens, 0), dtype=np.float32)
+    split = out.shape[1]
+    assert w.size == rows * cols and x.size == tokens * cols and out.shape[0] == tokens and (rows - split) % 2 == 0
+    gated = np.empty((tokens, (rows - split) // 2), dtype=np.uint16)
+    _check(ffi.lib().nerva_b200_block_projection(w.ctypes.data, x.ctypes.data, out.ctypes.data, gated.ctypes.data, rows, cols,
+                                                 tokens, split, activation), "block_projection")
+    return out, gated
+
+
 def projection_sustained(weight_bits: np.ndarray, x_bits: np.ndarray, rows: int, cols: int, tokens: int = 1,
                          copies: int = 2, warmup: int = 4, iterations: int = 20):
     """The same projection over `copies` device copies of the matrix (together larger than the L2),

@@ -123,6 +123,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     if (clock64() - start > kWaitCycleLimit) return false;
   }
 }
+// The same by a whole warp, with one verdict: each lane runs out of time by itself, and lanes that go on with different
+// verdicts would part in front of elect.sync, shuffles and MMAs, which wait for all of them.
+__device__ __forceinline__ bool warp_wait_bounded(uint64_t *bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
 // Generic-proxy accesses (the reads that just consumed a slot) are ordered
 // before the async-proxy write that refills it.
 __device__ __forceinline__ void fence_proxy_async() {

@@ -182,7 +182,7 @@ struct WarpRing {
   }
   // The oldest piece's slot, once it has landed.
   __device__ __forceinline__ const uint8_t *wait(uint32_t *error_word) {
-    if (!dead && !mbar_wait_bounded(&bars[slot], parity)) {
+    if (!dead && !warp_wait_bounded(&bars[slot], parity)) {
       dead = true;
       report_error(error_word, kErrTmaWaitTimeout);
     }

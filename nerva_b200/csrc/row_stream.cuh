@@ -323,7 +323,7 @@ template <uint32_t SLOTS>
 __device__ __forceinline__ const uint8_t *stream_wait(RowStream &rs, uint32_t *error_word) {
   const uint32_t slot = rs.consumed % SLOTS;
   const uint32_t parity = (rs.consumed / SLOTS) & 1u;
-  if (!rs.dead && !mbar_wait_bounded(&rs.bars[slot], parity)) {
+  if (!rs.dead && !warp_wait_bounded(&rs.bars[slot], parity)) {
     rs.dead = true;
     rs.drain_from = rs.consumed;
     rs.drain_to = rs.issued;

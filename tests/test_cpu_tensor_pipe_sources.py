@@ -71,6 +71,21 @@ def test_blocks_that_fit_on_an_sm_together_never_ask_for_more_tensor_memory_than
     assert most_columns(per_sm) <= 512
 
 
+def test_rings_that_issue_through_an_elected_lane_give_up_as_a_warp():
+    """elect.sync waits for all lanes: a ring whose copies are issued behind it may not be given up by some lanes only."""
+    rings = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        text = open(path).read()
+        if "elected()" not in text:
+            continue
+        for wait in re.findall(r"if \(!(?:\w+\.)?dead && !(\w+)\(", text):
+            assert wait == "warp_wait_bounded", os.path.basename(path)
+            rings += 1
+    assert rings == 2  # row_stream.cuh, moe.cu
+    common = open(os.path.join(CSRC, "common.cuh")).read()
+    assert re.search(r"bool warp_wait_bounded\([^)]*\) \{\s*return __all_sync\(0xffffffffu, mbar_wait_bounded\(bar, parity\)\);", common)
+
+
 @pytest.mark.parametrize("name", sorted(KERNELS))
 def test_no_lane_leaves_a_loop_of_warp_wide_loads_on_its_own(name):
     body = KERNELS[name]

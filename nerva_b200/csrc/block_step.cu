@@ -835,12 +835,6 @@ cudaError_t enqueue_chunked_prefill(NervaCudaHfDecodeSequenceSession *s, uint32_
         err = cudaMemcpyAsync(wanted.logits + static_cast<uint64_t>(place[i + k]) * d.vocab,
                               ws.logits + static_cast<uint64_t>(k) * d.vocab,
                               static_cast<uint64_t>(d.vocab) * sizeof(float), cudaMemcpyDeviceToHost, s->stream);
-      for (uint32_t k = 0; err == cudaSuccess && wanted.last != nullptr && !*wanted.last && k < count; ++k) {
-        if (begin + row[i + k] + 1u != prompt_count) continue;
-        err = cudaMemcpyAsync(s->logits, ws.logits + static_cast<uint64_t>(k) * d.vocab, static_cast<uint64_t>(d.vocab) * sizeof(float),
-                              cudaMemcpyDeviceToDevice, s->stream);
-        *wanted.last = true;
-      }
     }
   }
   return err;

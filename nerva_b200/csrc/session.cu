@@ -2615,26 +2615,12 @@ extern "C" int nerva_b200_session_append(Session *s, const uint32_t *tokens, uin
   s->started = false;
   s->prompt_count = end;
   if (chunked) {
-    bool last_logits = false;
-    const WantedLogits wanted{want, want_count, logits, &last_logits};
+    const WantedLogits wanted{want, want_count, logits};
     if (err == cudaSuccess) err = enqueue_chunked_prefill(s, begin, end, wanted, nullptr);
     const uint32_t last = end - 1u;
     if (err == cudaSuccess)
       err = cudaMemcpyAsync(s->device_cursor, &last, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream);
-    if (last_logits) {
-      // the last token's logits were wanted and stand in s->logits: sampled from, without another pass over the head (40 tokens
-      // through 8 layers of the 8B shapes 1.30 and 1.13 ms)
-      const BlockWorkspace &ws = s->weights->block_ws;
-      if (err == cudaSuccess && s->sample_kind == 2u) {
-        err = launch_sample_general(s->stream, step_state(s), s->logits, s->device_sampler, s->use_pdl);
-      } else if (err == cudaSuccess) {
-        err = launch_argmax_partials(s->stream, s->logits, s->dims.vocab, 1, kBlockArgmaxChunks, ws.best_value, ws.best_index, s->use_pdl);
-        if (err == cudaSuccess)
-          err = launch_sample_greedy(s->stream, step_state(s), ws.best_value, ws.best_index, kBlockArgmaxChunks, s->sample_kind, s->use_pdl, nullptr);
-      }
-    } else if (err == cudaSuccess) {
-      err = enqueue_step(s, splits_for(s, end), s->sample_kind, nullptr, nullptr, true);
-    }
+    if (err == cudaSuccess) err = enqueue_step(s, splits_for(s, end), s->sample_kind, nullptr, nullptr, true);
   } else {
     for (uint32_t i = 0; err == cudaSuccess && i < count; ++i) {
       bool sampled = i + 1u == count;

@@ -283,7 +283,6 @@ struct WantedLogits {
   const uint32_t *places = nullptr;
   uint32_t count = 0;
   float *logits = nullptr;
-  bool *last = nullptr;  // optional: set when the last position's logits were wanted and have been copied to the session's own
 };
 // Prompt positions [begin, prompt_count) of one session through every layer in chunks of up to
 // kBlockMaxRows tokens, writing the same paged bf16 K/V the decode step reads, then the final

@@ -16,16 +16,18 @@
 //  * Every call on one device shares the one array and it keeps its last
 //    contents.  The kernels write every (m, l) slot they later read and skip the
 //    accumulator of a slot whose l is 0, so only the error word has to start at
-//    zero; a call that finds it set clears it.  Two calls that overlap on
+//    zero; a call clears it on its own stream unless the one before it ended well.  Two calls that overlap on
 //    one device (two streams, two threads) race on the array: serialise them.
 //  * The first call on each device does the set-up (address of the array, SM
 //    count, shared-memory attributes of the kernels, host memory that the device can
-//    write) with that device current.
+//    write) with that device current.  The set-up works on no stream, so that it does not break another
+//    thread's stream capture.
 //  * The call returns after `stream` has finished the work, because it reads the
 //    kernel's error word.  The merge launch writes it to host memory when it is set: clearing
 //    and fetching it around the two launches, the fetch into pageable memory, took as
 //    long as the launches (one sequence of 8192 tokens: 39 us a call, 11 of them on the device; 30
 //    without the copies).
+#include <atomic>
 #include <mutex>
 
 #include "kernels.cuh"
@@ -53,12 +55,13 @@ struct DeviceSetup {
   uint32_t sm_count = 0;
   volatile uint32_t *host_error = nullptr;  // null: the error word is cleared and fetched by copies
   uint32_t *host_error_on_device = nullptr;
+  std::atomic<bool> clean{false};  // the device's word is known to be zero: the last call ran to its end and found no error
 };
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mutex;
 
 // Once per device, with that device current.
-cudaError_t setup_current_device(const DeviceSetup **out) {
+cudaError_t setup_current_device(DeviceSetup **out) {
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;
@@ -74,16 +77,15 @@ cudaError_t setup_current_device(const DeviceSetup **out) {
     if (err != cudaSuccess) return err;
     err = configure_attention_kernels();
     if (err != cudaSuccess) return err;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // a capture of another thread does not refuse the registration
+    cudaThreadExchangeStreamCaptureMode(&mode);
     static const bool registered =
         cudaHostRegister(const_cast<uint32_t *>(g_host_error), sizeof(g_host_error), cudaHostRegisterPortable | cudaHostRegisterMapped) ==
         cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     uint32_t *line = const_cast<uint32_t *>(g_host_error) + static_cast<size_t>(device) * kLineWords;
     void *mapped = nullptr;
     if (registered && cudaHostGetDevicePointer(&mapped, line, 0) == cudaSuccess) {
-      // the device's word is zero between calls from here on
-      err = cudaMemset(ptr + kScratchFloats, 0, sizeof(uint32_t));
-      if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
-      if (err != cudaSuccess) return err;
       d.host_error = line;
       d.host_error_on_device = static_cast<uint32_t *>(mapped);
     } else {
@@ -118,7 +120,7 @@ extern "C" int nerva_b200_gqa_decode_attention_static_scratch(
     set_last_error("misaligned buffer: q, key_pages and value_pages must start on a 16-byte boundary");
     return -1;
   }
-  const DeviceSetup *setup = nullptr;
+  DeviceSetup *setup = nullptr;
   cudaError_t err = setup_current_device(&setup);
   if (err != cudaSuccess) {
     set_last_error(cudaGetErrorString(err));
@@ -163,18 +165,13 @@ extern "C" int nerva_b200_gqa_decode_attention_static_scratch(
   if (told) {
     *setup->host_error = 0;
     p.host_error = setup->host_error_on_device;
-  } else {
-    err = cudaMemsetAsync(error_word, 0, sizeof(uint32_t), stream);
   }
+  if (!setup->clean.exchange(false) || !told) err = cudaMemsetAsync(error_word, 0, sizeof(uint32_t), stream);
   if (err == cudaSuccess) err = launch_attention(stream, p);
   if (err == cudaSuccess && !told)
     err = cudaMemcpyAsync(&device_error, error_word, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
   if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
-  if (err == cudaSuccess && told && *setup->host_error != 0) {
-    device_error = *setup->host_error;
-    err = cudaMemsetAsync(error_word, 0, sizeof(uint32_t), stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
-  }
+  if (err == cudaSuccess && told) device_error = *setup->host_error;
   if (err != cudaSuccess) {
     set_last_error(cudaGetErrorString(err));
     return -1;
@@ -183,5 +180,6 @@ extern "C" int nerva_b200_gqa_decode_attention_static_scratch(
     set_last_error("attention kernel reported a page index outside the page table");
     return -1;
   }
+  setup->clean = true;
   return 0;
 }

@@ -106,3 +106,13 @@ def test_shared_arrays_that_are_accessed_in_wider_pieces_are_aligned():
                       for line in re.findall(r"__shared__[^;]*;", kernel) for name in re.findall(r"(\w+)\[", line)}
             for name in re.findall(r"reinterpret_cast<(?:const )?(?:float|uint)[24] \*>\((\w+)", kernel):
                 assert arrays.get(name, True), (os.path.basename(path), name)
+
+
+def test_static_scratch_error_word_is_trusted_only_behind_a_call_that_ended_well():
+    """A launch that fails between the kernel that sets the word and the one that reports it leaves it set: whatever way a call
+    ends but the last one, the next call clears the word."""
+    text = open(os.path.join(CSRC, "attention_static_scratch.cu")).read()
+    call = text[text.index("int nerva_b200_gqa_decode_attention_static_scratch("):]
+    taken, launched = call.index("clean.exchange(false)"), call.index("launch_attention(")
+    assert taken < launched and "cudaMemsetAsync(error_word, 0" in call[taken:launched]
+    assert text.count("clean = true") == 1 and call.index("clean = true") > call.rindex("return -1;")

@@ -119,3 +119,49 @@ def test_page_index_outside_the_table_is_reported_and_forgotten(built_lib, heads
             _static_scratch(q, k, v, bad, 1, 500, heads, kv_heads, head_dim)
     again = _static_scratch(q, k, v, table, 1, 500, heads, kv_heads, head_dim)
     assert np.array_equal(again, good)
+
+
+_FIRST_CALL_DURING_A_CAPTURE = """
+import ctypes
+import threading
+import torch
+from nerva_b200 import ops
+q, out = torch.randn(8 * 64, device="cuda"), torch.zeros(8 * 64, device="cuda")
+keys, values = (torch.randn(48, 128, device="cuda").to(torch.bfloat16) for _ in range(2))
+table, side = torch.arange(3, dtype=torch.int32, device="cuda"), torch.cuda.Stream()
+failure = []
+
+def call():
+    try:
+        ops.gqa_decode_attention_static_scratch(q.data_ptr(), keys.data_ptr(), values.data_ptr(), table.data_ptr(), out.data_ptr(),
+                                                1, 48, 8, 2, 64, stream=side.cuda_stream)
+    except RuntimeError as e:
+        failure.append(e)
+
+def ok(status):
+    assert status == 0, status
+
+ops.greedy_argmax(torch.zeros(8).numpy())  # the library's context and kernels are there
+y = torch.ones(64, dtype=torch.int32, device="cuda")
+torch.cuda.synchronize()
+runtime = ctypes.CDLL("libcudart.so.12")
+stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+ok(runtime.cudaStreamCreate(ctypes.byref(stream)))  # one that waits for the legacy stream
+ok(runtime.cudaStreamBeginCapture(stream, 1))  # thread-local
+ok(runtime.cudaMemsetAsync(ctypes.c_void_p(y.data_ptr()), 0, 256, stream))
+thread = threading.Thread(target=call)
+thread.start()
+thread.join()
+ok(runtime.cudaStreamEndCapture(stream, ctypes.byref(graph)))
+assert not failure, failure
+assert torch.isfinite(out).all() and out.abs().sum().item() > 0 and y.sum().item() == 64
+"""
+
+
+def test_first_call_leaves_another_threads_capture_alone(built_lib):
+    """The set-up on the first call of a process touches no stream but the caller's."""
+    import subprocess
+    import sys
+    from tests.conftest import ROOT
+    done = subprocess.run([sys.executable, "-c", _FIRST_CALL_DURING_A_CAPTURE], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]

@@ -68,20 +68,23 @@ def test_kernel_matches_oracle(built_lib, oracle_mod, name):
 
 
 def _arranged(kind, count):
-    """The kernel's cluster takes index i in slice i % 8192 // 32; the bound of its list comes from the slices' maxima."""
+    """The kernel's cluster takes index i in slice i % 8192 // 32 (of fewer than 8192 logits: i % 256); the bound of its list
+    comes from the slices' maxima."""
     rng = np.random.default_rng(count)
     out = (rng.standard_normal(count) * 3.0).astype(np.float32)
+    index = np.arange(count)
+    few = np.isin(index % 8192 // 32 if count >= 8192 else index % 256, (3, 4, 250))
     if kind == "few slices":  # hold all of the largest: more keys reach the bound than the list takes
-        out[np.isin(np.arange(count) % 8192 // 32, (3, 4, 250))] += 40.0
+        out[few] += 40.0
     elif kind == "finite in few slices":  # fewer maxima than candidates: no bound
-        out[~np.isin(np.arange(count) % 8192 // 32, (3, 4, 250))] = np.nan
+        out[~few] = np.nan
     elif kind == "ascending":
         out.sort()
     return out
 
 
 @pytest.mark.parametrize("kind", ["random", "few slices", "finite in few slices", "ascending"])
-@pytest.mark.parametrize("count", [2, 128, 255, 8191, 8193, 65537, 151936])
+@pytest.mark.parametrize("count", [2, 128, 255, 1024, 1025, 4064, 4065, 8191, 8192, 8193, 65537, 151936])
 def test_candidates_at_the_edges_of_slices(built_lib, oracle_mod, kind, count):
     logits = _arranged(kind, count)
     for temperature, top_p, top_k in [(1.0, 1.0, 0), (0.9, 0.95, 0), (1.5, 1.0, 128), (0.7, 0.9, 50), (1.0, 0.5, 2)]:

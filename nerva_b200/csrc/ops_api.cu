@@ -673,6 +673,12 @@ extern "C" int nerva_cuda_projection_bench(const NervaCudaProjectionBenchRequest
     }
   }
   // check against an fp64 host dot product of the same bf16 inputs on a row sample
+  auto compare = [out](float y, double want) {
+    const float diff = fabsf(y - static_cast<float>(want));
+    const bool number = diff <= INFINITY;  // a result that is not one has no distance: it counts as the largest
+    if (!number || diff > out->max_abs_diff) out->max_abs_diff = number ? diff : INFINITY;
+    if (!(diff <= 0.25f)) out->mismatch_count += 1;  // the reference's tolerance (:843-845)
+  };
   std::vector<float> h_y(rows);
   if (err == cudaSuccess) err = cudaMemcpy(h_y.data(), d_y, rows * 4u, cudaMemcpyDeviceToHost);
   if (err == cudaSuccess) {
@@ -684,9 +690,7 @@ extern "C" int nerva_cuda_projection_bench(const NervaCudaProjectionBenchRequest
         const float xv = __builtin_bit_cast(float, static_cast<uint32_t>(h_x[k]) << 16);
         acc += static_cast<double>(w) * xv;
       }
-      const float diff = fabsf(h_y[r] - static_cast<float>(acc));
-      if (diff > out->max_abs_diff) out->max_abs_diff = diff;
-      if (diff > 0.25f) out->mismatch_count += 1;  // the reference's tolerance (:843-845)
+      compare(h_y[r], acc);
     }
   }
   if (err == cudaSuccess && tokens > 1) {
@@ -705,9 +709,7 @@ extern "C" int nerva_cuda_projection_bench(const NervaCudaProjectionBenchRequest
           const float xv = __builtin_bit_cast(float, static_cast<uint32_t>(h_xb[static_cast<uint64_t>(m) * cols + k]) << 16);
           acc += static_cast<double>(w) * xv;
         }
-        const float diff = fabsf(h_yb[static_cast<uint64_t>(m) * rows + r] - static_cast<float>(acc));
-        if (diff > out->max_abs_diff) out->max_abs_diff = diff;
-        if (!(diff <= 0.25f)) out->mismatch_count += 1;
+        compare(h_yb[static_cast<uint64_t>(m) * rows + r], acc);
       }
     }
   }

@@ -7,7 +7,7 @@ import os
 import numpy as np
 import pytest
 
-from tests.conftest import GOLDEN, _has_gpu
+from tests.conftest import GOLDEN, ROOT, _has_gpu
 from nerva_b200 import ffi, ops, session, synth
 
 
@@ -298,3 +298,13 @@ def test_kv_page_pool_caches_prefix_keys_and_retain_hits(built_lib):
     assert L.nerva_b200_kv_page_pool_evict_cached(pool, handle) == 0
     L.nerva_b200_kv_page_pool_free(pool)
     L.nerva_b200_static_arena_free(arena)
+
+
+def test_projection_check_counts_results_that_are_no_numbers():
+    """Comparisons with a NaN are false: the check of the projection benchmark must be written so that it fails then."""
+    text = open(os.path.join(ROOT, "nerva_b200", "csrc", "ops_api.cu")).read()
+    check = text[text.index("auto compare = [out](float y, double want)"):]
+    check = check[:check.index("};")]
+    assert "!(diff <= 0.25f)" in check and "diff <= INFINITY" in check
+    assert text.count("compare(h_y[r], acc);") == 1 and text.count("compare(h_yb[") == 1
+    assert "mismatch_count += 1" not in text.replace(check, "").replace("if (device_error != 0) out->mismatch_count += 1;", "")

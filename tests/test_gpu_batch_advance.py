@@ -141,3 +141,31 @@ def test_stop_token_and_context_end_finish_a_session(built_lib, tiny_checkpoint)
     out = CudaHfDecodeSequenceSession.batch_advance_one([s], 1, 1)
     assert out.status == SmokeStatus.OK and out.reason == 3 and out.tokens == [NOT_TAKEN]
     s.destroy()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (4, 4, 128)])
+def test_one_span_of_the_cache_and_several_agree(built_lib, heads, kv_heads, head_dim):
+    """A packed step walks the cache in as many spans as its longest session takes; with one span its attention launch finishes
+    the rows itself, with more a merge does.  Sessions of 1 to 64 tokens beside each other (one span) and beside 300 more."""
+    import dataclasses
+    from nerva_b200 import ops
+    cfg = dataclasses.replace(synth.TINY_QWEN3, layers=2, heads=heads, kv_heads=kv_heads, head_dim=head_dim, vocab=4096)
+    checkpoint = synth.dense_checkpoint(cfg, fill=ops.synth_normal_bf16)
+    parent, loop = _started(checkpoint, synth.uniform_u32(9, synth.T_PROMPT, 300, cfg.vocab), max_context=512)
+    loop.advance(1)
+    short = []
+    for count in (1, 2, 15, 16, 17, 31, 62):
+        s = parent.fork_shared_weights()
+        assert CudaHfDecodeSequenceLoop.start(s, synth.uniform_u32(count, synth.T_PROMPT, count, cfg.vocab))[0].status == SmokeStatus.OK
+        CudaHfDecodeSequenceLoop(s).advance(1)
+        short.append(s)
+    twins = [s.fork_shared_weights() for s in short]
+    one = CudaHfDecodeSequenceSession.batch_advance_one(short, 16, 2)
+    several = CudaHfDecodeSequenceSession.batch_advance_one(twins + [parent], 16, 2)
+    assert one.status == SmokeStatus.OK and one.block_tokens == len(short), one.error
+    assert several.status == SmokeStatus.OK and several.block_tokens == len(twins) + 1, several.error
+    for s, twin in zip(short, twins):
+        a, b = s.read_logits(), twin.read_logits()
+        assert np.isfinite(a).all() and np.abs(a - b).max() <= 2e-2
+    for s in short + twins + [parent]:
+        s.destroy()

@@ -175,3 +175,18 @@ def test_single_token_sums_are_those_of_fp32(built_lib, rows, cols):
         assert (np.abs(error) <= (cols / 32 + 24) * 2.0 ** -24 * size).all()
         if sign:
             assert abs((error / size).mean()) <= 1e-8
+
+
+@pytest.mark.parametrize("rows,cols", [(33, 264), (301, 512), (299, 1032), (1001, 2048), (37, 4096), (149, 12288)])
+def test_a_weight_that_is_not_finite_stays_in_its_row(built_lib, rows, cols):
+    """Short rows share a chunk of the ring with their neighbour, others with what the ring held before."""
+    w, x = _weights(rows, cols).reshape(rows, cols), _acts(cols)
+    clean, _ = ops.projection(w, x, rows, cols)
+    bad = w.copy()
+    spoiled = sorted({0, 3, rows // 2, rows - 1})
+    for i, r in enumerate(spoiled):
+        bad[r, (7 * r + 5) % cols] = (0x7F80, 0xFF80, 0x7FC0, 0x7F80)[i]  # infinities and a NaN
+    y, _ = ops.projection(bad, x, rows, cols)
+    rest = np.setdiff1d(np.arange(rows), spoiled)
+    assert np.array_equal(y[0][rest], clean[0][rest])
+    assert not np.isfinite(y[0][spoiled]).any()

@@ -77,9 +77,8 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 // One lane of a converged warp.  A branch on it, unlike one on the lane's number, tells the compiler that a single thread
-// runs what follows, so the operands of copies and MMAs need no move to uniform registers each.  Those moves made the
-// issuing threads the bound of all kernels here: prompts through 8 layers of the 8B shapes and the head, `lane == 0` and this:
-// 300 tokens 2.54 and 1.99 ms, 2048 tokens 6.85 and 5.95.
+// runs what follows.  Issuing copies and MMAs behind it instead of behind `lane == 0`: prompts through 8 layers of the 8B
+// shapes and the head, 300 tokens 2.54 and 1.99 ms, 2048 tokens 6.85 and 5.95.
 __device__ __forceinline__ bool elected() {
   uint32_t leader;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));

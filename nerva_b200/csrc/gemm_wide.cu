@@ -16,14 +16,14 @@
 // columns), and the last one is not hidden: hence eight warps, values without branches and residuals a group ahead
 // (row_epilogue, row_residual).
 //
-// Measured back to back, other weights each time, 2048 tokens, with four warps and a branch per value, with this epilogue, and
-// with it and issuing threads chosen by elect.sync: 24576 x 4096 with SwiGLU 394, 311, 260 us, 1586 TFLOP/s of the last; 4096 x 12288 with residual
-// 178, 158, 140; 6144 x 4096 96, 89, 71; 4096 x 4096 with residual 85, 62, 52.
+// Measured back to back, other weights each time, 2048 tokens, and in brackets with four epilogue warps, a branch per value and
+// issuing threads chosen by lane: 24576 x 4096 with SwiGLU 260 us, 1586 TFLOP/s (394); 4096 x 12288 with residual 140 (178);
+// 6144 x 4096 71 (96); 4096 x 4096 with residual 52 (85).
 //
 // Roles inside a block (320 threads), as in gemm_tc.cu: warp 0 issues the TMA copies into the block's own ring,
 // warp 1 of the pair's first block issues the MMAs for both (its `full` barriers count the bytes of both blocks),
-// warps 2..9 read the accumulator and run the epilogue, four of them every second group of tokens.  Commits of the MMAs are signalled to both blocks.  Two
-// accumulator buffers of 256 columns let the epilogue of one tile run under the MMAs of the next.  Every wait is
+// warps 2..9 read the accumulator and run the epilogue, four of them every second group of tokens.  Commits of the MMAs
+// are signalled to both blocks.  Two accumulator buffers of 256 columns let the epilogue of one tile run under the MMAs of the next.  Every wait is
 // bounded; a wait that gives up sets the error word and the block's abort flag, the block drains and the pair
 // leaves together.  No copy is multicast.
 #include "gemm_device.cuh"
@@ -262,7 +262,8 @@ uint32_t wide_smem_bytes(uint32_t tile_tokens) {
 
 // Tokens per tile: the size with the shortest run of the slowest pair.  A slice costs a pair the larger of its MMA
 // time (2 cycles per token) and the time its shared memory takes to fill (about 45 bytes per cycle and SM with all
-// SMs loading), so narrow tiles pay for the weight rows they re-read; wide ones may leave a last wave nearly empty.
+// SMs loading and issuing threads chosen by lane; loads alone now take in 57, which changes the size for none of eight
+// matrices of 2048 to 24576 rows at ten counts from 257 to 2048), so narrow tiles pay for the weight rows they re-read; wide ones may leave a last wave nearly empty.
 uint32_t choose_tile_tokens(uint32_t rows, uint32_t tokens, uint32_t pairs) {
   const uint32_t row_tiles = (rows + kPairRows - 1u) / kPairRows;
   uint32_t best = kMaxTileTokens;

@@ -9,13 +9,12 @@
 // Queries and probabilities are fp32 values; each enters as a bf16 rounding and its remainder, two MMAs into the same
 // accumulator, so a product loses only the rounding of the cached row (the contract of the other attention kernels).
 //
-// What bounds it: the MMAs, 4 x 512 cycles a tile (two parts of Q, two of P), and the hand-overs between them.  With probes a
-// tile of a long walk takes 3500 cycles, 2090 of them issuing MMAs (2680 of 3920 while a lane's number chose the issuing
-// thread); the softmax warps wait 64 % of the time: a tile of theirs is 120 cycles of loads, 320 for the maximum, 1700 for 128
-// exponentials a thread, their sums and two packs.  S has two buffers: S(j+1) is computed while the
-// softmax works on S(j), but S(j+2) goes where P(j) is and waits for its PV.  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since
-// the reference it uses (the probabilities stay below 2^8, the sums exact to fp32): after the first tiles that almost
-// never happens.
+// What bounds it: the MMAs, 4 x 512 cycles a tile (two parts of Q, two of P), and the hand-overs between them.  By clock stamps
+// in a copy of this kernel a tile of a long walk takes 3500 cycles, 2090 of them issuing MMAs; the softmax warps wait 64 % of
+// the time: a tile of theirs is 120 cycles of loads, 320 for the maximum, 1700 for 128 exponentials a thread, their sums and
+// two packs.  S has two buffers: S(j+1) is computed while the softmax works on S(j), but S(j+2) goes where P(j) is and waits
+// for its PV.  The output accumulator is rescaled only when a row's maximum has grown by more than 2^8 since the reference
+// it uses (the probabilities stay below 2^8, the sums exact to fp32): after the first tiles that almost never happens.
 // One 128-row tile per block (both parts of Q, 64 KB, and two stages of K and V, 128 KB, fill shared memory), and two
 // groups of softmax warps, each with every second tile, a running maximum, a sum and an output accumulator of its own,
 // added at the end.  The second group gives little: 2048 tokens, 32 heads, 117 us with one group, 114 with two when it was added.
@@ -309,7 +308,7 @@ __global__ void __launch_bounds__(kAttentionThreads, 1) prefill_attention_kernel
   }
 
   if (warp == kMmaWarp) {
-    // ---------------- MMA issuer: the warp waits together, its first lane issues ----------------
+    // ---------------- MMA issuer: the warp waits together, an elected lane issues ----------------
     if (tiles != 0) {
       const uint32_t idesc_s = attention_instr_desc(kKeys, false), idesc_o = attention_instr_desc(D, true);
       auto scores = [&](uint32_t j) {  // S(j) = Q K(j)^T; its buffer held P(j - 2), which PV(j - 2) has read
